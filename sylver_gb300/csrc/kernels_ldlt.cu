@@ -781,33 +781,70 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
 
 // ---------------------------------------------------------------------------
 // L*D of contribution rows [n, m) over columns [0, nelim) (F.p = nelim).
+// A slice's CTAs stride over tiles of LDLT_RT rows x CLD columns, one row per
+// thread, CLD_U loads in flight.  (With all nelim columns on the thread of a
+// row the kernel was one latency chain: 39 us per launch on the shifted
+// 7-point 48^3 matrix, 51 us in FP64 on a 14^3 saddle point.)  Each column is
+// independent: the 2x2 coefficients are formed once per tile, and every
+// element keeps its operations, so the results keep their bits.
+constexpr int CLD = LDLT_CLD, CLD_U = 8;
 template <typename T>
 __global__ void __launch_bounds__(LDLT_RT) k_ldlt_calc_ld(const T* __restrict__ arena,
                                                          T* __restrict__ scratch,
                                                          const LdltFront* __restrict__ fr,
                                                          const CtaMap* __restrict__ cm,
                                                          LdltStep st) {
+  // column k: 0 divide by ca, 1 first of a 2x2 pair (l_k ca + l_k+1 cb),
+  // 2 second of a pair (l_k-1 ca + l_k cb), 3 zero pivot
+  __shared__ int kind[CLD];
+  __shared__ double ca[CLD], cb[CLD];
   const CtaMap c = cm[blockIdx.x];
   const LdltFront F = fr[c.f];
   const T* A = arena + F.off;
   const double* D = st.dall + F.d_off;
   T* out = scratch + F.ldp_off;
-  const int ne = F.p, ldo = F.m;
-  for (int r = F.n + c.local * LDLT_RT + threadIdx.x; r < F.m; r += c.count * LDLT_RT) {
-    for (int k = 0; k < ne;) {
-      if (k + 1 < ne && isinf(D[2 * k + 2])) {
-        const double a = D[2 * k], b = D[2 * k + 1], cc = D[2 * k + 3];
+  const int ne = F.p, tid = threadIdx.x;
+  const int64_t ldo = F.m, ld = F.ld;
+  const int nr = (F.m - F.n + LDLT_RT - 1) / LDLT_RT, nc = (ne + CLD - 1) / CLD;
+  for (int t = c.local; t < nr * nc; t += c.count) {
+    const int k0 = t / nr * CLD, kw = min(CLD, ne - k0);
+    const int r = F.n + t % nr * LDLT_RT + tid;
+    __syncthreads();
+    if (tid < kw) {
+      const int k = k0 + tid;
+      const bool second = k > 0 && isinf(D[2 * k]);
+      if (second || (k + 1 < ne && isinf(D[2 * k + 2]))) {
+        const int p = second ? k - 1 : k;
+        const double a = D[2 * p], b = D[2 * p + 1], cc = D[2 * p + 3];
         const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
-        const double d11 = cc / det, d21 = -b / det, d22 = a / det;
-        const double l1 = A[(int64_t)k * F.ld + r], l2 = A[(int64_t)(k + 1) * F.ld + r];
-        out[(int64_t)k * ldo + r] = (T)fma_(l1, d11, mul_(l2, d21));
-        out[(int64_t)(k + 1) * ldo + r] = (T)fma_(l1, d21, mul_(l2, d22));
-        k += 2;
+        kind[tid] = second ? 2 : 1;
+        ca[tid] = second ? -b / det : cc / det;
+        cb[tid] = second ? a / det : -b / det;
       } else {
-        const double d = D[2 * k];
-        const T l = A[(int64_t)k * F.ld + r];
-        out[(int64_t)k * ldo + r] = (d == 0.0) ? T(0) : l / (T)d;
-        k += 1;
+        kind[tid] = D[2 * k] == 0.0 ? 3 : 0;
+        ca[tid] = D[2 * k];
+      }
+    }
+    __syncthreads();
+    if (r >= F.m) continue;
+    for (int j0 = 0; j0 < kw; j0 += CLD_U) {
+      // l[u] = L(r, k0 + j0 + u - 1): one column more on either side, for pairs
+      T l[CLD_U + 2];
+#pragma unroll
+      for (int u = 0; u < CLD_U + 2; ++u) {
+        const int k = k0 + j0 + u - 1;
+        l[u] = (k >= 0 && k < ne) ? A[k * ld + r] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < CLD_U; ++u) {
+        const int j = j0 + u;
+        if (j >= kw) break;
+        const int kd = kind[j];
+        T v = T(0);
+        if (kd == 0) v = l[u + 1] / (T)ca[j];
+        else if (kd == 1) v = (T)fma_((double)l[u + 1], ca[j], mul_((double)l[u + 2], cb[j]));
+        else if (kd == 2) v = (T)fma_((double)l[u], ca[j], mul_((double)l[u + 1], cb[j]));
+        out[(k0 + j) * ldo + r] = v;
       }
     }
   }

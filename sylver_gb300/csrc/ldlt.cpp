@@ -70,6 +70,12 @@ namespace {
 
 inline int round_up(int v, int a) { return (v + a - 1) / a * a; }
 
+// elements per CTA of the zeroing and copying of whole spans: enough CTAs to
+// fill the chip for one front of a few hundred rows (spans of 2^20 elements
+// took 62 us per level on the shifted 7-point 48^3 matrix, and 96 us in FP64
+// on a 14^3 saddle point, nearly all of it one CTA's share)
+constexpr int64_t kSpan = 1 << 14;
+
 // threshold of the relaxed pass at the roots (keeps only the small-pivot test)
 constexpr double kRootU = 1e-300;
 inline int64_t round_up64(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
@@ -237,8 +243,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       L.ld[s2] = round_up(std::max(L.m[s2], 1), 4);
       const int64_t blk = round_up64((int64_t)L.ld[s2] * L.m[s2], 64);
       L.off[s2] = L.alloc.alloc(blk);
-      for (int64_t z = 0; z < blk; z += (int64_t)1 << 20)
-        zsp.push_back({L.off[s2] + z, std::min<int64_t>((int64_t)1 << 20, blk - z)});
+      for (int64_t z = 0; z < blk; z += kSpan)
+        zsp.push_back({L.off[s2] + z, std::min(kSpan, blk - z)});
       for (int c : st.children[s2]) L.pending.push_back(c);
       L.d_off[s2] = L.d_used;
       L.d_used += 2 * (int64_t)std::max(L.n[s2], 1);
@@ -497,8 +503,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
         const int64_t len = (int64_t)L.ld[s2] * L.nelim[s2];
         L.foff[s2] = L.fused;
         L.fused += round_up64(len, 64);
-        for (int64_t z = 0; z < len; z += (int64_t)1 << 20)
-          cs.push_back({L.off[s2] + z, L.foff[s2] + z, std::min<int64_t>((int64_t)1 << 20, len - z)});
+        for (int64_t z = 0; z < len; z += kSpan)
+          cs.push_back({L.off[s2] + z, L.foff[s2] + z, std::min(kSpan, len - z)});
       }
       if ((size_t)L.fused * sizeof(T) > fk.fstore.bytes)
         grow(fk.fstore, (size_t)L.fused * sizeof(T), s);
@@ -531,7 +537,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
         cscr += (int64_t)m * ne;
         int kf = (int)cfr.size();
         cfr.push_back(f);
-        add_slice(cm, kf, ceil_div(m - n, LDLT_RT));
+        add_slice(cm, kf, ceil_div(m - n, LDLT_RT) * ceil_div(ne, LDLT_CLD));
         const int mc = m - n;
         if (tc_ok && tc_min > 0 && mc >= tc_min) {
           pitch = std::max(pitch, (ne + TC_KCHUNK - 1) / TC_KCHUNK * TC_KCHUNK);

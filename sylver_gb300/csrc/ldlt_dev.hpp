@@ -7,6 +7,7 @@ namespace sylver_gb300 {
 
 constexpr int LDLT_BW = 32;   // block width of the a-posteriori pivoting
 constexpr int LDLT_RT = 128;  // rows per CTA tile in apply / commit / calc_ld
+constexpr int LDLT_CLD = 32;  // columns per CTA tile in calc_ld
 
 // One front of a level (fixed for the level; everything that pivoting
 // changes lives in the per-slot state arrays of LdltStep).
