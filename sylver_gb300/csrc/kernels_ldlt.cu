@@ -39,6 +39,7 @@
 // that a CPU restatement with std::fma in the same order reproduces the
 // factors bit for bit.
 #include <cfloat>
+#include <type_traits>
 
 #include "ldlt_dev.hpp"
 #include "tile_update.cuh"
@@ -80,7 +81,31 @@ __device__ __forceinline__ void warp_argmax(C& v, int& idx) {
 }
 
 // ---------------------------------------------------------------------------
-// Diagonal block of step k (one CTA per front, warp 0 pivots).
+// Magnitude keys for pivot searches: |v| as an unsigned integer, which orders
+// like the value, plus one; 0 for NaN (never chosen, as by `>` comparisons).
+__device__ __forceinline__ unsigned mag_key(float v) {
+  const unsigned b = __float_as_uint(v) & 0x7fffffffu;
+  return b > 0x7f800000u ? 0u : b + 1;
+}
+__device__ __forceinline__ unsigned long long mag_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b + 1;
+}
+__device__ __forceinline__ double key_mag(unsigned k) {
+  return k ? (double)__uint_as_float(k - 1) : -1.0;
+}
+__device__ __forceinline__ double key_mag(unsigned long long k) {
+  return k ? __longlong_as_double((long long)(k - 1)) : -1.0;
+}
+__device__ __forceinline__ unsigned warp_max(unsigned k) { return __reduce_max_sync(~0u, k); }
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
+  const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(~0u, hi);
+  const unsigned ml = __reduce_max_sync(~0u, hi == mh ? (unsigned)k : 0u);
+  return ((unsigned long long)mh << 32) | ml;
+}
+
+// ---------------------------------------------------------------------------
+// Diagonal block of step k (one CTA of eight warps per front).
 //   full block (32 columns): complete pivoting over the block, 1x1 or 2x2;
 //   partial block (w < 32 columns, the front's last): threshold partial
 //   pivoting over the w columns with rows = the w block rows followed by the
@@ -88,217 +113,259 @@ __device__ __forceinline__ void warp_argmax(C& v, int& idx) {
 // Output: the factored block (unit L, lower) in blk, D^-1, the local
 // permutation, the number of pivots taken (ndiag, also the initial
 // npass_raw), the L rows of the e extra rows into the apply panel; the block
-// permutation is applied to the rows of the eliminated columns [0, p) and to
-// the variable list.
+// permutation is applied to the variable list (k_app_commit applies it to the
+// rows of the eliminated columns).
+//
+// Bound by the serial chain of pivots.  The triangle stays in registers, three
+// entries per thread, and nothing is swapped: an entry keeps its two labels
+// (original panel rows) and lane x of every warp holds the current position of
+// label x.  A pivot takes two block barriers -- every warp reduces its entries'
+// magnitudes with redux, ties by position; the owners publish the pivot column
+// through shared memory; every thread updates its entries -- where one warp
+// with the triangle in shared memory took up to 32 shared-memory round trips
+// for the search and as many for the update.  Per launch on the shifted
+// 7-point 48^3 (FP32), on 27 x 24 x 21 and on a 14^3 saddle point (FP64): 93,
+// 119 and 104 us before, 30, 39 and 37 us now (of which the permutation of the
+// eliminated columns' rows moved to the commit).
+constexpr int DG_T = 256, DG_W = DG_T / 32, DG_E = 3;
 template <typename T>
-__global__ void __launch_bounds__(128) k_app_diag(T* __restrict__ arena, T* __restrict__ scratch,
-                                                  const LdltFront* __restrict__ fr,
-                                                  const CtaMap* __restrict__ cm, LdltStep st) {
+__global__ void __launch_bounds__(DG_T) k_app_diag(T* __restrict__ arena, T* __restrict__ scratch,
+                                                   const LdltFront* __restrict__ fr,
+                                                   const CtaMap* __restrict__ cm, LdltStep st) {
   using C = T;  // block arithmetic; FP64 for the pivot tests and 2x2 inverses
-  __shared__ C a[BW][LDB];  // a[j][i] = panel(i, j); i >= j, or i >= w (extra rows)
+  using K = decltype(mag_key(C(0)));
+  constexpr unsigned ALL = 0xffffffffu;
+  __shared__ C Ls[BW][LDB];  // Ls[s][x]: pivot s's column of L at label x
+  __shared__ C col1[BW], col2[BW], dg[BW];
+  __shared__ K pkey[DG_W];
+  __shared__ unsigned ptie[DG_W];
   __shared__ double dv[2 * BW];
   __shared__ int perm[BW];
-  __shared__ int s_nd;
   const LdltFront F = fr[cm[blockIdx.x].f];
   const int q = F.fidx, w = block_width(F, st.k), e = extra_rows(F, w), R = w + e;
   const int p = st.p_cur[q];
-  T* A = arena + F.off;
+  const T* A = arena + F.off;
   const int ld = F.ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto prow = [&](int i) { return i < w ? p + i : F.n + (i - w); };  // panel row -> front row
-  for (int idx = tid; idx < R * w; idx += blockDim.x) {
-    int i = idx % R, j = idx / R;
-    if (i >= j) a[j][i] = (C)A[(int64_t)(p + j) * ld + prow(i)];
+  // entries (er >= ec) of the 32 x 32 lower triangle: columns g and 31 - g
+  // together hold 33 of them
+  C v[DG_E];
+  int er[DG_E], ec[DG_E];
+#pragma unroll
+  for (int u = 0; u < DG_E; ++u) {
+    const int id = tid + DG_T * u, g = id / 33, o = id % 33;
+    const bool first = o < BW - g;
+    ec[u] = first ? g : BW - 1 - g;
+    er[u] = first ? g + o : o - 1;
+    if (g >= BW / 2 || er[u] >= R || ec[u] >= w) ec[u] = -1;
+    v[u] = ec[u] >= 0 ? (C)A[(int64_t)(p + ec[u]) * ld + prow(er[u])] : C(0);
   }
-  if (tid < BW) perm[tid] = tid;
+#pragma unroll
+  for (int u = 0; u < DG_E; ++u)
+    if (ec[u] >= 0 && er[u] == ec[u]) dg[ec[u]] = v[u];
+  for (int idx = tid; idx < BW * LDB; idx += DG_T) (&Ls[0][0])[idx] = C(0);
   if (tid < 2 * BW) dv[tid] = 0.0;
   __syncthreads();
-  if (warp == 0) {
-    __syncwarp();  // reconverge after the lane-dependent staging loop
-    // symmetric swap of candidates x < y (lower storage), rows [0, R)
-    auto swap_xy = [&](int x, int y) {
-      if (x == y) return;
-      if (x > y) { int t = x; x = y; y = t; }
-      int kk = lane;
-      if (kk < R) {
-        C t;
-        if (kk < x) { t = a[kk][x]; a[kk][x] = a[kk][y]; a[kk][y] = t; }
-        else if (kk == x) { t = a[x][x]; a[x][x] = a[y][y]; a[y][y] = t; }
-        else if (kk < y) { t = a[x][kk]; a[x][kk] = a[kk][y]; a[kk][y] = t; }
-        else if (kk > y) { t = a[x][kk]; a[x][kk] = a[y][kk]; a[y][kk] = t; }
+  int mp = lane;  // position of label `lane`
+  auto at = [&](int pos) { return __ffs(__ballot_sync(ALL, mp == pos)) - 1; };  // its label
+  auto swap_pos = [&](int x, int y) {
+    if (mp == x) mp = y;
+    else if (mp == y) mp = x;
+  };
+  // column of label l (every other label's entry with it) into dst
+  auto publish = [&](int l, C* dst) {
+#pragma unroll
+    for (int u = 0; u < DG_E; ++u)
+      if (ec[u] >= 0 && er[u] != ec[u]) {
+        if (ec[u] == l) dst[er[u]] = v[u];
+        else if (er[u] == l) dst[ec[u]] = v[u];
       }
-      if (lane == 0) { int t = perm[x]; perm[x] = perm[y]; perm[y] = t; }
-      __syncwarp();
-    };
-    // 1x1 pivot at s: candidate columns (s, cend), rows [j, R)
-    auto elim1 = [&](int s, int cend) {
-      const C di = C(1) / a[s][s];
-      const int j = lane;
-      if (j > s && j < cend) {
-        const C lj = mul_(a[s][j], di);
-        for (int i = j; i < R; ++i) a[j][i] = fma_(-a[s][i], lj, a[j][i]);
+  };
+  // update of the entries past position `last` with f(entry, later label,
+  // earlier label); the diagonal ones are published
+  auto update = [&](int last, auto f) {
+#pragma unroll
+    for (int u = 0; u < DG_E; ++u) {
+      const int pr = __shfl_sync(ALL, mp, er[u] & 31), pc = __shfl_sync(ALL, mp, ec[u] & 31);
+      if (ec[u] >= 0 && pr > last && pc > last) {
+        const bool rl = pr >= pc;
+        v[u] = f(v[u], rl ? er[u] : ec[u], rl ? ec[u] : er[u]);
+        if (er[u] == ec[u]) dg[ec[u]] = v[u];
       }
-      __syncwarp();
-      if (lane > s && lane < R) a[s][lane] = mul_(a[s][lane], di);
-      if (lane == 0) {
-        a[s][s] = C(1);
+    }
+  };
+  // 1x1 pivot at position s (label l, its column in col1)
+  auto elim1 = [&](int s, int l) {
+    const C di = C(1) / dg[l];
+    update(s, [&](C x, int i, int j) { return fma_(-col1[i], mul_(col1[j], di), x); });
+    if (warp == DG_W - 1) {
+      if (lane < R && mp > s) Ls[s][lane] = mul_(col1[lane], di);
+      if (lane == l) {
+        Ls[s][l] = C(1);
         dv[2 * s] = (double)di;
         dv[2 * s + 1] = 0.0;
       }
-      __syncwarp();
-    };
-    // 2x2 pivot at (s, s+1)
-    auto elim2 = [&](int s, int cend) {
-      const double a11 = a[s][s], a21 = a[s][s + 1], a22 = a[s + 1][s + 1];
-      const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
-      const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
-      const int j = lane;
-      if (j > s + 1 && j < cend) {
-        const double w1 = a[s][j], w2 = a[s + 1][j];
-        const C l1 = (C)fma_(i11, w1, mul_(i12, w2)), l2 = (C)fma_(i12, w1, mul_(i22, w2));
-        for (int i = j; i < R; ++i) a[j][i] = fma_(-a[s + 1][i], l2, fma_(-a[s][i], l1, a[j][i]));
+    }
+  };
+  // 2x2 pivot at positions s, s + 1 (labels l1, l2; columns in col1, col2)
+  auto elim2 = [&](int s, int l1, int l2) {
+    const double a11 = dg[l1], a21 = col1[l2], a22 = dg[l2];
+    const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
+    const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+    update(s + 1, [&](C x, int i, int j) {
+      const double w1 = col1[j], w2 = col2[j];
+      const C x1 = (C)fma_(i11, w1, mul_(i12, w2)), x2 = (C)fma_(i12, w1, mul_(i22, w2));
+      return fma_(-col2[i], x2, fma_(-col1[i], x1, x));
+    });
+    if (warp == DG_W - 1) {
+      if (lane < R && mp > s + 1) {
+        const double w1 = col1[lane], w2 = col2[lane];
+        Ls[s][lane] = (C)fma_(i11, w1, mul_(i12, w2));
+        Ls[s + 1][lane] = (C)fma_(i12, w1, mul_(i22, w2));
       }
-      __syncwarp();
-      if (lane > s + 1 && lane < R) {
-        const double w1 = a[s][lane], w2 = a[s + 1][lane];
-        a[s][lane] = (C)fma_(i11, w1, mul_(i12, w2));
-        a[s + 1][lane] = (C)fma_(i12, w1, mul_(i22, w2));
-      }
-      if (lane == 0) {
-        a[s][s] = C(1);
-        a[s][s + 1] = C(0);
-        a[s + 1][s + 1] = C(1);
+      if (lane == l1) {
+        Ls[s][l1] = C(1);
         dv[2 * s] = i11;
         dv[2 * s + 1] = i12;
         dv[2 * s + 2] = dinf();
         dv[2 * s + 3] = i22;
       }
-      __syncwarp();
-    };
-    // zero pivot at s: column of L is zero
-    auto elim0 = [&](int s) {
-      if (lane >= s && lane < R) a[s][lane] = (lane == s) ? C(1) : C(0);
-      if (lane == 0) {
-        dv[2 * s] = 0.0;
-        dv[2 * s + 1] = 0.0;
-        atomicOr(st.status, ST_ZERO_PIVOT);
-      }
-      __syncwarp();
-    };
-    int s = 0;
-    if (w == BW) {
-      // ---- complete pivoting (block_ldlt)
-      while (s < w) {
-        C best = C(-1);
-        int bi = -1, bj = -1;
-        if (lane >= s && lane < w)
-          for (int i = lane; i < w; ++i) {
-            C v = fabs(a[lane][i]);
-            if (v > best) { best = v; bi = i; bj = lane; }
-          }
-        for (int o = 16; o > 0; o >>= 1) {
-          C ob = __shfl_xor_sync(0xffffffffu, best, o);
-          int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-          if (ob > best || (ob == best && (oj < bj || (oj == bj && oi < bi)))) {
-            best = ob; bi = oi; bj = oj;
-          }
-        }
-        const double amax = best;
-        if (!(amax >= st.small)) {
-          // the rest of the block is (numerically) zero: zero pivots
-          for (int kk = s; kk < w; ++kk) {
-            if (lane >= kk && lane < w) a[kk][lane] = (lane == kk) ? C(1) : C(0);
-            if (lane == 0) { dv[2 * kk] = 0.0; dv[2 * kk + 1] = 0.0; }
-          }
-          if (lane == 0) atomicOr(st.status, st.action ? ST_ZERO_PIVOT : ST_SINGULAR);
-          __syncwarp();
-          s = w;
-          break;
-        }
-        const int t = bi, qq = bj;  // t >= qq
-        bool two = false;
-        int piv = t;
-        if (t != qq) {
-          double dt = fabs((double)a[t][t]), dq = fabs((double)a[qq][qq]);
-          if (fmax(dt, dq) >= mul_(st.u, amax)) piv = (dt >= dq) ? t : qq;
-          else two = true;
-        }
-        if (!two) {
-          swap_xy(s, piv);
-          elim1(s, w);
-          s += 1;
-        } else {
-          swap_xy(s, qq);
-          swap_xy(s + 1, (t == s) ? qq : t);
-          elim2(s, w);
-          s += 2;
+      if (lane == l2) Ls[s + 1][l2] = C(1);
+    }
+  };
+  int s = 0;
+  if (w == BW) {
+    // ---- complete pivoting (block_ldlt)
+    while (s < w) {
+      K key = 0;
+      unsigned tie = ~0u;
+#pragma unroll
+      for (int u = 0; u < DG_E; ++u) {
+        const int pr = __shfl_sync(ALL, mp, er[u] & 31), pc = __shfl_sync(ALL, mp, ec[u] & 31);
+        if (ec[u] >= 0 && pr >= s && pc >= s) {
+          const K ku = mag_key(v[u]);
+          const unsigned tu = min(pr, pc) * BW + max(pr, pc);  // column first, then row
+          if (ku > key || (ku == key && tu < tie)) { key = ku; tie = tu; }
         }
       }
-    } else {
-      // ---- threshold partial pivoting over the w candidates (ldlt_tpp_factor)
-      const double lim = 1.0 / st.u;
-      while (s < w) {
-        int decided = 0, piv = -1, tpiv = -1;
-        for (int c = s; c < w && !decided; ++c) {
-          auto colv = [&](int i, int col) -> double { return i > col ? a[col][i] : a[i][col]; };
-          double v = -1.0;
-          int vi = -1;
-          if (lane >= s && lane < R && lane != c) { v = fabs(colv(lane, c)); vi = lane; }
-          warp_argmax(v, vi);
-          const double amax = fmax(v, 0.0);
-          const int t = vi;
-          const double acc = fabs((double)a[c][c]);
-          if (amax < st.small && acc < st.small) { decided = 3; piv = c; break; }
-          if (acc >= mul_(st.u, amax)) { decided = 1; piv = c; break; }
-          if (t >= 0 && t < w) {
-            double v1 = -1.0, v2 = -1.0;
-            int d1 = -1, d2 = -1;
-            if (lane >= s && lane < R && lane != c && lane != t) {
-              v1 = fabs(colv(lane, c)); d1 = lane;
-              v2 = fabs(colv(lane, t)); d2 = lane;
-            }
-            warp_argmax(v1, d1);
-            warp_argmax(v2, d2);
-            const double ap2 = fmax(v1, 0.0), at2 = fmax(v2, 0.0);
-            const double a11 = a[c][c], a22 = a[t][t], a21 = colv(t, c);
-            const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
-            if (fabs(det) > st.small && isfinite(det)) {
-              const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
-              if (fma_(fabs(i11), ap2, mul_(fabs(i12), at2)) <= lim &&
-                  fma_(fabs(i12), ap2, mul_(fabs(i22), at2)) <= lim) {
-                decided = 2; piv = c; tpiv = t;
-              }
-            }
-          }
-        }
-        if (!decided) break;
-        if (decided == 3) {
-          if (!st.action) {
-            if (lane == 0) atomicOr(st.status, ST_SINGULAR);
-            break;
-          }
-          swap_xy(s, piv);
-          elim0(s);
-          s += 1;
-        } else if (decided == 1) {
-          swap_xy(s, piv);
-          elim1(s, w);
-          s += 1;
-        } else {
-          swap_xy(s, piv);
-          swap_xy(s + 1, (tpiv == s) ? piv : tpiv);
-          elim2(s, w);
-          s += 2;
-        }
+      {
+        const K m = warp_max(key);
+        const unsigned tm = __reduce_min_sync(ALL, key == m ? tie : ~0u);
+        if (lane == 0) { pkey[warp] = m; ptie[warp] = tm; }
+      }
+      __syncthreads();
+      key = pkey[lane & (DG_W - 1)];
+      tie = ptie[lane & (DG_W - 1)];
+      {
+        const K m = warp_max(key);
+        tie = __reduce_min_sync(ALL, key == m ? tie : ~0u);
+        key = m;
+      }
+      const double amax = key_mag(key);
+      if (!(amax >= st.small)) {
+        // the rest of the block is (numerically) zero: zero pivots, whose
+        // columns of L and D are zero
+        if (warp == 0 && mp >= s) Ls[mp][lane] = C(1);
+        if (tid == 0) atomicOr(st.status, st.action ? ST_ZERO_PIVOT : ST_SINGULAR);
+        s = w;
+        break;
+      }
+      const int t = tie % BW, qq = tie / BW;  // t >= qq
+      bool two = false;
+      int piv = t;
+      if (t != qq) {
+        const double dt = fabs((double)dg[at(t)]), dq = fabs((double)dg[at(qq)]);
+        if (fmax(dt, dq) >= mul_(st.u, amax)) piv = (dt >= dq) ? t : qq;
+        else two = true;
+      }
+      if (!two) {
+        const int l = at(piv);
+        swap_pos(s, piv);
+        publish(l, col1);
+        __syncthreads();
+        elim1(s, l);
+        s += 1;
+      } else {
+        const int l1 = at(qq), l2 = at(t);
+        swap_pos(s, qq);
+        swap_pos(s + 1, (t == s) ? qq : t);
+        publish(l1, col1);
+        publish(l2, col2);
+        __syncthreads();
+        elim2(s, l1, l2);
+        s += 2;
       }
     }
-    if (lane == 0) s_nd = s;
+  } else {
+    // ---- threshold partial pivoting over the w candidates (ldlt_tpp_factor)
+    const double lim = 1.0 / st.u;
+    while (s < w) {
+      int decided = 0, piv = -1, tpiv = -1, lc = -1, lt = -1;
+      for (int c = s; c < w && !decided; ++c) {
+        lc = at(c);
+        publish(lc, col1);
+        __syncthreads();
+        const bool in = lane < R && mp >= s && lane != lc;
+        K key = in ? mag_key(col1[lane]) : K(0);
+        K m = warp_max(key);
+        const unsigned tm = __reduce_min_sync(ALL, in && key == m && m ? (unsigned)mp : ~0u);
+        const double amax = fmax(key_mag(m), 0.0), acc = fabs((double)dg[lc]);
+        if (amax < st.small && acc < st.small) { decided = 3; piv = c; break; }
+        if (acc >= mul_(st.u, amax)) { decided = 1; piv = c; break; }
+        if (tm < (unsigned)w) {
+          lt = at(tm);
+          publish(lt, col2);
+          __syncthreads();
+          const bool in2 = in && lane != lt;
+          const double ap2 = fmax(key_mag(warp_max(in2 ? key : K(0))), 0.0);
+          const double at2 = fmax(key_mag(warp_max(in2 ? mag_key(col2[lane]) : K(0))), 0.0);
+          const double a11 = dg[lc], a22 = dg[lt], a21 = col1[lt];
+          const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
+          if (fabs(det) > st.small && isfinite(det)) {
+            const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+            if (fma_(fabs(i11), ap2, mul_(fabs(i12), at2)) <= lim &&
+                fma_(fabs(i12), ap2, mul_(fabs(i22), at2)) <= lim) {
+              decided = 2; piv = c; tpiv = tm;
+              break;
+            }
+          }
+        }
+        __syncthreads();  // the columns are read before the next candidate's
+      }
+      if (!decided) break;
+      if (decided == 3) {
+        if (!st.action) {
+          if (tid == 0) atomicOr(st.status, ST_SINGULAR);
+          break;
+        }
+        swap_pos(s, piv);
+        if (warp == 0 && lane == lc) {
+          Ls[s][lc] = C(1);
+          atomicOr(st.status, ST_ZERO_PIVOT);
+        }
+        s += 1;
+      } else if (decided == 1) {
+        swap_pos(s, piv);
+        elim1(s, lc);
+        s += 1;
+      } else {
+        swap_pos(s, piv);
+        swap_pos(s + 1, (tpiv == s) ? piv : tpiv);
+        elim2(s, lc, lt);
+        s += 2;
+      }
+      __syncthreads();  // the columns are read before the next pivot's
+    }
   }
+  const int nd = s;
+  if (warp == 0) perm[mp] = lane;
   __syncthreads();
-  const int nd = s_nd;
   C* blk = reinterpret_cast<C*>(st.blk) + (int64_t)q * BW * LDB;
-  for (int idx = tid; idx < BW * LDB; idx += blockDim.x) blk[idx] = (&a[0][0])[idx];
+  for (int idx = tid; idx < BW * LDB; idx += DG_T) {
+    const int i = idx % LDB, j = idx / LDB;
+    blk[idx] = i < BW ? Ls[j][perm[i]] : C(0);
+  }
   if (tid < 2 * BW) st.bdinv[q * 2 * BW + tid] = dv[tid];
   if (tid < BW) st.lperm[q * BW + tid] = perm[tid];
   if (tid == 0) {
@@ -308,48 +375,17 @@ __global__ void __launch_bounds__(128) k_app_diag(T* __restrict__ arena, T* __re
   // L of the extra rows (partial block) goes where apply puts rows below
   if (e > 0) {
     T* pan = scratch + F.pan_off;
-    for (int idx = tid; idx < e * nd; idx += blockDim.x) {
+    for (int idx = tid; idx < e * nd; idx += DG_T) {
       int i = w + idx % e, kk = idx / e;
-      pan[(int64_t)kk * F.m + prow(i)] = (T)a[kk][i];
+      pan[(int64_t)kk * F.m + prow(i)] = (T)Ls[kk][i];
     }
   }
-  // apply the block permutation to the rows of the eliminated columns [0, p)
-  // and to the variable list
-  for (int c = warp; c < p; c += blockDim.x / 32) {
-    T v = T(0);
-    if (lane < w) v = A[(int64_t)c * ld + p + perm[lane]];
-    __syncwarp();
-    if (lane < w) A[(int64_t)c * ld + p + lane] = v;
-  }
+  // the block permutation on the variable list
   if (warp == 0) {
     int* var = st.var + F.var_off + p;
-    int v = (lane < w) ? var[perm[lane]] : 0;
+    int vv = (lane < w) ? var[perm[lane]] : 0;
     __syncwarp();
-    if (lane < w) var[lane] = v;
-  }
-}
-
-// apply D^-1 to the first nd entries of a solved row (apply_pivot OP_N)
-template <typename C>
-__device__ __forceinline__ void apply_dinv(C* x, const double* dv, int nd, double small) {
-#pragma unroll
-  for (int k = 0; k < BW;) {
-    if (k >= nd) break;
-    if (k + 1 < nd && isinf(dv[2 * k + 2])) {
-      const double x1 = x[k], x2 = x[k + 1];
-      x[k] = (C)fma_(dv[2 * k], x1, mul_(dv[2 * k + 1], x2));
-      x[k + 1] = (C)fma_(dv[2 * k + 1], x1, mul_(dv[2 * k + 3], x2));
-      k += 2;
-    } else {
-      const double d = dv[2 * k];
-      if (d == 0.0) {
-        const double v = x[k];
-        x[k] = (C)((fabs(v) < small) ? 0.0 : dinf() * v);
-      } else {
-        x[k] = mul_(x[k], (C)d);
-      }
-      k += 1;
-    }
+    if (lane < w) var[lane] = vv;
   }
 }
 
@@ -361,59 +397,121 @@ struct BelowRows {
   __device__ int row(int ci) const { return ci < n - lo ? lo + ci : n + e + (ci - (n - lo)); }
 };
 
+// Pivot kinds of a diagonal block's first `cnt` columns (D^-1 in dv)
+enum { PV_ONE, PV_FIRST, PV_SECOND, PV_ZERO };
+__device__ __forceinline__ int pivot_kind(const double* dv, int k, int cnt) {
+  if (k > 0 && isinf(dv[2 * k])) return PV_SECOND;
+  if (k + 1 < cnt && isinf(dv[2 * k + 2])) return PV_FIRST;
+  return dv[2 * k] == 0.0 ? PV_ZERO : PV_ONE;
+}
+// |x| > lim in integer or FP32 arithmetic (false for NaN): same outcome as the
+// FP64 comparison, off the FP64 pipe.  lim > 0.
+__device__ __forceinline__ bool above(float x, double lim) {
+  return fabsf(x) > __double2float_rd(lim);
+}
+__device__ __forceinline__ bool above(double x, double lim) {
+  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+  return b > __double_as_longlong(lim) && b <= 0x7ff0000000000000ll;
+}
+
 // ---------------------------------------------------------------------------
 // Rows below the diagonal block: x = a P L_kk^-T D^-1 over the ndiag pivots,
 // into the apply panel; the least pivot with |x| > 1/u lowers npass_raw.
+// One row per thread with its 32 values in registers, every load in flight at
+// once, L read from shared memory in 16-byte broadcasts (with the row in shared
+// memory a multiply-add took two shared loads and a store).  FP64 is bound by
+// the FP64 pipe (560 multiply-adds per row at 2 per clock and SM, a warp
+// instruction every 64 clocks), so its rows are spread in CTAs of one warp.
+// Per launch on the shifted 48^3 (FP32) and the 14^3 saddle point (FP64): 42
+// and 50 us before, 14 and 31 us now.
 template <typename T>
-__global__ void __launch_bounds__(LDLT_RT) k_app_apply(const T* __restrict__ arena,
-                                                      T* __restrict__ scratch,
-                                                      const LdltFront* __restrict__ fr,
-                                                      const CtaMap* __restrict__ cm,
-                                                      LdltStep st) {
+__global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict__ arena,
+                                                             T* __restrict__ scratch,
+                                                             const LdltFront* __restrict__ fr,
+                                                             const CtaMap* __restrict__ cm,
+                                                             LdltStep st) {
   using C = T;
-  __shared__ C L[BW][LDB];
+  constexpr int RT = AppRows<T>::v, V = 16 / (int)sizeof(C), LP = BW + V;
+  using Vec = typename std::conditional<sizeof(C) == 4, float4, double2>::type;
+  __shared__ __align__(16) C L[BW][LP];  // zero past the ndiag pivots
   __shared__ double dv[2 * BW];
-  __shared__ int perm[BW];
-  __shared__ C xs[BW][LDLT_RT + 1];
+  __shared__ int perm[BW], kind[BW];
   __shared__ int fail;
   const CtaMap c = cm[blockIdx.x];
   const LdltFront F = fr[c.f];
   const int q = F.fidx, w = block_width(F, st.k), e = extra_rows(F, w);
   const int p = st.p_cur[q], nd = st.ndiag[q];
+  if (nd == 0) return;
   const T* A = arena + F.off;
-  const int ld = F.ld, tid = threadIdx.x;
+  const int64_t ld = F.ld, pm = F.m;
+  const int tid = threadIdx.x;
   const C* blk = reinterpret_cast<const C*>(st.blk) + (int64_t)q * BW * LDB;
-  for (int idx = tid; idx < BW * LDB; idx += blockDim.x) (&L[0][0])[idx] = blk[idx];
-  if (tid < 2 * BW) dv[tid] = st.bdinv[q * 2 * BW + tid];
+  for (int idx = tid; idx < BW * BW; idx += RT) {
+    const int j = idx / BW, k = idx % BW;
+    L[j][k] = (j < nd && k < nd) ? blk[j * LDB + k] : C(0);
+  }
+  for (int k = tid; k < 2 * BW; k += RT) dv[k] = st.bdinv[q * 2 * BW + k];
   if (tid < BW) perm[tid] = st.lperm[q * BW + tid];
   if (tid == 0) fail = nd;
+  __syncthreads();
+  if (tid < BW) kind[tid] = pivot_kind(dv, tid, nd);
   __syncthreads();
   const BelowRows br{p + w, F.n, e, F.m};
   const int nrow = br.count();
   const double lim = 1.0 / st.u;
   T* pan = scratch + F.pan_off;
-  for (int t0 = c.local * LDLT_RT; t0 < nrow; t0 += c.count * LDLT_RT) {
+  for (int t0 = c.local * RT; t0 < nrow; t0 += c.count * RT) {
     const int ci = t0 + tid;
     if (ci < nrow) {
       const int r = br.row(ci);
-      for (int k = 0; k < nd; ++k) xs[k][tid] = (C)A[(int64_t)(p + perm[k]) * ld + r];
-      // x L^T = a  (unit lower L)
-      for (int j = 0; j < nd; ++j) {
-        const C xj = xs[j][tid];
-        for (int k = j + 1; k < nd; ++k) xs[k][tid] = fma_(-xj, L[j][k], xs[k][tid]);
-      }
       C x[BW];
 #pragma unroll
-      for (int k = 0; k < BW; ++k) x[k] = (k < nd) ? xs[k][tid] : C(0);
-      apply_dinv(x, dv, nd, st.small);
+      for (int k = 0; k < BW; ++k) x[k] = k < nd ? (C)A[(p + perm[k]) * ld + r] : C(0);
+      // x L^T = a  (unit lower L)
+#pragma unroll
+      for (int j = 0; j < BW - 1; ++j) {
+        if (j >= nd) break;
+        const C xj = -x[j];
+#pragma unroll
+        for (int kv = (j + 1) / V * V; kv < BW; kv += V) {
+          const Vec lv = *reinterpret_cast<const Vec*>(&L[j][kv]);
+          if constexpr (V == 4) {
+            if (kv > j) x[kv] = fma_(xj, lv.x, x[kv]);
+            if (kv + 1 > j) x[kv + 1] = fma_(xj, lv.y, x[kv + 1]);
+            if (kv + 2 > j) x[kv + 2] = fma_(xj, lv.z, x[kv + 2]);
+            x[kv + 3] = fma_(xj, lv.w, x[kv + 3]);
+          } else {
+            if (kv > j) x[kv] = fma_(xj, lv.x, x[kv]);
+            x[kv + 1] = fma_(xj, lv.y, x[kv + 1]);
+          }
+        }
+      }
+      // times D^-1 (apply_pivot OP_N)
+#pragma unroll
+      for (int k = 0; k < BW; ++k) {
+        if (k >= nd) break;
+        const int kd = kind[k];
+        if (kd == PV_ONE) {
+          x[k] = mul_(x[k], (C)dv[2 * k]);
+        } else if (kd == PV_FIRST) {
+          if (k + 1 < BW) {
+            const double x1 = x[k], x2 = x[k + 1];
+            x[k] = (C)fma_(dv[2 * k], x1, mul_(dv[2 * k + 1], x2));
+            x[k + 1] = (C)fma_(dv[2 * k + 1], x1, mul_(dv[2 * k + 3], x2));
+          }
+        } else if (kd == PV_ZERO) {
+          const double v = x[k];
+          x[k] = (C)((fabs(v) < st.small) ? 0.0 : dinf() * v);
+        }
+      }
       int first = nd;
 #pragma unroll
       for (int k = BW - 1; k >= 0; --k)
-        if (k < nd && fabs((double)x[k]) > lim) first = k;
+        if (k < nd && above(x[k], lim)) first = k;
       if (first < nd) atomicMin(&fail, first);
 #pragma unroll
       for (int k = 0; k < BW; ++k)
-        if (k < nd) pan[(int64_t)k * F.m + r] = (T)x[k];
+        if (k < nd) pan[k * pm + r] = (T)x[k];
     }
   }
   __syncthreads();
@@ -425,95 +523,124 @@ __global__ void __launch_bounds__(LDLT_RT) k_app_apply(const T* __restrict__ are
 // p + npass on, for the trailing update), failed columns get back their
 // values from before the step in the block's symmetric order (the front
 // itself is the backup: nothing before the commit writes it in the block's
-// columns).  The CTA with local index 0 stores D and the state.
+// columns).  The block's permutation is applied to its rows of the eliminated
+// columns.  The CTA with local index 0 stores D and the state.  One row per
+// thread, its 32 values in registers: 35 -> 16 us per launch on the shifted
+// 48^3 (FP32), 38 -> 22 us on the 14^3 saddle point (FP64; half of it the 32
+// FP64 divisions of a row).
 template <typename T>
-__global__ void __launch_bounds__(LDLT_RT) k_app_commit(T* __restrict__ arena,
-                                                       T* __restrict__ scratch,
-                                                       const LdltFront* __restrict__ fr,
-                                                       const CtaMap* __restrict__ cm,
-                                                       LdltStep st) {
+__global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ arena,
+                                                              T* __restrict__ scratch,
+                                                              const LdltFront* __restrict__ fr,
+                                                              const CtaMap* __restrict__ cm,
+                                                              LdltStep st) {
   using C = T;
+  constexpr int RT = AppRows<T>::v;
   __shared__ C L[BW][LDB];
   __shared__ double dv[2 * BW];
-  __shared__ int perm[BW];
-  __shared__ C orig[BW][LDLT_RT + 1];
+  __shared__ double dca[BW], dcb[BW];  // D of a 2x2 pair's two columns
+  __shared__ int perm[BW], kind[BW];
   const CtaMap c = cm[blockIdx.x];
   const LdltFront F = fr[c.f];
   const int q = F.fidx, w = block_width(F, st.k);
   const int p = st.p_cur[q], nd = st.ndiag[q];
   T* A = arena + F.off;
-  const int ld = F.ld, tid = threadIdx.x;
+  const int64_t ld = F.ld, pm = F.m;
+  const int tid = threadIdx.x;
   const C* blk = reinterpret_cast<const C*>(st.blk) + (int64_t)q * BW * LDB;
-  for (int idx = tid; idx < BW * LDB; idx += blockDim.x) (&L[0][0])[idx] = blk[idx];
-  if (tid < 2 * BW) dv[tid] = st.bdinv[q * 2 * BW + tid];
+  // only the tile of the block's own rows reads L (the rest come from apply)
+  if (c.local == 0)
+    for (int idx = tid; idx < BW * LDB; idx += RT) (&L[0][0])[idx] = blk[idx];
+  for (int k = tid; k < 2 * BW; k += RT) dv[k] = st.bdinv[q * 2 * BW + k];
   if (tid < BW) perm[tid] = st.lperm[q * BW + tid];
   __syncthreads();
+  // the block's permutation on its rows of the eliminated columns [0, p),
+  // shared by the front's CTAs, PU columns in flight per warp (one CTA with
+  // one column in flight took most of the diagonal kernel at the top fronts)
+  {
+    constexpr int PU = 4;
+    const int lane = tid & 31, pl = perm[lane];
+    if (__any_sync(0xffffffffu, lane < w && pl != lane))
+      for (int c0 = (c.local * (RT / 32) + (tid >> 5)) * PU; c0 < p;
+           c0 += c.count * (RT / 32) * PU) {
+        T v[PU];
+#pragma unroll
+        for (int u = 0; u < PU; ++u)
+          v[u] = (lane < w && c0 + u < p) ? A[(c0 + u) * ld + p + pl] : T(0);
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < PU; ++u)
+          if (lane < w && c0 + u < p) A[(c0 + u) * ld + p + lane] = v[u];
+      }
+  }
   // Column::adjust: drop the first half of a 2x2 pivot split by the test
   int np = min(st.npass_raw[q], nd);
   if (np > 0 && isfinite(dv[2 * (np - 1)]) && dv[2 * (np - 1) + 1] != 0.0) np--;
+  if (tid < BW) {
+    const int kd = pivot_kind(dv, tid, np);
+    kind[tid] = kd;
+    if (kd == PV_FIRST || (kd == PV_SECOND && tid < np)) {
+      const int k = kd == PV_FIRST ? tid : tid - 1;
+      const double a = dv[2 * k], b = dv[2 * k + 1], cc = dv[2 * k + 3];
+      const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
+      dca[tid] = kd == PV_FIRST ? cc / det : -b / det;
+      dcb[tid] = kd == PV_FIRST ? -b / det : a / det;
+    }
+  }
+  __syncthreads();
   const T* pan = scratch + F.pan_off;
   T* ldp = scratch + F.ldp_off;
-  const int ldp_ = F.m;
-  for (int t0 = p + c.local * LDLT_RT; t0 < F.m; t0 += c.count * LDLT_RT) {
+  for (int t0 = p + c.local * RT; t0 < F.m; t0 += c.count * RT) {
     const int r = t0 + tid;
     const bool in_blk = r < p + w;
     const int i = r - p;
-    // phase 1: the values failed columns keep (in-block rows all belong to
-    // the tile that starts at p, so no other CTA writes what this one reads)
-    if (r < F.m) {
-      for (int k = np; k < w; ++k) {
-        C v = C(0);
-        if (in_blk) {
-          if (i >= k) {
-            int ai = perm[i], ak = perm[k];
-            int rr = max(ai, ak), cc = min(ai, ak);
-            v = (C)A[(int64_t)(p + cc) * ld + p + rr];
-          }
-        } else {
-          v = (C)A[(int64_t)(p + perm[k]) * ld + r];
-        }
-        orig[k][tid] = v;
-      }
-    }
-    __syncthreads();
-    if (r < F.m) {
-      C l[BW];
+    // phase 1: L of the passed columns, the values failed columns keep
+    // (in-block rows all belong to the tile that starts at p, so no other
+    // CTA writes what this one reads)
+    C l[BW];
+    if (r < F.m && !in_blk) {
+#pragma unroll
+      for (int k = 0; k < BW; ++k)
+        l[k] = k < np ? (C)pan[k * pm + r] : k < w ? (C)A[(p + perm[k]) * ld + r] : C(0);
+    } else if (r < F.m) {
 #pragma unroll
       for (int k = 0; k < BW; ++k) {
         C v = C(0);
         if (k < np) {
-          if (in_blk) v = (i > k) ? L[k][i] : (i == k ? C(1) : C(0));
-          else v = (C)pan[(int64_t)k * ldp_ + r];
+          v = (i > k) ? L[k][i] : (i == k ? C(1) : C(0));
+        } else if (k < w && i >= k) {
+          const int ai = perm[i], ak = perm[k];
+          v = (C)A[(p + min(ai, ak)) * ld + p + max(ai, ak)];
         }
         l[k] = v;
       }
-      for (int k = 0; k < w; ++k) {
-        if (in_blk && i < k) continue;
-        C v = (k < np) ? l[k] : orig[k][tid];
-        A[(int64_t)(p + k) * ld + r] = (T)v;
-      }
+    }
+    __syncthreads();
+    if (r < F.m) {
+#pragma unroll
+      for (int k = 0; k < BW; ++k)
+        if (k < w && !(in_blk && i < k)) A[(p + k) * ld + r] = (T)l[k];
       if (r >= p + np) {
-        for (int k = 0; k < np;) {
-          if (k + 1 < np && isinf(dv[2 * k + 2])) {
-            const double a = dv[2 * k], b = dv[2 * k + 1], cc = dv[2 * k + 3];
-            const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
-            const double d11 = cc / det, d21 = -b / det, d22 = a / det;
-            const double l0 = l[k], l1 = l[k + 1];
-            ldp[(int64_t)k * ldp_ + r] = (T)fma_(l0, d11, mul_(l1, d21));
-            ldp[(int64_t)(k + 1) * ldp_ + r] = (T)fma_(l0, d21, mul_(l1, d22));
-            k += 2;
-          } else {
-            const double d = dv[2 * k];
-            ldp[(int64_t)k * ldp_ + r] = (T)((d == 0.0) ? C(0) : l[k] / (C)d);
-            k += 1;
+#pragma unroll
+        for (int k = 0; k < BW; ++k) {
+          if (k >= np) break;
+          const int kd = kind[k];
+          C v = C(0);
+          if (kd == PV_ONE) {
+            v = l[k] / (C)dv[2 * k];
+          } else if (kd == PV_FIRST) {
+            if (k + 1 < BW) v = (C)fma_((double)l[k], dca[k], mul_((double)l[k + 1], dcb[k]));
+          } else if (kd == PV_SECOND) {
+            if (k > 0) v = (C)fma_((double)l[k - 1], dca[k], mul_((double)l[k], dcb[k]));
           }
+          ldp[k * pm + r] = (T)v;
         }
       }
     }
     __syncthreads();
   }
   if (c.local == 0) {
-    if (tid < 2 * np) st.dall[F.d_off + 2 * p + tid] = dv[tid];
+    for (int k = tid; k < 2 * np; k += RT) st.dall[F.d_off + 2 * p + k] = dv[k];
     if (tid == 0) {
       const int nf = st.nf_cur[q];
       st.npass[q] = np;
@@ -878,17 +1005,17 @@ __global__ void k_solve_diag(const FrontDesc* __restrict__ fr, const int* __rest
 template <typename T>
 void launch_app_diag(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                      LdltStep st, cudaStream_t s) {
-  if (ncta > 0) k_app_diag<T><<<ncta, 128, 0, s>>>(arena, scratch, fr, cm, st);
+  if (ncta > 0) k_app_diag<T><<<ncta, DG_T, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_apply(const T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                       LdltStep st, cudaStream_t s) {
-  if (ncta > 0) k_app_apply<T><<<ncta, LDLT_RT, 0, s>>>(arena, scratch, fr, cm, st);
+  if (ncta > 0) k_app_apply<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_commit(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                        LdltStep st, cudaStream_t s) {
-  if (ncta > 0) k_app_commit<T><<<ncta, LDLT_RT, 0, s>>>(arena, scratch, fr, cm, st);
+  if (ncta > 0) k_app_commit<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_move(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
@@ -901,7 +1028,7 @@ template <typename T>
 void launch_app_update(T* arena, const T* scratch, const LdltFront* fr, const CtaMap* cm,
                        int ncta, LdltStep st, cudaStream_t s) {
   if (ncta > 0)
-    k_app_update<T, Tiles<T>::TM, 16><<<ncta, 256, 0, s>>>(arena, scratch, fr, cm, st);
+    k_app_update<T, AppTile<T>::v, 16><<<ncta, 256, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_ldlt_tpp(T* arena, const LdltFront* fr, int nf, LdltStep st, double u_eff,

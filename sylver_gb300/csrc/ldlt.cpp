@@ -400,11 +400,14 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
           const int w = std::min(LDLT_BW, f.n - LDLT_BW * k);
           const int p0 = LDLT_BW * k;  // block start when nothing failed so far
           int cnt = 1;
-          if (kind == 1) cnt = ceil_div(std::max(f.m - p0 - w, 1), LDLT_RT);
-          if (kind == 2) cnt = ceil_div(f.m - p0, LDLT_RT);
+          if (kind == 1) cnt = ceil_div(std::max(f.m - p0 - w, 1), AppRows<T>::v);
+          // commit: row tiles, and at least one CTA per 64 eliminated columns, whose
+          // rows in the block it permutes
+          if (kind == 2) cnt = std::max(ceil_div(f.m - p0, AppRows<T>::v), ceil_div(p0, 64));
           if (kind == 3) {
             const int o = std::min(p0 + w, f.n - 1);
-            const int R = ceil_div(f.m - o, TM), C = ceil_div(f.n - o, TM);
+            constexpr int AT = AppTile<T>::v;
+            const int R = ceil_div(f.m - o, AT), C = ceil_div(f.n - o, AT);
             cnt = C * R - C * (C - 1) / 2;
           }
           if (kind == 4) cnt = ceil_div(f.n, 8);
