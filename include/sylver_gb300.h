@@ -323,6 +323,12 @@ int sylver_gb300_profile_solve(void* fkeep, int nrhs, double* ms, long* launches
  * update on a synthetic rows x k panel and report max|C - C_ref| / max|C_ref|
  * against an FP64 host product.  Returns 0 or a reference flag. */
 int sylver_gb300_tc_selfcheck(int rows, int k, double* max_rel_err);
+/* Self-check of the FP64 tensor-core update: entries spread over 2^spread (and
+ * rows scaled by powers of two when spread > 0), an infinity in row `special`
+ * (none if < 0).  *max_err: largest entry error over the product of the two
+ * row norms, in units of 2^-53; infinite if the infinity is not confined to
+ * NaNs in its row and column. */
+int sylver_gb300_tc64_selfcheck(int rows, int k, int spread, int special, double* max_err);
 
 /* Diagnostic: the bounded wait of the dataflow solve sweep on a synthetic
  * one-task sweep.  starve != 0: the task waits on a counter nothing sets, so

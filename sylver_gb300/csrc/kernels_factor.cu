@@ -479,9 +479,10 @@ void prepare_factor_kernels() {
   constexpr int SM = Tiles<T>::SMALL_M;
   SG_CUDA(cudaFuncSetAttribute(k_small_chol<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(sizeof(T) * SM * (SM + 1))));
-  SG_CUDA(cudaFuncSetAttribute(k_panel_trsm<T, Tiles<T>::NB, Tiles<T>::RT>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)panel_smem<T>()));
+  if constexpr (std::is_same<T, float>::value)
+    SG_CUDA(cudaFuncSetAttribute(k_panel_trsm<T, Tiles<T>::NB, Tiles<T>::RT>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)panel_smem<T>()));
 }
 
 template <typename T>
@@ -527,11 +528,12 @@ void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, cudaStr
                                    const int*, const int64_t*, const int*, const EaItem*,   \
                                    const ChildDesc*, const int*, cudaStream_t);             \
   template void launch_small_chol<T>(T*, const SmallTask*, int, int, unsigned*, cudaStream_t); \
-  template void launch_diag_chol<T>(T*, const PanelTask*, int, unsigned*, cudaStream_t);     \
-  template void launch_panel_trsm<T>(T*, const PanelTask*, int, cudaStream_t);               \
   template void launch_update<T>(T*, const T*, const UpdTask*, int, cudaStream_t);
 SG_INST(float)
 SG_INST(double)
 #undef SG_INST
+// panel steps of the FP32 SIMT path (FP64 fronts: kernels_panel64.cu)
+template void launch_diag_chol<float>(float*, const PanelTask*, int, unsigned*, cudaStream_t);
+template void launch_panel_trsm<float>(float*, const PanelTask*, int, cudaStream_t);
 
 }  // namespace sylver_gb300

@@ -33,11 +33,8 @@
 // tile.
 // Every mbarrier wait is bounded: on timeout the CTA records an error bit,
 // skips the epilogue, waits (bounded) for its own copies and frees TMEM.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
-#include "device.hpp"
 #include "tc.hpp"
+#include "tc_ptx.cuh"
 
 namespace sylver_gb300 {
 
@@ -48,74 +45,6 @@ constexpr int TC_STAGES = 2;
 constexpr int TC_PLANES = 3;                        // BF16 parts of an operand
 constexpr int TILE_BYTES = TC_M * TC_KC * 2;        // 16 KiB per operand tile
 constexpr int STAGE_BYTES = 2 * TC_PLANES * TILE_BYTES;  // A0 A1 A2 B0 B1 B2
-constexpr long WAIT_LIMIT = 1L << 24;               // try_wait polls before giving up
-
-__device__ __forceinline__ uint32_t su32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(su32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// bounded wait (poll count and one second of wall time); false, with the
-// error bit set, on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, unsigned* err) {
-  const uint64_t t0 = global_ns();
-  for (long it = 0; it < WAIT_LIMIT; ++it) {
-    if (mbar_try(b, parity)) return true;
-    if ((it & 255) == 255 && global_ns() - t0 > 1000000000ull) break;
-  }
-  atomicOr(err, ST_TIMEOUT);
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(su32(dst)),
-      "l"((uint64_t)map), "r"(x), "r"(y), "r"(su32(bar))
-      : "memory");
-}
-
-// K-major, 128-byte swizzle shared-memory matrix descriptor (tcgen05 format:
-// start >> 4 in bits 0-13, leading byte offset >> 4 in 16-29 (unused for a
-// swizzled K-major tile), stride byte offset >> 4 in 32-45 = 1024 B between
-// 8-row groups, version 1 in bits 46-47, swizzle mode 2 (128 B) in 61-63).
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 
 // instruction descriptor (kind::f16): D f32 (bits 4-5 = 1), A and B bf16
 // (bits 7-9 and 10-12 = 1), both K-major, N >> 3 in bits 17-22, M >> 4 in
@@ -123,45 +52,6 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
 __host__ __device__ constexpr uint32_t bf16_idesc() {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_N >> 3) << 17) |
          ((uint32_t)(TC_M >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t ad, uint64_t bd,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          su32(bar))
-      : "memory");
-}
-
-template <int N>
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[N]);
-
-template <>
-__device__ __forceinline__ void tmem_ld32<32>(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-        "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-        "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // ---------------------------------------------------------------------------
@@ -172,27 +62,6 @@ constexpr int TC_EPI_COLS = TC_N / 2;            // columns per epilogue thread
 constexpr int TC_THREADS = 32 * (TC_EPI_WARP0 + TC_EPI_WARPS);
 constexpr int TC_NACC = 4;                       // accumulators in the TMEM ring
 constexpr int TC_TMEM_COLS = TC_NACC * TC_N;     // all 512 TMEM columns
-
-// arrive on an mbarrier (one arrival)
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
-}
-
-// bounded wait that also gives up once another role has aborted
-__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* b, uint32_t parity, unsigned* err,
-                                                   volatile int* abort_flag) {
-  const uint64_t t0 = global_ns();
-  for (long it = 0; it < WAIT_LIMIT; ++it) {
-    if (mbar_try(b, parity)) return true;
-    if ((it & 255) == 255) {
-      if (*abort_flag) return false;
-      if (global_ns() - t0 > 1000000000ull) break;
-    }
-  }
-  atomicOr(err, ST_TIMEOUT);
-  *abort_flag = 1;
-  return false;
-}
 
 // Persistent: CTA b processes tiles b, b + gridDim.x, ...
 //   warp 0 lane 0 : TMA producer over a TC_STAGES ring shared by all tiles,
@@ -358,12 +227,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < TC_EPI_COLS / 32; ++c) {
-          float v[32];
-          tmem_ld32<32>(tmem + ((uint32_t)(q * 32) << 16) +
+          uint32_t v[32];
+          tmem_ld32_async(tmem + ((uint32_t)(q * 32) << 16) +
                             (uint32_t)(a * TC_N + h * TC_EPI_COLS + c * 32),
-                        v);
+                          v);
+          tmem_ld_wait(v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) cv[c * 32 + j] -= v[j];
+          for (int j = 0; j < 32; ++j) cv[c * 32 + j] -= __uint_as_float(v[j]);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -434,18 +304,6 @@ __global__ void __launch_bounds__(256) k_split_t(const float* __restrict__ arena
     planes[pstride + o] = b1;
     planes[2 * pstride + o] = b2;
   }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    cudaDriverEntryPointQueryResult q;
-    void* p = nullptr;
-    SG_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q));
-    if (q != cudaDriverEntryPointSuccess || !p) throw CudaError("cuTensorMapEncodeTiled missing");
-    fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
 }
 
 }  // namespace

@@ -1,0 +1,467 @@
+// Tensor-core Schur-complement update for FP64 fronts: C -= A B^T with FP64
+// accuracy on the BF16 tensor cores (tcgen05, kind::f16).
+//
+// GB300 runs two FP64 multiply-adds per clock and SM; its BF16 tensor cores
+// run about 4000.  Every operand row (the K entries of one front row) is
+// written as x = 2^(e - 62) F with a power of two 2^e >= the row's 2-norm and
+// F a 63-bit integer (rounded to nearest), and F is cut into seven signed
+// digits of nine bits, d1 .. d7, |d| <= 256, exact in BF16 (an error-free
+// splitting after Ozaki, Ogita, Oishi and Rump, "Error-free transformations
+// of matrix multiplication by using fast routines of matrix multiplication
+// and its applications", 2012).  The 28 digit products with index sum
+// s = p + q <= 8 are formed on the tensor cores, one FP32 accumulator per s and
+// 64 columns of k: its terms are integers and their sums stay below 2^24, so
+// nothing is rounded there (s = 7 and 8 can pass 2^24 when nearly all digits
+// sit at +-256; what is lost then is below 2^-60 of the norms).  The epilogue converts each accumulator to an
+// integer and adds it, shifted by 62 - (9 s - 2) bits, to a 64-bit fixed-point
+// sum in units of 2^(e_i + e_j - 62); the row norms bound that sum by 2^62
+// (Cauchy-Schwarz).  The dropped products, the rounding of F and of the sum
+// are each below 2^-62 of the product of the two row norms, against
+// 2^-53 per term of an FP64 sum; C itself is updated by one FP64 subtraction.
+//
+// A row with an infinity or NaN gets a scale exponent that turns every entry
+// it touches into NaN, as the FP64 products would.
+#include "digits.cuh"
+#include "tc.hpp"
+#include "tc_ptx.cuh"
+
+namespace sylver_gb300 {
+
+namespace {
+
+constexpr int OT = 128, ON = 64;                   // tile rows and columns
+constexpr int OZ_STAGES = 2;
+constexpr int OZ_A_TILE = OT * OZ_KC * 2;          // one digit plane of an operand tile: 8, 4 KiB
+constexpr int OZ_B_TILE = ON * OZ_KC * 2;
+constexpr int OZ_A_BYTES = OZ_DIGITS * OZ_A_TILE;
+constexpr int OZ_B_BYTES = OZ_DIGITS * OZ_B_TILE;
+constexpr int OZ_STAGE_BYTES = OZ_A_BYTES + OZ_B_BYTES;  // 84 KiB
+constexpr int OZ_GROUPS = OZ_DIGITS;               // s = 2 .. 8
+constexpr int OZ_DRAIN = 2;                        // k chunks summed in an accumulator
+constexpr int OZ_EPI_WARP0 = 2;
+constexpr int OZ_EPI_WARPS = 8;
+constexpr int OZ_THREADS = 32 * (OZ_EPI_WARP0 + OZ_EPI_WARPS);
+constexpr int OZ_TMEM_COLS = 512;                  // seven accumulators of 64 columns
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y,
+                                            int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(su32(dst)),
+      "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(su32(bar))
+      : "memory");
+}
+
+// K-major, 64-byte swizzle descriptor: 512 B between 8-row groups, swizzle
+// mode 4 (64 B); the other fields as in sw128_desc.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)4 << 61;
+  return d;
+}
+
+// kind::f16, FP32 accumulator, BF16 operands, both K-major, 128 x n
+__device__ __forceinline__ uint32_t oz_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(OT >> 4) << 24);
+}
+
+// acc 2^(e - 62), |e| <= OZ_EXP_SAFE, rounded to nearest in integer arithmetic
+// (conversions and FP64 multiplies run at two per clock and SM)
+constexpr int OZ_EXP_SAFE = 900;
+__device__ __forceinline__ double fixed_to_double(long long acc, int e) {
+  const unsigned long long sgn = (unsigned long long)acc & 0x8000000000000000ull;
+  unsigned long long u = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
+  const int lz = __clzll((long long)u);
+  u <<= lz & 63;
+  const unsigned long long m = (u >> 11) + ((u >> 10) & 1);
+  // biased exponent of the leading bit: 1024 + e - lz; m carries its low bit
+  const unsigned long long b = sgn | (((unsigned long long)(1023 + e - lz) << 52) + m);
+  return __longlong_as_double(u ? (long long)b : 0ll);
+}
+
+// 2^(e - clamp(e)) for row and column exponents outside the safe range; NaN
+// where a row or column had a non-finite entry
+__device__ __noinline__ double extreme_scale(int e) {
+  if (e > OZ_NONFINITE / 2) return __longlong_as_double(0x7ff8000000000000ll);
+  const int r = e - max(-OZ_EXP_SAFE, min(OZ_EXP_SAFE, e));
+  return __longlong_as_double((long long)(1023 + max(-1000, min(1000, r))) << 52);
+}
+
+// fixed-point sum += G * 2^(62 - (9 s - 2)) for group s = G + 2
+template <int G>
+__device__ __forceinline__ void add_group(long long& acc, int v) {
+  constexpr int SH = 46 - 9 * G;  // 46, 37, 28, 19, 10, 1, -8
+  if constexpr (SH >= 32) {
+    const unsigned hi = (unsigned)((unsigned long long)acc >> 32) + ((unsigned)v << (SH - 32));
+    acc = (long long)(((unsigned long long)hi << 32) | (unsigned)acc);
+  } else if constexpr (SH >= 0) {
+    acc += (long long)v * (long long)(1 << SH);
+  } else {
+    acc += (long long)((v + (1 << (-SH - 1))) >> (-SH));
+  }
+}
+
+// Persistent: CTA b processes tiles b, b + gridDim.x, ...
+//   warp 0 lane 0 : TMA producer (one 3D load of all seven digit tiles per
+//                   operand and 32-wide k chunk),
+//   warp 1 lane 0 : MMA issuer; the seven groups have an accumulator each,
+//                   which sums two k chunks before the epilogue takes it; group
+//                   after group, so that its reads overlap the MMAs of the
+//                   other groups; tiles narrower than 64 columns take narrower
+//                   MMAs,
+//   warps 2..9    : epilogue; each thread keeps the fixed-point sums of one
+//                   row and 32 columns in registers and reads the next group's
+//                   accumulator while it adds the current one.
+// Seven accumulators fill the tensor memory at 64 columns; with 128 columns
+// and four accumulators in turn each k chunk had to be drained by itself, and the
+// float-to-integer conversions (16 per clock and SM) alone took as long as the
+// MMAs.
+__global__ void __launch_bounds__(OZ_THREADS, 1)
+    k_update_tc64(const __grid_constant__ CUtensorMap mapa,
+                  const __grid_constant__ CUtensorMap mapb, double* __restrict__ arena,
+                  const int* __restrict__ sexp, const TcTask* __restrict__ tasks, int ntask,
+                  unsigned* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t full[OZ_STAGES], empty[OZ_STAGES], acc_full[OZ_GROUPS],
+      acc_empty[OZ_GROUPS], done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  volatile int* abortp = &abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < OZ_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < OZ_GROUPS; ++a) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], OZ_EPI_WARPS);
+    }
+    mbar_init(&done, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     su32(&tmem_slot)),
+                 "r"(OZ_TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+
+  int issued = 0;  // TMA chunks issued by the producer
+  if (warp == 0) {
+    if (lane == 0) {
+      int g = 0;
+      for (int ti = blockIdx.x; ti < ntask && !*abortp; ti += gridDim.x) {
+        const TcTask t = tasks[ti];
+        bool ok = true;
+        for (int kc = 0; kc < t.nk; ++kc, ++g) {
+          const int s = g % OZ_STAGES;
+          if (g >= OZ_STAGES &&
+              !mbar_wait_or_abort(&empty[s], ((g / OZ_STAGES) - 1) & 1, err, abortp)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = smem + s * OZ_STAGE_BYTES;
+          mbar_expect_tx(&full[s], OZ_STAGE_BYTES);
+          const int x = (t.kc0 + kc) * OZ_KC;
+          tma_load_3d(st, &mapa, x, t.a_row, 0, &full[s]);
+          tma_load_3d(st + OZ_A_BYTES, &mapb, x, t.b_row, 0, &full[s]);
+          issued = g + 1;
+        }
+        if (!ok) break;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int g = 0, it = 0;  // k chunks; uses of each accumulator
+      bool ok = true;
+      for (int ti = blockIdx.x; ti < ntask && ok; ti += gridDim.x) {
+        const int nk = tasks[ti].nk;
+        const uint32_t idesc =
+            oz_idesc(min(ON, (tasks[ti].colEnd - tasks[ti].col0 + 15) & ~15));
+        for (int kc = 0; kc < nk && ok; ++kc, ++g) {
+          const int s = g % OZ_STAGES;
+          const bool first = kc % OZ_DRAIN == 0;
+          const bool last = kc % OZ_DRAIN == OZ_DRAIN - 1 || kc == nk - 1;
+          if (!mbar_wait_or_abort(&full[s], (g / OZ_STAGES) & 1, err, abortp)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t ad = sw64_desc(su32(smem + s * OZ_STAGE_BYTES));
+          const uint64_t bd = sw64_desc(su32(smem + s * OZ_STAGE_BYTES + OZ_A_BYTES));
+          for (int gr = 0; gr < OZ_GROUPS; ++gr) {
+            // the epilogue has read this accumulator's previous sum
+            if (first && it > 0) {
+              if (!mbar_wait_or_abort(&acc_empty[gr], (it - 1) & 1, err, abortp)) {
+                ok = false;
+                break;
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            const uint32_t d = tmem + (uint32_t)(gr * ON);
+            for (int p = 0; p <= gr; ++p) {
+              const uint64_t ap = ad + (uint64_t)(p * (OZ_A_TILE >> 4));
+              const uint64_t bq = bd + (uint64_t)((gr - p) * (OZ_B_TILE >> 4));
+#pragma unroll
+              for (int kk = 0; kk < OZ_KC / 16; ++kk)
+                mma_bf16(d, ap + 2 * kk, bq + 2 * kk, idesc,
+                         (first && p == 0 && kk == 0) ? 0u : 1u);
+            }
+            if (last) mma_commit(&acc_full[gr]);
+          }
+          if (last) ++it;
+          if (ok) mma_commit(&empty[s]);
+        }
+      }
+      // every MMA issued so far has completed once `done` fires
+      mma_commit(&done);
+    }
+  } else {
+    // TMEM lanes [32q, 32q + 32) are this warp's, and columns [32h, 32h + 32)
+    // of each tile
+    const int q = warp & 3, h = (warp - OZ_EPI_WARP0) >> 2;
+    const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * 32);
+    int it = 0;
+    bool ok = true;
+    // wait for group gr's accumulator and start its read into v (warp-uniform:
+    // tcgen05.ld is a warp-collective instruction)
+    auto fetch = [&](int gr, uint32_t (&v)[32]) {
+      int ready = 0;
+      if (lane == 0) ready = mbar_wait_or_abort(&acc_full[gr], it & 1, err, abortp);
+      ready = __shfl_sync(0xffffffffu, ready, 0);
+      if (!ready) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_ld32_async(ta + (uint32_t)(gr * ON), v);
+      return true;
+    };
+    // the read of group gr has landed: hand the accumulator back
+    auto landed = [&](int gr, uint32_t (&v)[32]) {
+      tmem_ld_wait(v);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[gr]);
+    };
+    for (int ti = blockIdx.x; ti < ntask && ok; ti += gridDim.x) {
+      const TcTask t = tasks[ti];
+      const int rt = q * 32 + lane, row = t.row0 + rt;
+      const int c0 = t.col0 + h * 32;
+      const bool on = c0 < t.colEnd;  // warp-uniform
+      const bool has = row < t.rowEnd;
+      // row exponent; lane j holds column c0 + j's
+      const int ei = has ? sexp[t.a_row + rt] : 0;
+      const int ejl = c0 + lane < t.colEnd ? sexp[t.b_row + h * 32 + lane] : 0;
+      long long acc[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = 0;
+      for (int kc = 0; kc < t.nk; kc += OZ_DRAIN) {
+        uint32_t va[32], vb[32];
+        auto add = [&](auto gc, uint32_t (&v)[32]) {
+          if (on) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              add_group<decltype(gc)::value>(acc[j], __float2int_rn(__uint_as_float(v[j])));
+          }
+        };
+        auto step = [&](auto gc, uint32_t (&cur)[32], uint32_t (&nxt)[32]) {
+          constexpr int G = decltype(gc)::value;
+          if (!ok) return;
+          landed(G, cur);
+          if constexpr (G + 1 < OZ_GROUPS) ok = fetch(G + 1, nxt);
+          add(gc, cur);
+        };
+        ok = fetch(0, va);
+        step(std::integral_constant<int, 0>{}, va, vb);
+        step(std::integral_constant<int, 1>{}, vb, va);
+        step(std::integral_constant<int, 2>{}, va, vb);
+        step(std::integral_constant<int, 3>{}, vb, va);
+        step(std::integral_constant<int, 4>{}, va, vb);
+        step(std::integral_constant<int, 5>{}, vb, va);
+        step(std::integral_constant<int, 6>{}, va, vb);
+        if (!ok) break;
+        ++it;
+      }
+      if (!ok) break;
+      if (!on) continue;
+      // columns [c0, cend) of this row are updated (lower triangle, in range)
+      const int cend = has ? min(t.colEnd, row + 1) : c0;
+      const bool safe = __all_sync(0xffffffffu, abs(ei) <= OZ_EXP_SAFE / 2 &&
+                                                    abs(ejl) <= OZ_EXP_SAFE / 2);
+      double* cp = arena + t.c_off + row + (int64_t)c0 * t.ldc;
+      double cv[2][8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) cv[0][j] = c0 + j < cend ? cp[(int64_t)j * t.ldc] : 0.0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        if (b < 3) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            cv[(b + 1) & 1][j] =
+                c0 + 8 * b + 8 + j < cend ? cp[(int64_t)(8 * b + 8 + j) * t.ldc] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int jj = 8 * b + j;
+          const int e = ei + __shfl_sync(0xffffffffu, ejl, jj);
+          double d;
+          if (safe) {
+            d = fixed_to_double(acc[jj], e);
+          } else {
+            d = fixed_to_double(acc[jj], max(-OZ_EXP_SAFE, min(OZ_EXP_SAFE, e)));
+            d *= extreme_scale(e);
+          }
+          if (c0 + jj < cend) cp[(int64_t)jj * t.ldc] = cv[b & 1][j] - d;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // all MMAs this CTA issued have drained once `done` fires; wait for it even
+  // after a failure, before TMEM is freed
+  mbar_wait(&done, 0, err);
+  // copies still in flight after a failure: wait (bounded) for the last one
+  // issued on each stage before the shared memory they target goes away
+  if (*abortp && warp == 0 && lane == 0) {
+    for (int g = issued - 1; g >= 0 && g >= issued - OZ_STAGES; --g)
+      mbar_wait(&full[g % OZ_STAGES], (g / OZ_STAGES) & 1, err);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(OZ_TMEM_COLS)
+                 : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Scale exponent and digits of 32 front rows (one CTA): a first pass over
+// the K columns for the row norms (exponents and a 24-bit sum of squares,
+// integer and FP32 arithmetic only), a second one, from L2, for the digits.
+
+constexpr int SPLIT_ROWS = 32, SPLIT_K = 64;
+
+__global__ void __launch_bounds__(256) k_oz_split(const double* __restrict__ arena,
+                                                  const OzSplit* __restrict__ sp,
+                                                  uint16_t* __restrict__ planes,
+                                                  int64_t pstride, int pitch,
+                                                  int* __restrict__ sexp) {
+  __shared__ long long F[SPLIT_ROWS][SPLIT_K + 1];
+  __shared__ int re[8][SPLIT_ROWS], rbad[8][SPLIT_ROWS];
+  __shared__ float rs[8][SPLIT_ROWS];
+  const OzSplit t = sp[blockIdx.x];
+  const int i0 = blockIdx.y * SPLIT_ROWS;
+  if (i0 >= t.rows) return;  // uniform over the CTA
+  const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const bool has = i0 + lane < t.rows;
+  const long long* src = reinterpret_cast<const long long*>(arena) + t.off +
+                         (int64_t)t.c0 * t.ld + t.r0 + i0 + lane;
+  int e = OZ_EMPTY;
+  float s = 0.f;
+  bool bad = false;
+  for (int k0 = ty; k0 < t.K; k0 += 64) {
+    long long x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + 8 * u;
+      x[u] = (has && k < t.K) ? src[(int64_t)k * t.ld] : 0ll;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) norm_add(e, s, x[u], bad);
+  }
+  re[ty][lane] = e;
+  rs[ty][lane] = s;
+  rbad[ty][lane] = bad;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) e = max(e, re[w][lane]);
+  s = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const int d = e - re[w][lane];
+    if (d <= 60) s += rs[w][lane] * __uint_as_float((unsigned)(127 - 2 * d) << 23);
+    bad = bad || rbad[w][lane];
+  }
+  e = norm_exponent(e, s);
+  if (ty == 0 && has) sexp[t.base + i0 + lane] = bad ? OZ_NONFINITE : e;
+  const bool zero = bad || !(s > 0.f);
+  const int kpad = (t.K + OZ_KC - 1) / OZ_KC * OZ_KC;
+  for (int k0 = 0; k0 < kpad; k0 += SPLIT_K) {
+    long long x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + ty + 8 * u;
+      x[u] = (has && k < t.K) ? src[(int64_t)k * t.ld] : 0ll;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) F[lane][ty + 8 * u] = zero ? 0ll : to_fixed(x[u], e);
+    __syncthreads();
+    if (k0 + 2 * lane < kpad) {
+      for (int r = ty; r < SPLIT_ROWS && i0 + r < t.rows; r += 8) {
+        store_digits(F[r][2 * lane], F[r][2 * lane + 1],
+                     planes + (int64_t)(t.base + i0 + r) * pitch + k0 + 2 * lane, pstride);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+static size_t tc64_smem_bytes() { return (size_t)OZ_STAGES * OZ_STAGE_BYTES + 1024; }
+
+static int g_num_sms64 = 0;
+
+void prepare_tc64_kernels() {
+  SG_CUDA(cudaFuncSetAttribute(k_update_tc64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)tc64_smem_bytes()));
+  int dev = 0;
+  SG_CUDA(cudaGetDevice(&dev));
+  SG_CUDA(cudaDeviceGetAttribute(&g_num_sms64, cudaDevAttrMultiProcessorCount, dev));
+}
+
+void make_digit_maps(CUtensorMap* maps, const uint16_t* planes, int64_t pstride, int64_t rows,
+                     int pitch) {
+  cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)std::max<int64_t>(rows, 1), OZ_DIGITS};
+  cuuint64_t strides[2] = {(cuuint64_t)pitch * sizeof(uint16_t),
+                           (cuuint64_t)pstride * sizeof(uint16_t)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  for (int q = 0; q < 2; ++q) {
+    cuuint32_t box[3] = {OZ_KC, (cuuint32_t)(q ? ON : OT), OZ_DIGITS};
+    CUresult r = encode_fn()(&maps[q], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)planes, dims,
+                             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled failed");
+  }
+}
+
+void launch_oz_split(const double* arena, const OzSplit* sp, int nsplit, int64_t max_rows,
+                     uint16_t* planes, int64_t pstride, int pitch, int* sexp, cudaStream_t s) {
+  if (nsplit <= 0 || max_rows <= 0) return;
+  dim3 grid((unsigned)nsplit, (unsigned)((max_rows + SPLIT_ROWS - 1) / SPLIT_ROWS));
+  k_oz_split<<<grid, 256, 0, s>>>(arena, sp, planes, pstride, pitch, sexp);
+}
+
+void launch_update_tc64(const CUtensorMap* maps, double* arena, const int* sexp, const TcTask* t,
+                        int ntask, unsigned* err, cudaStream_t s) {
+  if (ntask <= 0) return;
+  const int grid = std::min(ntask, g_num_sms64 > 0 ? g_num_sms64 : 148);
+  k_update_tc64<<<grid, OZ_THREADS, tc64_smem_bytes(), s>>>(maps[0], maps[1], arena, sexp, t, ntask,
+                                                               err);
+}
+
+}  // namespace sylver_gb300

@@ -52,6 +52,7 @@ bool Runtime::init() {
     prepare_factor_kernels<float>();
     prepare_factor_kernels<double>();
     prepare_tc_kernels();
+    prepare_tc64_kernels();
     prepare_blocked_kernels();
     prepare_solve_kernels<float>();
     prepare_solve_kernels<double>();
@@ -371,6 +372,9 @@ void FKeep::plan_cholesky() {
   std::vector<PanelTask> panels, diags;
   std::vector<UpdTask> upds;
   std::vector<TcSplit> tcs;
+  std::vector<OzSplit> ozs;
+  std::vector<P64Task> pan64, dst64;
+  dstore_blocks = 0;
   std::vector<TcTask> tct;
   std::vector<double> tc_flops;
   std::vector<std::pair<size_t, double>> tcop_flops;  // (op index, flops) of grouped updates
@@ -379,6 +383,56 @@ void FKeep::plan_cholesky() {
   blkinv_count = 0;
   const int PW = (f32 && use_tc) ? sched.panel_cols() : 0;
   blk_pw = PW;
+  // FP64 fronts: panel steps of NB columns in groups of OZ_GW, updates on the
+  // tensor cores from operands cut into digits (kernels_tc64.cu)
+  const bool oz = !f32 && use_tc && TC_ROWS > 0;
+  // one update of rows [c, m) x columns [c, ce) of the given fronts by their
+  // columns [k0, k0 + K), from digits of rows [c, m); with split a launch
+  // before it cuts them, else the panel kernel did (level oz_level made)
+  struct OzUpd {
+    int s, c, ce, k0, K, base;
+  };
+  auto oz_level = [&](std::vector<OzUpd>& us, int unit) {
+    int64_t rows = 0, mxr = 0;
+    int pitch = 0;
+    for (OzUpd& u : us) {
+      const int mr = st.nrow[u.s] - u.c;
+      u.base = (int)rows;
+      rows += mr;
+      mxr = std::max<int64_t>(mxr, mr);
+      pitch = std::max(pitch, round_up(u.K, unit));
+    }
+    tclev.push_back({pitch, rows, mxr});
+    tc_flops.push_back(0.0);
+    return (int)tclev.size() - 1;
+  };
+  auto oz_update = [&](std::vector<OzUpd>& us, bool split, int lvl) {
+    if (us.empty()) return;
+    if (split) {
+      lvl = oz_level(us, 64);
+      const int64_t sp0 = (int64_t)ozs.size();
+      for (const OzUpd& u : us)
+        ozs.push_back({off[u.s], ld[u.s], u.c, st.nrow[u.s] - u.c, u.k0, u.K, u.base});
+      ops.push_back({Op::SPLIT, sp0, (int64_t)ozs.size(), lvl});
+    }
+    // 64-column tiles; 32-column ones when those leave SMs idle
+    int64_t nt = 0;
+    for (const OzUpd& u : us)
+      for (int col0 = u.c; col0 < u.ce; col0 += OZ_TILE_COLS)
+        nt += (st.nrow[u.s] - col0 + 127) / 128;
+    const int tw = nt <= OZ_FEW_TILES / 2 ? OZ_TILE_COLS / 2 : OZ_TILE_COLS;
+    const int64_t tk0 = (int64_t)tct.size();
+    for (const OzUpd& u : us) {
+      const int m = st.nrow[u.s], nk = (u.K + OZ_KC - 1) / OZ_KC;
+      for (int col0 = u.c; col0 < u.ce; col0 += tw)
+        for (int row0 = col0; row0 < m; row0 += 128)
+          tct.push_back({off[u.s], ld[u.s], row0, col0, m, std::min(u.ce, col0 + tw),
+                         u.base + row0 - u.c, u.base + col0 - u.c, nk, 0});
+      tc_flops[lvl] += 2.0 * u.K * ((double)(u.ce - u.c) * m -
+                                    0.5 * (u.ce * (u.ce - 1.0) - u.c * (u.c - 1.0)));
+    }
+    ops.push_back({Op::TCUPD, tk0, (int64_t)tct.size(), lvl});
+  };
   std::vector<int> pos(st.n, -1);
   ops.clear();
   op_level.clear();
@@ -587,41 +641,103 @@ void FKeep::plan_cholesky() {
     } else {
       for (int s : large) maxsteps = std::max(maxsteps, (st.ncol[s] + NB - 1) / NB);
     }
+    const int64_t ds0 = (int64_t)dst64.size();
     for (int step = 0; step < maxsteps; ++step) {
       int64_t p0 = (int64_t)panels.size(), u0 = (int64_t)upds.size();
-      int64_t d0 = (int64_t)diags.size();
+      int64_t d0 = (int64_t)diags.size(), q0 = (int64_t)pan64.size();
+      const int k0 = step * NB;
+      // FP64 on the tensor cores: within a group each panel updates the
+      // group's later columns; its last one leaves the columns past the
+      // group to one update by the whole group
+      std::vector<OzUpd> ozp;
+      const int g0 = k0 / OZ_GW * OZ_GW, o = k0 + NB;
+      const bool gend = o == g0 + OZ_GW;
+      int64_t below = 0;
       for (int s : large) {
-        int m = st.nrow[s], n = st.ncol[s];
-        int k0 = step * NB;
+        const int m = st.nrow[s], n = st.ncol[s];
+        if (k0 < n) below += m - std::min(o, n);
+        if (oz && o < n)
+          ozp.push_back(gend ? OzUpd{s, o, n, g0, OZ_GW, 0}
+                             : OzUpd{s, o, std::min(n, g0 + OZ_GW), k0, NB, 0});
+      }
+      int lvl = -1;
+      if (!gend && !ozp.empty()) lvl = oz_level(ozp, OZ_KC);
+      // rows per panel CTA: all SMs busy, then as few repeats of the
+      // diagonal block's factorization as that allows
+      const int rt64 = below <= OZ_FEW_TILES * 16 / 2
+                           ? 16
+                           : std::max(32, std::min(256, (int)(below / OZ_FEW_TILES) / 32 * 32));
+      size_t qi = 0;
+      for (int s : large) {
+        const int m = st.nrow[s], n = st.ncol[s];
         if (k0 >= n) continue;
-        int w = std::min(NB, n - k0);
-        diags.push_back({off[s], ld[s], k0, w, k0, k0 + w, 0});
-        for (int r0 = k0 + w; r0 < m; r0 += RT)
-          panels.push_back({off[s], ld[s], k0, w, r0, std::min(r0 + RT, m), 0});
-        int o = k0 + w;
-        if (o < n) {
-          for (int cj = 0; o + cj * TM < n; ++cj)
-            for (int ri = cj; o + ri * TM < m; ++ri)
-              upds.push_back({off[s], off[s], off[s], ld[s], ld[s], ld[s], o + ri * TM,
-                              o + cj * TM, m, n, k0, k0 + w, 0});
+        const int w = std::min(NB, n - k0);
+        if (!f32) {
+          int base = -1;
+          if (lvl >= 0 && qi < ozp.size() && ozp[qi].s == s) base = ozp[qi++].base;
+          const int didx = (int)((int64_t)dst64.size() - ds0);
+          int r0 = k0 + w;
+          do {
+            const int r1 = std::min(r0 + rt64, m);
+            pan64.push_back({off[s], ld[s], k0, w, r0, r1, base < 0 ? -1 : base + r0 - (k0 + w),
+                             r0 == k0 + w ? didx : -1, 0});
+            r0 = r1;
+          } while (r0 < m);
+          dst64.push_back({off[s], ld[s], k0, w, 0, 0, -1, didx, 0});
+        } else {
+          diags.push_back({off[s], ld[s], k0, w, k0, k0 + w, 0});
+          for (int r0 = k0 + w; r0 < m; r0 += RT)
+            panels.push_back({off[s], ld[s], k0, w, r0, std::min(r0 + RT, m), 0});
+        }
+        if (!oz && k0 + w < n) {
+          const int c0 = k0 + w;
+          for (int cj = 0; c0 + cj * TM < n; ++cj)
+            for (int ri = cj; c0 + ri * TM < m; ++ri)
+              upds.push_back({off[s], off[s], off[s], ld[s], ld[s], ld[s], c0 + ri * TM,
+                              c0 + cj * TM, m, n, k0, k0 + w, 0});
         }
       }
       if ((int64_t)diags.size() > d0) ops.push_back({Op::DIAG, d0, (int64_t)diags.size(), 0});
       if ((int64_t)panels.size() > p0) ops.push_back({Op::PANEL, p0, (int64_t)panels.size(), 0});
+      if ((int64_t)pan64.size() > q0) ops.push_back({Op::PANEL, q0, (int64_t)pan64.size(), lvl, rt64});
       if ((int64_t)upds.size() > u0) ops.push_back({Op::UPD, u0, (int64_t)upds.size(), 0});
+      oz_update(ozp, gend, lvl);
+    }
+    if ((int64_t)dst64.size() > ds0) {
+      ops.push_back({Op::DIAG, ds0, (int64_t)dst64.size(), 0});
+      dstore_blocks = std::max(dstore_blocks, (int64_t)dst64.size() - ds0);
     }
     // contribution blocks: one Schur-complement update with K = n, on the
     // tensor cores (FP32, 3xBF16) for blocks of at least 64 rows
     int64_t u0 = (int64_t)upds.size();
+    std::vector<OzUpd> ozc;
     for (int s : large) {
       int m = st.nrow[s], n = st.ncol[s];
       if (m <= n || cbb[s] >= 0) continue;
+      if (oz) {
+        ozc.push_back({s, n, m, 0, n, 0});
+        continue;
+      }
       for (int cj = 0; n + cj * TM < m; ++cj)
         for (int ri = cj; n + ri * TM < m; ++ri)
           upds.push_back({off[s], off[s], off[s], ld[s], ld[s], ld[s], n + ri * TM,
                           n + cj * TM, m, m, 0, n, 0});
     }
     if ((int64_t)upds.size() > u0) ops.push_back({Op::UPD, u0, (int64_t)upds.size(), 0});
+    // FP64: fronts of like K together, so that the common pitch pads little,
+    // and at most 2^29 operand elements a launch (more only for one front)
+    std::stable_sort(ozc.begin(), ozc.end(), [](const OzUpd& x, const OzUpd& y) { return x.K > y.K; });
+    for (size_t q = 0; q < ozc.size();) {
+      std::vector<OzUpd> us;
+      const int pitch = round_up(ozc[q].K, 64), kmin = ozc[q].K / 2;
+      int64_t rows = 0;
+      while (q < ozc.size() && ozc[q].K >= kmin) {
+        rows += st.nrow[ozc[q].s] - ozc[q].c;
+        if (!us.empty() && rows * pitch > (1ll << 29)) break;
+        us.push_back(ozc[q++]);
+      }
+      oz_update(us, true, -1);
+    }
     if (!tcf.empty()) {
       const int pitch = cb_pitch;
       int64_t rows = 0, mx = cb_mx;
@@ -694,6 +810,9 @@ void FKeep::plan_cholesky() {
   panel.upload(panels, s);
   diagt.upload(diags, s);
   tcsplit.upload(tcs, s);
+  ozsplit.upload(ozs, s);
+  panel64.upload(pan64, s);
+  diagst64.upload(dst64, s);
   tctask.upload(tct, s);
   blkdiag.upload(blkd, s);
   blkpanel.upload(blkp, s);
@@ -734,8 +853,23 @@ void FKeep::upload_static(cudaStream_t s) {
     if (splan.dataflow && splan.p_elems > 0) splan.pmat.ensure((size_t)splan.p_elems * sizeof(float));
   }
   tcerr.ensure(sizeof(unsigned));
+  if (dstore_blocks > 0) dstore64.ensure((size_t)dstore_blocks * 32 * 32 * sizeof(double));
   if (blkinv_count > 0) blkinv.ensure((size_t)blkinv_count * BLK_B * BLK_B * sizeof(float));
-  if (!tclev.empty()) {
+  if (!tclev.empty() && precision != 1) {
+    // one buffer of seven digit planes and row exponents for all launches
+    int64_t cap = 1, rows = 1;
+    for (auto& L : tclev) {
+      cap = std::max(cap, L.rows * L.pitch);
+      rows = std::max(rows, L.rows);
+    }
+    plane_stride = round_up64(cap, 64);
+    tcplanes.ensure((size_t)OZ_DIGITS * plane_stride * sizeof(uint16_t));
+    ozexp.ensure((size_t)rows * sizeof(int));
+    tmaps.resize(2 * tclev.size());
+    for (size_t l = 0; l < tclev.size(); ++l)
+      make_digit_maps(&tmaps[2 * l], tcplanes.as<uint16_t>(), plane_stride, tclev[l].rows,
+                     tclev[l].pitch);
+  } else if (!tclev.empty()) {
     int64_t cap = 0, cbcap = 0;
     for (auto& L : tclev) (L.cb ? cbcap : cap) = std::max(L.cb ? cbcap : cap, L.rows * L.pitch);
     // three BF16 planes of cap elements each (plane stride rounded to 64
@@ -786,10 +920,19 @@ void FKeep::run_ops(cudaStream_t s) {
         launch_small_chol<T>(A, small.as<SmallTask>() + op.a, (int)cnt, op.aux, stp, s);
         break;
       case Op::DIAG:
-        launch_diag_chol<T>(A, diagt.as<PanelTask>() + op.a, (int)cnt, stp, s);
+        if constexpr (std::is_same<T, float>::value)
+          launch_diag_chol<T>(A, diagt.as<PanelTask>() + op.a, (int)cnt, stp, s);
+        else
+          launch_diag_store64(A, diagst64.as<P64Task>() + op.a, (int)cnt, dstore64.as<double>(),
+                              s);
         break;
       case Op::PANEL:
-        launch_panel_trsm<T>(A, panel.as<PanelTask>() + op.a, (int)cnt, s);
+        if constexpr (std::is_same<T, float>::value)
+          launch_panel_trsm<T>(A, panel.as<PanelTask>() + op.a, (int)cnt, s);
+        else
+          launch_panel64(A, panel64.as<P64Task>() + op.a, (int)cnt, op.rows, dstore64.as<double>(),
+                         tcplanes.as<uint16_t>(), plane_stride,
+                         op.aux >= 0 ? tclev[op.aux].pitch : 0, ozexp.as<int>(), stp, s);
         break;
       case Op::UPD:
         launch_update<T>(A, A, upd.as<UpdTask>() + op.a, (int)cnt, s);
@@ -801,6 +944,10 @@ void FKeep::run_ops(cudaStream_t s) {
         if constexpr (std::is_same<T, float>::value)
           launch_split_t(A, tcsplit.as<TcSplit>() + op.a, (int)cnt, tclev[op.aux].max_rows,
                          tcplanes.as<uint16_t>(), plane_stride, tclev[op.aux].pitch, s);
+        else
+          launch_oz_split(A, ozsplit.as<OzSplit>() + op.a, (int)cnt, tclev[op.aux].max_rows,
+                          tcplanes.as<uint16_t>(), plane_stride, tclev[op.aux].pitch,
+                          ozexp.as<int>(), s);
         break;
       case Op::BDIAG:
         if constexpr (std::is_same<T, float>::value)
@@ -816,6 +963,9 @@ void FKeep::run_ops(cudaStream_t s) {
         if constexpr (std::is_same<T, float>::value)
           launch_update_tc(&tmaps[3 * op.aux], A, tctask.as<TcTask>() + op.a, (int)cnt,
                            tcerr.as<unsigned>(), s);
+        else
+          launch_update_tc64(&tmaps[2 * op.aux], A, ozexp.as<int>(), tctask.as<TcTask>() + op.a,
+                             (int)cnt, tcerr.as<unsigned>(), s);
         break;
     }
   }

@@ -120,6 +120,7 @@ struct Op {
   enum Kind { MEMSET, INIT, EA, SMALL, PANEL, UPD, DIAG, INV, SPLIT, TCUPD, BDIAG, BPANEL, EAG, ASM } kind;
   int64_t a = 0, b = 0;  // task range [a, b)
   int aux = 0;           // SMALL: max front rows; SPLIT/TCUPD: tensor-core level
+  int rows = 0;          // PANEL (FP64): most rows of a task
 };
 
 struct Level {
@@ -222,6 +223,10 @@ struct FKeep {
   std::vector<TcLevel> tclev;
   std::vector<CUtensorMap> tmaps;   // three per tensor-core launch (one per BF16 plane)
   DevMem tcsplit, tctask, tcplanes, tcerr;
+  // FP64: digit splits and row scale exponents; panel and diagonal-store
+  // tasks, and the factorised diagonal blocks of a level's panels
+  DevMem ozsplit, ozexp, panel64, diagst64, dstore64;
+  int64_t dstore_blocks = 0;
   int64_t plane_stride = 0;        // elements between the BF16 planes
   DevMem cbplanes;                 // contribution-block operands written by the panel kernel
   int64_t cb_stride = 0;

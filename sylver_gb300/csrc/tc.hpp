@@ -37,4 +37,43 @@ void launch_split_t(const float* arena, const TcSplit* sp, int nsplit, int64_t m
 void launch_update_tc(const CUtensorMap* maps, float* arena, const TcTask* t, int ntask,
                       unsigned* err, cudaStream_t s);
 
+// FP64 fronts (kernels_tc64.cu): C -= P_a P_b^T on the BF16 tensor cores with
+// operands cut into seven signed 9-bit digits of a per-row fixed-point
+// scaling.  TcTask's nk and kc0 count chunks of OZ_KC columns here.
+constexpr int OZ_KC = 32;
+constexpr int OZ_DIGITS = 7;
+constexpr int OZ_TILE_COLS = 64;  // tiles are 128 x 64 or narrower
+constexpr int OZ_GW = 256;  // fully-summed columns per trailing update
+constexpr int OZ_FEW_TILES = 304;  // launches below this many CTAs take smaller tiles
+// Digits of front rows [r0, r0 + rows) x columns [c0, c0 + K): stacked rows
+// [base, base + rows) of the seven planes (zeros from K to K rounded up to
+// OZ_KC), and each row's scale exponent in sexp[base ..].
+struct OzSplit {
+  int64_t off;
+  int ld, r0, rows, c0, K, base;
+};
+// Panel step of an FP64 front (kernels_panel64.cu): the w x w diagonal block at
+// (k0, k0), w <= 32, and rows [r0, r1) below it; base >= 0: stacked row of
+// r0 in the digit planes; didx >= 0: this CTA stores the factorised block as
+// block didx of the level's store.
+struct P64Task {
+  int64_t off;
+  int ld, k0, w, r0, r1, base, didx, pad;
+};
+// rows: most rows of a task (16 or fewer take the kernel for short tasks)
+void launch_panel64(double* arena, const P64Task* t, int ntask, int rows, double* dstore,
+                    uint16_t* planes, int64_t pstride, int pitch, int* sexp, unsigned* status,
+                    cudaStream_t s);
+void launch_diag_store64(double* arena, const P64Task* t, int ntask, const double* dstore,
+                         cudaStream_t s);
+void prepare_tc64_kernels();
+// Maps of all seven planes (plane q at planes + q * pstride) with the boxes
+// of the A (128 rows) and the B operand (64 rows).
+void make_digit_maps(CUtensorMap* maps, const uint16_t* planes, int64_t pstride, int64_t rows,
+                     int pitch);
+void launch_oz_split(const double* arena, const OzSplit* sp, int nsplit, int64_t max_rows,
+                     uint16_t* planes, int64_t pstride, int pitch, int* sexp, cudaStream_t s);
+void launch_update_tc64(const CUtensorMap* maps, double* arena, const int* sexp, const TcTask* t,
+                        int ntask, unsigned* err, cudaStream_t s);
+
 }  // namespace sylver_gb300
