@@ -559,33 +559,71 @@ __global__ void k_lscatter(const LTask* __restrict__ tasks, LsArgs<T, ACC> a, bo
   scatter_body<T, ACC>(tasks[blockIdx.x], a, fwd);
 }
 
-// X = L^-1 for one diagonal block, thread j computes column j; L is read
-// straight from the front (all threads read the same element: broadcast).
+// X = L^-1 for one LB x LB diagonal block (identity beyond bw): four lanes per
+// column, lane c holding rows c, c + 4, ...  The substitution runs on
+// z_k = x_k L(k, k) with L(i, k) / L(k, k) in shared memory, one shuffle and one
+// multiply-add per step, and divides at the end.  Bound by the FP64 pipe (the
+// block's 44k multiply-adds on one SM); one thread per column with L read from
+// the front took 170 us for any number of blocks.
 template <typename T>
-__global__ void __launch_bounds__(LB) k_inv_diag(const T* __restrict__ arena,
-                                                 const FrontDesc* __restrict__ fr,
-                                                 const LTask* __restrict__ tasks,
-                                                 T* __restrict__ inv,
-                                                 const int64_t* __restrict__ inv_off, bool unit) {
-  __shared__ T Xs[LB][LB + 1];  // Xs[j][i] = X(i, j)
+__global__ void __launch_bounds__(4 * LB) k_inv_diag(const T* __restrict__ arena,
+                                                     const FrontDesc* __restrict__ fr,
+                                                     const LTask* __restrict__ tasks,
+                                                     T* __restrict__ inv,
+                                                     const int64_t* __restrict__ inv_off,
+                                                     bool unit) {
+  __shared__ T Ls[LB][LB + 1];  // Ls[k][i] = L(i, k), then L(i, k) / L(k, k)
+  __shared__ T dg[LB], rd[LB];
   const LTask t = tasks[blockIdx.x];
   const FrontDesc f = fr[t.f];
-  const T* L = arena + f.off;
-  const int c0 = t.c0, bw = t.bw, j = threadIdx.x;
-  auto l = [&](int i, int k) -> T {  // padded block: identity outside bw
-    if (i >= bw || k >= bw) return (i == k) ? T(1) : T(0);
-    if (i == k && unit) return T(1);
-    return L[(int64_t)(c0 + k) * f.ld + c0 + i];
-  };
-  for (int i = 0; i < LB; ++i) {
-    T acc = (i == j) ? T(1) : T(0);
-    if (i > j)
-      for (int k = j; k < i; ++k) acc -= l(i, k) * Xs[j][k];
-    Xs[j][i] = (i >= j) ? acc / l(i, i) : T(0);
+  const int c0 = t.c0, bw = t.bw, tid = threadIdx.x;
+  const T* L = arena + f.off + (int64_t)c0 * f.ld + c0;
+#pragma unroll 8
+  for (int e = tid; e < LB * LB; e += 4 * LB) {
+    const int i = e % LB, k = e / LB;
+    T v = i == k ? T(1) : T(0);
+    if (i < bw && k < bw && i >= k && !(i == k && unit)) v = L[(int64_t)k * f.ld + i];
+    Ls[k][i] = v;
   }
-  T* out = inv + inv_off[t.f] + (int64_t)(c0 / LB) * LB * LB;
   __syncthreads();
-  for (int e = j; e < LB * LB; e += LB) out[e] = Xs[e / LB][e % LB];
+  if (tid < LB) {
+    dg[tid] = Ls[tid][tid];
+    rd[tid] = T(1) / Ls[tid][tid];
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int e = tid; e < LB * LB; e += 4 * LB) {
+    const int i = e % LB, k = e / LB;
+    if (i > k) Ls[k][i] *= rd[k];
+  }
+  __syncthreads();
+  constexpr int NU = LB / 4;
+  const int lane = tid & 31, c = lane & 3, j = tid >> 2;
+  const int w8 = (tid >> 5) * 8;  // first column of this warp: rows above are zero
+  T z[NU];
+#pragma unroll
+  for (int u = 0; u < NU; ++u) z[u] = 4 * u + c == j ? T(1) : T(0);
+#pragma unroll
+  for (int u0 = 0; u0 < NU; ++u0) {
+    if (4 * u0 < w8) continue;  // warp-uniform
+#pragma unroll 1
+    for (int cc = 0; cc < 4; ++cc) {
+      const T zk = __shfl_sync(0xffffffffu, z[u0], (lane & ~3) | cc);
+      const T* lk = &Ls[4 * u0 + cc][c];
+      if (c > cc) z[u0] -= zk * lk[4 * u0];
+#pragma unroll
+      for (int u = u0 + 1; u < NU; ++u) z[u] -= zk * lk[4 * u];
+    }
+  }
+  T* out = inv + inv_off[t.f] + (int64_t)(c0 / LB) * LB * LB + (int64_t)j * LB;
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    const int i = 4 * u + c;
+    // z / L(i, i): product with the reciprocal, corrected by its remainder
+    const T q = z[u] * rd[i];
+    const T r = fma(-q, dg[i], z[u]);
+    out[i] = fma(r, rd[i], q);
+  }
 }
 
 // Block steps of SW = LSOLVE_BW2 columns.  Each diagonal block has an
@@ -608,7 +646,11 @@ template <typename ACC> struct RGP { static constexpr int v = RGn<ACC>::v + 16 /
 
 // X = inverse of the SW-column diagonal block of a step (column-major, ld SW,
 // lower): X_jj = Inv64_j and X_ij = -Inv64_i * sum_{k=j}^{i-1} L_ik X_kj for
-// i > j, with 64x64 blocks; identity beyond bw.
+// i > j, with 64x64 blocks; identity beyond bw.  One CTA per 16 columns of a
+// block (columns of an inverse do not depend on one another): in FP64 the
+// products of a whole block kept one SM's pipe busy for 1.2 ms.  The strip's
+// rows above block j and the zero halves of X_jj and Inv64_i are skipped.
+constexpr int IVC = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) k_inv_block(const T* __restrict__ arena,
                                                 const FrontDesc* __restrict__ fr,
@@ -619,86 +661,71 @@ __global__ void __launch_bounds__(256) k_inv_block(const T* __restrict__ arena,
                                                 T* __restrict__ inv2t,
                                                 const int64_t* __restrict__ inv2_off) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* As = reinterpret_cast<T*>(sm_raw);  // As[k*65 + r] = A(r, k)
-  T* Bs = As + 64 * 65;                  // Bs[c*65 + k] = B(k, c)
-  const LTask t = tasks[blockIdx.x];
+  T* Xs = reinterpret_cast<T*>(sm_raw);  // Xs[r*IVC + q] = X(r, s0 + q)
+  T* As = Xs + SW * IVC;                 // As[k*65 + r] = A(r, k)
+  const LTask t = tasks[blockIdx.x / (SW / IVC)];
   const FrontDesc f = fr[t.f];
-  const T* L = arena + f.off;
+  const int s0 = blockIdx.x % (SW / IVC) * IVC, j = s0 / LB;
   const int c0 = t.c0, bw = t.bw, tid = threadIdx.x;
-  T* X = inv2 + inv2_off[t.f] + (int64_t)(c0 / SW) * SW * SW;
+  const T* L = arena + f.off + (int64_t)c0 * f.ld + c0;
   const T* I64 = inv64 + inv_off[t.f] + (int64_t)(c0 / LB) * LB * LB;
   const int nb = (bw + LB - 1) / LB;
-  for (int e = tid; e < SW * SW; e += blockDim.x) X[e] = T(0);
-  __syncthreads();
-  for (int j = 0; j < SW / LB; ++j)
-    for (int e = tid; e < LB * LB; e += blockDim.x) {
-      int i = e % LB, k = e / LB;
-      X[(int64_t)(LB * j + k) * SW + LB * j + i] =
-          (j < nb) ? I64[(int64_t)j * LB * LB + k * LB + i] : T(i == k ? 1 : 0);
-    }
-  __syncthreads();
-  const int r = tid % LB, cq = tid / LB;  // output row, 16-column quarter
-  for (int j = 0; j < nb; ++j)
-    for (int i = j + 1; i < nb; ++i) {
-      T acc[16];
+  for (int e = tid; e < SW * IVC; e += 256) {
+    const int r = e % SW, q = e / SW;
+    T v = r == s0 + q ? T(1) : T(0);
+    if (j < nb && r / LB == j) v = I64[(int64_t)j * LB * LB + (s0 + q - LB * j) * LB + r - LB * j];
+    Xs[r * IVC + q] = v;
+  }
+  const int r = tid % LB, q0 = tid / LB * 4;  // output row, four of the strip's columns
+  // acc += As X(rows x0 ..), k in [ka, kb)
+  auto mul = [&](T (&acc)[4], const T* x, int ka, int kb) {
+#pragma unroll 4
+    for (int k = ka; k < kb; ++k) {
+      const T a = As[k * 65 + r];
 #pragma unroll
-      for (int q = 0; q < 16; ++q) acc[q] = T(0);
-      for (int k = j; k < i; ++k) {
-        // both tiles read along their stored columns (consecutive threads,
-        // consecutive addresses)
-        for (int e = tid; e < LB * LB; e += blockDim.x) {
-          const int rr = e % LB, kk = e / LB;
-          const int grow = LB * i + rr, gcol = LB * k + kk;
-          As[kk * 65 + rr] = (grow < bw && gcol < bw) ? L[(int64_t)(c0 + gcol) * f.ld + c0 + grow] : T(0);
-        }
-        for (int e = tid; e < LB * LB; e += blockDim.x) {
-          const int kk = e % LB, rr = e / LB;
-          Bs[rr * 65 + kk] = X[(int64_t)(LB * j + rr) * SW + LB * k + kk];  // B(kk, rr) = X_kj
-        }
-        __syncthreads();
+      for (int q = 0; q < 4; ++q) acc[q] += a * x[k * IVC + q0 + q];
+    }
+  };
+  for (int i = j + 1; i < nb; ++i) {
+    T acc[4] = {T(0), T(0), T(0), T(0)};
+    for (int k = j; k < i; ++k) {
+      __syncthreads();  // As is free, Xs complete
 #pragma unroll 8
-        for (int kk = 0; kk < LB; ++kk) {
-          const T a = As[kk * 65 + r];
-#pragma unroll
-          for (int q = 0; q < 16; ++q) acc[q] += a * Bs[(cq * 16 + q) * 65 + kk];
-        }
-        __syncthreads();
-      }
-      // X_ij = -Inv64_i S
-#pragma unroll
-      for (int q = 0; q < 16; ++q) Bs[(cq * 16 + q) * 65 + r] = acc[q];
-      for (int e = tid; e < LB * LB; e += blockDim.x) {
-        int rr = e % LB, kk = e / LB;
-        As[kk * 65 + rr] = I64[(int64_t)i * LB * LB + kk * LB + rr];
+      for (int e = tid; e < LB * LB; e += 256) {
+        const int rr = e % LB, kk = e / LB;
+        const int grow = LB * i + rr, gcol = LB * k + kk;
+        As[kk * 65 + rr] = (grow < bw && gcol < bw) ? L[(int64_t)gcol * f.ld + grow] : T(0);
       }
       __syncthreads();
+      mul(acc, Xs + LB * k * IVC, k == j ? s0 - LB * j : 0, LB);
+    }
+    __syncthreads();
 #pragma unroll
-      for (int q = 0; q < 16; ++q) acc[q] = T(0);
+    for (int q = 0; q < 4; ++q) Xs[(LB * i + r) * IVC + q0 + q] = acc[q];
 #pragma unroll 8
-      for (int kk = 0; kk < LB; ++kk) {
-        const T a = As[kk * 65 + r];
+    for (int e = tid; e < LB * LB; e += 256)
+      As[e / LB * 65 + e % LB] = I64[(int64_t)i * LB * LB + e];
+    __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] += a * Bs[(cq * 16 + q) * 65 + kk];
-      }
+    for (int q = 0; q < 4; ++q) acc[q] = T(0);
+    mul(acc, Xs + LB * i * IVC, 0, (r | 31) + 1);
+    __syncthreads();
 #pragma unroll
-      for (int q = 0; q < 16; ++q) X[(int64_t)(LB * j + cq * 16 + q) * SW + LB * i + r] = -acc[q];
-      __syncthreads();
-    }
-  // transposed copy, XT[k*256 + i] = X(k, i), through 64 x 64 shared tiles
-  T* XT = inv2t + inv2_off[t.f] + (int64_t)(c0 / SW) * SW * SW;
-  for (int bj = 0; bj < SW / LB; ++bj)
-    for (int bi = 0; bi < SW / LB; ++bi) {
-      for (int e = tid; e < LB * LB; e += blockDim.x) {
-        const int rr = e % LB, kk = e / LB;  // X(LB*bi + rr, LB*bj + kk)
-        As[kk * 65 + rr] = X[(int64_t)(LB * bj + kk) * SW + LB * bi + rr];
-      }
-      __syncthreads();
-      for (int e = tid; e < LB * LB; e += blockDim.x) {
-        const int kk = e % LB, rr = e / LB;  // XT(LB*bj + kk, LB*bi + rr)
-        XT[(int64_t)(LB * bi + rr) * SW + LB * bj + kk] = As[kk * 65 + rr];
-      }
-      __syncthreads();
-    }
+    for (int q = 0; q < 4; ++q) Xs[(LB * i + r) * IVC + q0 + q] = -acc[q];
+  }
+  __syncthreads();
+  // the strip, and its transposed copy XT[k*256 + i] = X(k, i)
+  T* X = inv2 + inv2_off[t.f] + (int64_t)(c0 / SW) * SW * SW + (int64_t)s0 * SW;
+  T* XT = inv2t + inv2_off[t.f] + (int64_t)(c0 / SW) * SW * SW + s0;
+  for (int e = tid; e < SW * IVC; e += 256) {
+    X[e] = Xs[(e % SW) * IVC + e / SW];
+    XT[(int64_t)(e / IVC) * SW + e % IVC] = Xs[e];
+  }
+}
+
+template <typename T>
+constexpr size_t inv_block_smem() {
+  return sizeof(T) * (SW * IVC + 64 * 65);
 }
 
 // P_ib = L_ib X_b (FP32), 64 rows per task: thread (rows 4tr .. 4tr + 3,
@@ -1701,7 +1728,7 @@ template <typename T>
 void launch_inv_diag(const T* arena, const FrontDesc* fr, const LTask* tasks, int ntask,
                      T* inv, const int64_t* inv_off, bool unit, cudaStream_t s) {
   if (ntask <= 0) return;
-  k_inv_diag<T><<<ntask, LB, 0, s>>>(arena, fr, tasks, inv, inv_off, unit);
+  k_inv_diag<T><<<ntask, 4 * LB, 0, s>>>(arena, fr, tasks, inv, inv_off, unit);
 }
 
 template <typename T, int RQ>
@@ -1715,7 +1742,7 @@ void set_rect_smem() {
 template <typename T>
 void prepare_solve_kernels() {
   SG_CUDA(cudaFuncSetAttribute(k_inv_block<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(2 * 64 * 65 * sizeof(T))));
+                               (int)inv_block_smem<T>()));
   SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, false>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_mv_smem<T, T>()));
   SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, true>,
@@ -1755,8 +1782,9 @@ void launch_inv_block(const T* arena, const FrontDesc* fr, const LTask* tasks, i
                    const T* inv64, const int64_t* inv_off, T* inv2, T* inv2t,
                    const int64_t* inv2_off, cudaStream_t s) {
   if (ntask <= 0) return;
-  k_inv_block<T><<<ntask, 256, 2 * 64 * 65 * sizeof(T), s>>>(arena, fr, tasks, inv64, inv_off,
-                                                           inv2, inv2t, inv2_off);
+  k_inv_block<T><<<ntask * (SW / IVC), 256, inv_block_smem<T>(), s>>>(arena, fr, tasks, inv64,
+                                                                      inv_off, inv2, inv2t,
+                                                                      inv2_off);
 }
 template void prepare_solve_kernels<float>();
 template void prepare_solve_kernels<double>();
