@@ -372,9 +372,10 @@ int spldlt_tree_solve_fwd_noalloc_dbl(bool posdef, void const* tree, int nrhs, d
  * front, never the arithmetic.  0 keeps the built-in default. */
 typedef struct {
   int small_front_rows;  /* Cholesky: fronts with at most this many rows are factorised whole
-                            by one CTA (capped at 96 FP64 / 128 FP32; default 96) */
+                            by one CTA (capped at 96 FP64 / 128 FP32; default 80 / 128) */
   int tc_min_cb_rows;    /* FP32 Cholesky: contribution blocks with at least this many rows
-                            use the tensor-core update (default 64; negative: never) */
+                            use the tensor-core update (default 64; negative: never, and
+                            FP64 fronts then keep to the FP64 pipe as well) */
   int solve_large_cols;  /* fronts with at least this many eliminated columns use the blocked
                             multi-CTA solve (default 96) */
   int ldlt_tpp_cols;     /* LDL^T: fronts with at most this many fully-summed columns skip the

@@ -13,6 +13,7 @@
 // Reference behaviour replaced: factorize_diag_block, solve_block
 // (src/kernels/factor.hxx:56-160).
 #include "digits.cuh"
+#include "pivot.cuh"
 
 namespace sylver_gb300 {
 
@@ -21,33 +22,6 @@ namespace {
 constexpr int PB = 32;         // panel width
 constexpr int PLD = PB + 1;
 constexpr int P64_THREADS = 128;
-
-// 1 / sqrt(d) where d has no normal exponent
-__device__ __noinline__ double rsqrt64_slow(double d) { return 1.0 / sqrt(d); }
-
-// 1 / sqrt(d), d > 0, to within 2^-59 before the rounding: the FP32 estimate
-// y0 of the mantissa's and one step y0 (1 + e / 2 + 3 e^2 / 8), e = 1 - f y0^2, in
-// integer arithmetic, whose latency is a fraction of the FP64 pipe's.
-__device__ __forceinline__ double rsqrt64(double d) {
-  const long long b = __double_as_longlong(d);
-  const int ex = (int)(b >> 52);  // d > 0: no sign bit
-  if (ex == 0 || ex == 0x7ff) return rsqrt64_slow(d);
-  const int q = (ex - 1023) >> 1, odd = (ex - 1023) & 1;
-  // d = f 4^q, f = m 2^(odd - 52) in [1, 4)
-  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (1ull << 52);
-  const float ff = __uint_as_float(((unsigned)(127 + odd) << 23) | (unsigned)((m >> 29) & 0x7fffff));
-  // y0 = Y 2^-24 in [1/2, 1)
-  const unsigned Y = min((unsigned)(rsqrtf(ff) * 16777216.f), 16777215u);
-  const unsigned long long P = (unsigned long long)Y * Y;
-  // e in units of 2^-62
-  const unsigned long long hi = __umul64hi(m << 11, P << 16);
-  const long long e = (long long)((1ull << (63 - odd)) - hi) >> (1 - odd);
-  const int t = (int)(e >> 21);
-  const long long dl = (e >> 1) + (((long long)t * t * 3) >> 23);
-  const long long y = ((long long)Y << 39) + (((long long)Y * (dl >> 4)) >> 19);
-  const unsigned long long r = (unsigned long long)(y + (1 << 9)) >> 10;  // 53 bits
-  return __longlong_as_double((long long)(((unsigned long long)(1021 - q) << 52) + r));
-}
 
 // One CTA of four warps: rows [r0, r1) of a panel.
 //   diagonal block: in blocks of eight columns; one warp, a row per lane,

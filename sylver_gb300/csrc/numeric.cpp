@@ -180,7 +180,7 @@ void FKeep::plan_cholesky() {
   const int NB = f32 ? Tiles<float>::NB : Tiles<double>::NB;
   const int RT = f32 ? Tiles<float>::RT : Tiles<double>::RT;
   const Schedule& sched = Schedule::current();
-  const int SMALL_M = sched.small_rows(f32 ? Tiles<float>::SMALL_M : Tiles<double>::SMALL_M);
+  const int SMALL_M = sched.small_rows(f32 ? Tiles<float>::SMALL_M : Tiles<double>::SMALL_M, f32);
   const int TC_ROWS = sched.tc_rows();
 
   order.resize(ns);

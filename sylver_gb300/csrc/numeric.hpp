@@ -62,10 +62,13 @@ struct Schedule {
   int solve_dataflow = 0;    // large-front solve sweeps (FP32): one dataflow launch per
                              // level (Cholesky >= 0, LDL^T > 0) or one launch per block step
   static Schedule& current();
-  // default 96 rows: measured faster than the FP32 cap of 128 on 40^3, 56^3 and
-  // 80^3 log-normal 27-point matrices (schedule sweeps of the learned scheduler)
-  int small_rows(int compiled_max) const {
-    return std::min(small_front_rows > 0 ? small_front_rows : 96, compiled_max);
+  // Default: every FP32 front its kernel takes (128 rows; 300 grids of 8^2 to
+  // 64^2 in one batch 0.99 ms, with 96 rows 1.09 ms, with 64 1.62 ms), and 80
+  // rows in FP64, where the FP64 pipe makes longer fronts faster on the panel
+  // path (grid 360x300: 2.51 ms, 96 rows 2.54, 64 rows 2.74; grid 100^2: 0.96,
+  // 0.99, 0.87).
+  int small_rows(int compiled_max, bool f32) const {
+    return std::min(small_front_rows > 0 ? small_front_rows : f32 ? 128 : 80, compiled_max);
   }
   int tc_rows() const { return tc_min_cb_rows == 0 ? 64 : tc_min_cb_rows; }
   int solve_cols() const { return solve_large_cols > 0 ? solve_large_cols : 96; }

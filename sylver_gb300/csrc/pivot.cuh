@@ -1,0 +1,55 @@
+// Reciprocal square roots of Cholesky pivots without IEEE square root and
+// division, which cost several times as long on the chain of pivots.
+#pragma once
+
+#include <cfloat>
+
+#include "device.hpp"
+
+namespace sylver_gb300 {
+
+namespace {
+
+// 1 / sqrt(d) where d has no normal exponent
+__device__ __noinline__ double rsqrt64_slow(double d) { return 1.0 / sqrt(d); }
+
+// 1 / sqrt(d), d > 0, to within 2^-59 before the rounding: the FP32 estimate
+// y0 of the mantissa's and one step y0 (1 + e / 2 + 3 e^2 / 8), e = 1 - f y0^2, in
+// integer arithmetic, whose latency is a fraction of the FP64 pipe's.
+__device__ __forceinline__ double rsqrt64(double d) {
+  const long long b = __double_as_longlong(d);
+  const int ex = (int)(b >> 52);  // d > 0: no sign bit
+  if (ex == 0 || ex == 0x7ff) return rsqrt64_slow(d);
+  const int q = (ex - 1023) >> 1, odd = (ex - 1023) & 1;
+  // d = f 4^q, f = m 2^(odd - 52) in [1, 4)
+  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (1ull << 52);
+  const float ff = __uint_as_float(((unsigned)(127 + odd) << 23) | (unsigned)((m >> 29) & 0x7fffff));
+  // y0 = Y 2^-24 in [1/2, 1)
+  const unsigned Y = min((unsigned)(rsqrtf(ff) * 16777216.f), 16777215u);
+  const unsigned long long P = (unsigned long long)Y * Y;
+  // e in units of 2^-62
+  const unsigned long long hi = __umul64hi(m << 11, P << 16);
+  const long long e = (long long)((1ull << (63 - odd)) - hi) >> (1 - odd);
+  const int t = (int)(e >> 21);
+  const long long dl = (e >> 1) + (((long long)t * t * 3) >> 23);
+  const long long y = ((long long)Y << 39) + (((long long)Y * (dl >> 4)) >> 19);
+  const unsigned long long r = (unsigned long long)(y + (1 << 9)) >> 10;  // 53 bits
+  return __longlong_as_double((long long)(((unsigned long long)(1021 - q) << 52) + r));
+}
+
+// the same in FP32: the hardware estimate and one Newton step (about 1 ulp)
+__device__ __forceinline__ float rsqrt32(float d) {
+  const float r = rsqrtf(d);
+  return d <= FLT_MAX ? r * fmaf(-0.5f * d * r, r, 1.5f) : 0.f;
+}
+__device__ __forceinline__ double pivot_rsqrt(double d) { return rsqrt64(d); }
+__device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrt32(d); }
+// sqrt(d) from r = pivot_rsqrt(d): d r corrected by its remainder
+template <typename T> __device__ __forceinline__ T pivot_sqrt(T d, T r) {
+  const T s = d * r;
+  return r > T(0) ? fma(fma(-s, s, d), T(0.5) * r, s) : d;
+}
+
+}  // namespace
+
+}  // namespace sylver_gb300
