@@ -221,6 +221,7 @@ void launch_extend_add_grouped(T* arena, const ChildDesc* cd, const EaItem* item
 // arow/asrc[acp[cbase + j], acp[cbase + j + 1]) (distinct rows >= j) and the
 // children's CB columns that land in it are items[gptr[cbase + j],
 // gptr[cbase + j + 1]) in child order (at most 32, maps that keep row order).
+constexpr int ASM_TASKS = 152 * 6;  // CTAs a level's assembly is cut into, if it can be
 struct AsmTask {
   int64_t off;
   int ld, m, j0, j1, cbase, pad;

@@ -234,7 +234,7 @@ void FKeep::plan_cholesky() {
     arena_elems = std::max<int64_t>(al.high_water(), 1);
   }
   // zeroing (or one-pass assembly) tasks: each front's lower triangle in
-  // column ranges of about 64K entries, level by level (zlv[l] = first task
+  // column ranges, level by level (zlv[l] = first task
   // of level l); colbase[k] = first column of level-ordered front k in the
   // per-column tables of the one-pass assembly
   std::vector<ZeroTask> zt;
@@ -244,13 +244,19 @@ void FKeep::plan_cholesky() {
   for (int k = 0; k < ns; ++k) colbase[k + 1] = colbase[k] + st.nrow[order[k]];
   for (size_t l = 0; l < levels.size(); ++l) {
     zlv[l] = (int64_t)zt.size();
+    // entries per task: at most 64K, fewer where a level would leave SMs
+    // without work (a CTA's eight warps take a column each)
+    int64_t total = 0;
+    for (int k = levels[l].f0; k < levels[l].f1; ++k)
+      total += (int64_t)st.nrow[order[k]] * (st.nrow[order[k]] + 1) / 2;
+    const int64_t cap = std::min<int64_t>(65536, total / ASM_TASKS);
     for (int k = levels[l].f0; k < levels[l].f1; ++k) {
       const int s = order[k], m = st.nrow[s];
       int j0 = 0;
       while (j0 < m) {
         int64_t acc = 0;
         int j1 = j0;
-        while (j1 < m && acc < 65536) acc += m - j1++;
+        while (j1 < m && (acc < cap || j1 - j0 < 8)) acc += m - j1++;
         zt.push_back({off[s], ld[s], m, j0, j1});
         at.push_back({off[s], ld[s], m, j0, j1, (int)colbase[k], 0});
         j0 = j1;
