@@ -22,6 +22,7 @@ namespace {
 constexpr int PB = 32;         // panel width
 constexpr int PLD = PB + 1;
 constexpr int P64_THREADS = 128;
+constexpr int NUM_SMS = 152;
 
 // One CTA of four warps: rows [r0, r1) of a panel.
 //   diagonal block: in blocks of eight columns; one warp, a row per lane,
@@ -73,7 +74,8 @@ __global__ void __launch_bounds__(P64_THREADS)
   bool bad = false;
 #pragma unroll 1
   for (int b = 0; b < PB; b += CB) {
-    if (warp == (b / CB)) {
+    // (another scheduler's FP64 pipe in each of the CTAs that share an SM)
+    if (warp == ((b / CB + blockIdx.x / NUM_SMS) & 3)) {
       double c[CB];
 #pragma unroll
       for (int u = 0; u < CB; ++u) c[u] = Ls[(b + u) * PLD + lane];

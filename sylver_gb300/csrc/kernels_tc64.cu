@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapa) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapb) : "memory");
     for (int s = 0; s < OZ_STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
@@ -234,10 +236,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   } else {
     // TMEM lanes [32q, 32q + 32) are this warp's, and columns [32h, 32h + 32)
     // of each tile
+    // (of a tile of at most 32 columns: [16h, 16h + 16))
     const int q = warp & 3, h = (warp - OZ_EPI_WARP0) >> 2;
-    const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * 32);
     int it = 0;
     bool ok = true;
+    uint32_t ta = 0;  // this warp's columns of accumulator 0
     // wait for group gr's accumulator and start its read into v (warp-uniform:
     // tcgen05.ld is a warp-collective instruction)
     auto fetch = [&](int gr, uint32_t (&v)[32]) {
@@ -259,12 +262,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     for (int ti = blockIdx.x; ti < ntask && ok; ti += gridDim.x) {
       const TcTask t = tasks[ti];
       const int rt = q * 32 + lane, row = t.row0 + rt;
-      const int c0 = t.col0 + h * 32;
-      const bool on = c0 < t.colEnd;  // warp-uniform
+      const int hw = t.colEnd - t.col0 <= 32 ? 16 : 32;
+      ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * hw);
+      const int c0 = t.col0 + h * hw, ce = min(t.colEnd, c0 + hw);
+      const bool on = c0 < ce;  // warp-uniform
       const bool has = row < t.rowEnd;
       // row exponent; lane j holds column c0 + j's
       const int ei = has ? sexp[t.a_row + rt] : 0;
-      const int ejl = c0 + lane < t.colEnd ? sexp[t.b_row + h * 32 + lane] : 0;
+      const int ejl = c0 + lane < ce ? sexp[t.b_row + h * hw + lane] : 0;
       long long acc[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) acc[j] = 0;
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       if (!ok) break;
       if (!on) continue;
       // columns [c0, cend) of this row are updated (lower triangle, in range)
-      const int cend = has ? min(t.colEnd, row + 1) : c0;
+      const int cend = has ? min(ce, row + 1) : c0;
       const bool safe = __all_sync(0xffffffffu, abs(ei) <= OZ_EXP_SAFE / 2 &&
                                                     abs(ejl) <= OZ_EXP_SAFE / 2);
       double* cp = arena + t.c_off + row + (int64_t)c0 * t.ldc;
@@ -307,6 +312,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       for (int j = 0; j < 8; ++j) cv[0][j] = c0 + j < cend ? cp[(int64_t)j * t.ldc] : 0.0;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
+        if (c0 + 8 * b >= ce) break;  // warp-uniform
         if (b < 3) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
