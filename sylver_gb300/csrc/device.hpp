@@ -243,7 +243,8 @@ void launch_diag_chol(T* arena, const PanelTask* t, int ntask, unsigned* status,
 template <typename T>
 void launch_panel_trsm(T* arena, const PanelTask* t, int ntask, cudaStream_t s);
 template <typename T>
-void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, cudaStream_t s);
+void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, int tile,
+                   cudaStream_t s);
 
 // Launchers (kernels_blocked.cu), FP32 only.  xinv holds one 64 x 64
 // inverse per diagonal-block task of the launch.

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256) k_assemble(T* __restrict__ arena,
 
 // ---------------------------------------------------------------------------
 // Whole-front partial Cholesky in shared memory (m <= SMALL_M): the first n
-// columns are eliminated in blocks of eight.  Per block, warp 0 factorises it
+// columns are eliminated in blocks of eight.  Per block, one warp factorises it
 // with a row per lane (rows b .. b + 31) in registers, the threads solve the
 // rows further down, and all of them update the triangle behind it by register
 // tiles.  Bound by latency (FP32) and by the FP64 pipe: a rank-1 step
@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(256) k_small_chol(T* __restrict__ arena,
 #pragma unroll 1
   for (int b = 0; b < n; b += 8) {
     const int w = min(8, n - b);
-    if (warp == 0) {
+    // (CTAs that share an SM spread over its schedulers)
+    if (warp == (blockIdx.x / 152 & 7)) {
       const int i = b + lane;
       T c[8], d[8], r[8];
 #pragma unroll
@@ -592,9 +593,13 @@ void launch_panel_trsm(T* arena, const PanelTask* t, int ntask, cudaStream_t s) 
 }
 
 template <typename T>
-void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, cudaStream_t s) {
+void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, int tile,
+                   cudaStream_t s) {
   if (ntask <= 0) return;
-  k_update<T, Tiles<T>::TM, Tiles<T>::TN, 16><<<ntask, 256, 0, s>>>(arena, abuf, t);
+  if (sizeof(T) == 8 && tile == Tiles<T>::TM / 2)
+    k_update<T, Tiles<T>::TM / 2, Tiles<T>::TN / 2, 16><<<ntask, 256, 0, s>>>(arena, abuf, t);
+  else
+    k_update<T, Tiles<T>::TM, Tiles<T>::TN, 16><<<ntask, 256, 0, s>>>(arena, abuf, t);
 }
 
 #define SG_INST(T)                                                                          \
@@ -612,7 +617,7 @@ void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, cudaStr
                                    const int*, const int64_t*, const int*, const EaItem*,   \
                                    const ChildDesc*, const int*, cudaStream_t);             \
   template void launch_small_chol<T>(T*, const SmallTask*, int, int, unsigned*, cudaStream_t); \
-  template void launch_update<T>(T*, const T*, const UpdTask*, int, cudaStream_t);
+  template void launch_update<T>(T*, const T*, const UpdTask*, int, int, cudaStream_t);
 SG_INST(float)
 SG_INST(double)
 #undef SG_INST

@@ -530,6 +530,19 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       int pitch = 0;
       const bool tc_ok = std::is_same<T, float>::value && fk.use_tc;
       const int tc_min = Schedule::current().tc_rows();
+      // FP64 tiles of half the size while the level's full-size ones are fewer
+      // than four per SM: a 64 x 64 tile keeps one SM's FP64 pipe busy for
+      // 1.2 us per column, and the levels near the root have a few dozen
+      // (14^3 saddle point: 92 us a level in 64 x 64 tiles)
+      int UT = TM;
+      if (sizeof(T) == 8) {
+        int64_t nt = 0;
+        for (int s2 : F) {
+          const int64_t c = ceil_div(L.m[s2] - L.n[s2], TM);
+          nt += c * (c + 1) / 2;
+        }
+        if (nt < 4 * 152) UT = TM / 2;
+      }
       for (int q = 0; q < nslot; ++q) {
         int s2 = F[q];
         int m = L.m[s2], n = L.n[s2], ne = L.nelim[s2];
@@ -555,9 +568,9 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
               tct.push_back({f.off, f.ld, n + ri * 128, n + cj * 128, m, m,
                              (int)(bd + ri * 128), (int)(bl + cj * 128), nk, 0});
         } else {
-          for (int cj = 0; n + cj * TM < m; ++cj)
-            for (int ri = cj; n + ri * TM < m; ++ri)
-              ut.push_back({f.off, f.ldp_off, f.off, f.ld, m, f.ld, n + ri * TM, n + cj * TM, m,
+          for (int cj = 0; n + cj * UT < m; ++cj)
+            for (int ri = cj; n + ri * UT < m; ++ri)
+              ut.push_back({f.off, f.ldp_off, f.off, f.ld, m, f.ld, n + ri * UT, n + cj * UT, m,
                             m, 0, ne, 0});
         }
       }
@@ -571,7 +584,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
         launches++;
         if (!ut.empty()) {
           put(L.up, ut, s);
-          launch_update<T>(A, L.sc2.as<T>(), L.up.as<UpdTask>(), (int)ut.size(), s);
+          launch_update<T>(A, L.sc2.as<T>(), L.up.as<UpdTask>(), (int)ut.size(), UT, s);
           launches++;
         }
         if constexpr (std::is_same<T, float>::value) {

@@ -941,7 +941,7 @@ void FKeep::run_ops(cudaStream_t s) {
                          op.aux >= 0 ? tclev[op.aux].pitch : 0, ozexp.as<int>(), stp, s);
         break;
       case Op::UPD:
-        launch_update<T>(A, A, upd.as<UpdTask>() + op.a, (int)cnt, s);
+        launch_update<T>(A, A, upd.as<UpdTask>() + op.a, (int)cnt, Tiles<T>::TM, s);
         break;
       case Op::INV:
         splan.compute_inverses<T>(A, dfr.as<FrontDesc>(), false, s);
