@@ -334,11 +334,16 @@ constexpr int LSOLVE_BW2 = 256;  // columns per solve step (diagonal block with 
 constexpr int LSOLVE_TW = 256;   // columns of the L tiles of the update and reduction tasks
 constexpr int LSOLVE_UPD_ROWS = 32;  // rows per forward-update CTA
 constexpr int LSOLVE_RED_ROWS = 64;  // rows per backward-reduction CTA
-constexpr int RECT_FWD_T = 128;      // threads of an LS_RECT_FWD task (two contribution rows each)
-constexpr int RECT_FWD_COLS = 128;   // pivot columns per LS_RECT_FWD task (partial sums add atomically)
-constexpr int RECT_BWD_COLS = 128;   // pivot columns per LS_RECT_BWD task
-constexpr int RECT_BWD_T = 128;      // threads of an LS_RECT_BWD task (two columns each, two row halves)
-constexpr int RECT_BWD_ROWS = 256;   // contribution rows per LS_RECT_BWD task
+// Contribution-row tasks: LS_RECT_FWD takes rect_fwd_rows x RECT_FWD_COLS of L,
+// LS_RECT_BWD RECT_BWD_ROWS x rect_bwd_cols.  FP64 tasks have a quarter of the
+// rows (columns): one SM's FP64 pipe takes 38 us for 256 x 128 entries times 4
+// right-hand sides, and a level may have fewer tasks than SMs.  The side that is
+// summed over stays long, so that each row (column) takes as few additions.
+constexpr int RECT_FWD_T = 128, RECT_BWD_T = 128;  // threads
+constexpr int RECT_FWD_COLS = 128;
+constexpr int RECT_BWD_ROWS = 256;
+constexpr int rect_fwd_rows(size_t elem) { return elem == 8 ? 64 : 256; }
+constexpr int rect_bwd_cols(size_t elem) { return elem == 8 ? 32 : 128; }
 // Large fronts are swept block by block over their fully-summed rows only.
 // The contribution rows (>= n) of every front of a level are one separate
 // launch per direction: forward after the pivot rows are solved (x(cb) -=
@@ -376,10 +381,8 @@ struct LsArgs {
   int* dfc;
   const int2* dfo;
   const int64_t* ttoff;
-  // dataflow sweeps (FP32): the products P_ib = L_ib X_b; pmode: the
-  // backward sweep leaves z in the xs slab for the scatter
+  // dataflow sweeps (FP32): the products P_ib = L_ib X_b
   const T* pmat;
-  int pmode;
 };
 // Inverse of each solve-step diagonal block (LSOLVE_BW2 columns) from its
 // 64x64 inverses: task (front f, c0, bw), output at inv2 + inv2_off[f] +

@@ -21,7 +21,7 @@ extern "C" int sylver_gb300_dataflow_selftest(int starve, unsigned* status, doub
     prepare_solve_kernels<float>();
     const int n = 32;
     const cudaStream_t s = rt.stream;
-    DevMem fr, scr, xs, ys, tt, ttoff, cnt, dfo, tasks, err, pm;
+    DevMem fr, scr, xs, ys, tt, ttoff, cnt, dfo, tasks, err, pm, rl, x;
     std::vector<FrontDesc> hfr(1);
     hfr[0] = FrontDesc{};
     hfr[0].off = 0;
@@ -32,6 +32,10 @@ extern "C" int sylver_gb300_dataflow_selftest(int starve, unsigned* status, doub
     scr.upload(std::vector<int64_t>{0}, s);
     ttoff.upload(std::vector<int64_t>{0}, s);
     dfo.upload(std::vector<int2>{make_int2(1, 4)}, s);
+    std::vector<int> rows(n);
+    for (int i = 0; i < n; ++i) rows[i] = i;
+    rl.upload(rows, s);
+    x.ensure(n * sizeof(float));
     xs.ensure(n * sizeof(float));
     ys.ensure(n * sizeof(float));
     tt.ensure((size_t)LSOLVE_BW2 * 32 * sizeof(float));
@@ -49,6 +53,8 @@ extern "C" int sylver_gb300_dataflow_selftest(int starve, unsigned* status, doub
     SG_CUDA(cudaMemsetAsync(err.p, 0, sizeof(unsigned), s));
     LsArgs<float, float> a{};
     a.fr = fr.as<FrontDesc>();
+    a.rlist = rl.as<int>();
+    a.x = x.as<float>();
     a.nrhs = 1;
     a.n = n;
     a.scratch = xs.as<float>();
@@ -59,7 +65,6 @@ extern "C" int sylver_gb300_dataflow_selftest(int starve, unsigned* status, doub
     a.dfo = dfo.as<int2>();
     a.ttoff = ttoff.as<int64_t>();
     a.pmat = pm.as<float>();
-    a.pmode = 1;
     SG_CUDA(cudaStreamSynchronize(s));
     const auto t0 = std::chrono::steady_clock::now();
     launch_chain(true, tasks.as<DfTask>(), 1, a, err.as<unsigned>(), s);

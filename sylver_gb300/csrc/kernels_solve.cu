@@ -12,6 +12,8 @@
 // blocks (warp 0 solves the diagonal block with shuffles, all warps apply the
 // off-diagonal block), and scattered back; rows below the pivots go to
 // ancestors with atomics because sibling fronts of a level share them.
+#include <type_traits>
+
 #include "device.hpp"
 
 namespace sylver_gb300 {
@@ -25,9 +27,15 @@ constexpr int GB = 8;       // gather/scatter elements in flight per thread
 // dynamic shared memory of the small-front triangle kernel (pivot rows of the
 // right-hand sides and their destinations)
 constexpr size_t TRI_SMEM = 96 * 1024;
-// right-hand sides per pass of the contribution-row kernels: 4 for a few,
-// else 16 (FP32) / 8 (FP64), more in several passes
-template <typename ACC> constexpr int RQ_MID = sizeof(ACC) == 8 ? 8 : 16;
+// Right-hand sides per pass of the sweeps' products.  FP32: 4 for a few, else
+// 16.  FP64: 1, 2, 4, 6 or 8, the fewest that need no more passes -- the FP64
+// pipe does two multiply-adds per clock and SM, so columns that a pass holds
+// but the call does not have cost as much as real ones.
+inline int rhs_per_pass(int nrhs, bool f64) {
+  if (!f64) return nrhs <= 4 ? 4 : 16;
+  const int np = (nrhs + 7) / 8, need = (nrhs + np - 1) / np;
+  return need <= 2 ? need : (need + 1) / 2 * 2;
+}
 
 template <typename T> __device__ __forceinline__ void aadd(T* p, T v) { atomicAdd(p, v); }
 
@@ -234,13 +242,31 @@ __global__ void __launch_bounds__(256) k_tri(const T* __restrict__ arena,
 #pragma unroll
       for (int u = 0; u < SB * SB / 256; ++u) {
         const int e = tid + 256 * u, i = e % SB, k = e / SB;
-        lv[u] = (i < bw && k < bw) ? (ACC)L[(int64_t)(c0 + k) * ld + c0 + i] : ACC(0);
+        lv[u] = (i < bw && k < bw) ? (ACC)L[(int64_t)(c0 + k) * ld + c0 + i] : ACC(i == k);
       }
+      if (unit) {
 #pragma unroll
-      for (int u = 0; u < SB * SB / 256; ++u) {
-        const int e = tid + 256 * u;
-        Ld[e / SB][e % SB] = lv[u];
-        if (e % SB == e / SB) rdg[e % SB] = (e % SB < bw && !unit) ? ACC(1) / lv[u] : ACC(1);
+        for (int u = 0; u < SB * SB / 256; ++u) {
+          const int e = tid + 256 * u;
+          Ld[e / SB][e % SB] = lv[u];
+          if (tid < SB) rdg[tid] = ACC(1);
+        }
+      } else {
+        // the substitution runs on z = x L(k, k): L by 1 / L(k, k), k the
+        // column whose x a step subtracts (one warp takes the reciprocals)
+#pragma unroll
+        for (int u = 0; u < SB * SB / 256; ++u) {
+          const int e = tid + 256 * u;
+          if (e % SB == e / SB) rdg[e % SB] = lv[u];
+        }
+        __syncthreads();
+        if (warp == 0) rdg[lane] = ACC(1) / rdg[lane];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < SB * SB / 256; ++u) {
+          const int e = tid + 256 * u;
+          Ld[e / SB][e % SB] = lv[u] * rdg[BWD ? e % SB : e / SB];
+        }
       }
     }
     __syncthreads();
@@ -258,35 +284,35 @@ __global__ void __launch_bounds__(256) k_tri(const T* __restrict__ arena,
         }
       }
       __syncwarp();  // converged before the shuffle chain
-      if (!BWD) {
-        for (int kk = 0; kk < bw; ++kk) {
-          const ACC vk = __shfl_sync(0xffffffffu, v, kk) * rdg[kk];
-          const ACC wk = __shfl_sync(0xffffffffu, w, kk) * rdg[kk];
-          if (lane == kk) {
-            v = vk;
-            w = wk;
+      // one shuffle and one multiply-add per step (two with a second right-hand side)
+      auto chain = [&](auto dual) {
+        constexpr bool D = decltype(dual)::value;
+        if (!BWD) {
+          for (int kk = 0; kk < bw; ++kk) {
+            const ACC zk = __shfl_sync(0xffffffffu, v, kk);
+            const ACC zw = D ? __shfl_sync(0xffffffffu, w, kk) : ACC(0);
+            if (lane > kk) {
+              const ACC l = Ld[kk][lane];
+              v -= l * zk;
+              if (D) w -= l * zw;
+            }
           }
-          if (lane > kk && lane < bw) {
-            const ACC l = Ld[kk][lane];
-            v -= l * vk;
-            w -= l * wk;
-          }
-        }
-      } else {
-        for (int kk = bw - 1; kk >= 0; --kk) {
-          if (lane == kk) {
-            v = v * rdg[kk];
-            w = w * rdg[kk];
-          }
-          const ACC zk = __shfl_sync(0xffffffffu, v, kk);
-          const ACC zw = __shfl_sync(0xffffffffu, w, kk);
-          if (lane < kk) {
-            const ACC l = Ld[lane][kk];
-            v -= l * zk;
-            w -= l * zw;
+        } else {
+          for (int kk = bw - 1; kk >= 0; --kk) {
+            const ACC zk = __shfl_sync(0xffffffffu, v, kk);
+            const ACC zw = D ? __shfl_sync(0xffffffffu, w, kk) : ACC(0);
+            if (lane < kk) {
+              const ACC l = Ld[lane][kk];
+              v -= l * zk;
+              if (D) w -= l * zw;
+            }
           }
         }
-      }
+        v *= rdg[lane];
+        if (D) w *= rdg[lane];
+      };
+      if (two) chain(std::true_type{});
+      else chain(std::false_type{});
       if (lane < bw) {
         ys[r * nc + c0 + lane] = v;
         if (two) ys[r2 * nc + c0 + lane] = w;
@@ -532,15 +558,15 @@ __device__ __forceinline__ void gather_body(const LTask& t, const LsArgs<T, ACC>
     if (r < a.nrhs) xs[(int64_t)r * f.m + i] = val[r];
 }
 
-// Scatter of the solved pivot rows (ys) of a large front back to x.
+// Scatter of the solved pivot rows (ys) of a large front back to x (block-step
+// launches; the dataflow sweeps store them there themselves).
 template <typename T, typename ACC>
-__device__ __forceinline__ void scatter_body(const LTask& t, const LsArgs<T, ACC>& a, bool fwd) {
+__device__ __forceinline__ void scatter_body(const LTask& t, const LsArgs<T, ACC>& a) {
   const FrontDesc f = a.fr[t.f];
   const int i = t.r0 + threadIdx.x;
   if (threadIdx.x >= 256 || i >= f.n) return;
   const int v = a.rlist[f.rl + i];
-  // the backward sweep with P leaves z in the xs slab
-  const ACC* src = (a.pmode && !fwd ? a.scratch : a.ys) + a.scr_off[t.f] * a.nrhs + i;
+  const ACC* src = a.ys + a.scr_off[t.f] * a.nrhs + i;
   ACC val[MAXR];
 #pragma unroll
   for (int r = 0; r < MAXR; ++r) val[r] = r < a.nrhs ? src[(int64_t)r * f.m] : ACC(0);
@@ -555,8 +581,8 @@ __global__ void k_lgather(const LTask* __restrict__ tasks, LsArgs<T, ACC> a, boo
 }
 
 template <typename T, typename ACC>
-__global__ void k_lscatter(const LTask* __restrict__ tasks, LsArgs<T, ACC> a, bool fwd) {
-  scatter_body<T, ACC>(tasks[blockIdx.x], a, fwd);
+__global__ void k_lscatter(const LTask* __restrict__ tasks, LsArgs<T, ACC> a) {
+  scatter_body<T, ACC>(tasks[blockIdx.x], a);
 }
 
 // X = L^-1 for one LB x LB diagonal block (identity beyond bw): four lanes per
@@ -598,8 +624,10 @@ __global__ void __launch_bounds__(4 * LB) k_inv_diag(const T* __restrict__ arena
   }
   __syncthreads();
   constexpr int NU = LB / 4;
-  const int lane = tid & 31, c = lane & 3, j = tid >> 2;
-  const int w8 = (tid >> 5) * 8;  // first column of this warp: rows above are zero
+  // eight columns per warp, long and short ones on each scheduler
+  const int lane = tid & 31, c = lane & 3, wq = tid >> 5;
+  const int w8 = 8 * (wq < 4 ? wq : 11 - wq);  // first column: rows above are zero
+  const int j = w8 + (lane >> 2);
   T z[NU];
 #pragma unroll
   for (int u = 0; u < NU; ++u) z[u] = 4 * u + c == j ? T(1) : T(0);
@@ -642,7 +670,9 @@ template <typename ACC> struct RGn { static constexpr int v = sizeof(ACC) == 8 ?
 // 16 bytes so that the transposing stores (consecutive lanes, consecutive k)
 // spread over the banks (4-way instead of 16-way conflicts for FP32) while
 // rows stay 16-byte aligned for the vector reads.
-template <typename ACC> struct RGP { static constexpr int v = RGn<ACC>::v + 16 / (int)sizeof(ACC); };
+template <typename ACC, int RG = RGn<ACC>::v> struct RGP {
+  static constexpr int v = RG == 1 ? 1 : RG + 16 / (int)sizeof(ACC);
+};
 
 // X = inverse of the SW-column diagonal block of a step (column-major, ld SW,
 // lower): X_jj = Inv64_j and X_ij = -Inv64_i * sum_{k=j}^{i-1} L_ik X_kj for
@@ -809,6 +839,13 @@ template <> struct Vec4<double> {
   using V = double2;
   static constexpr int W = 2;
 };
+// vector reads of a row of RG right-hand sides (single values when RG is one)
+template <typename ACC, int RG> struct RhsVec {
+  static constexpr bool vec = RG % Vec4<ACC>::W == 0;
+  static_assert(vec || RG == 1, "right-hand sides per pass");
+  static constexpr int W = vec ? Vec4<ACC>::W : 1;
+  using V = typename std::conditional<vec, typename Vec4<ACC>::V, ACC>::type;
+};
 
 // Diagonal block of a 256-column step as a product with its explicit
 // inverse, DR output rows per task (256 / DR tasks per block), 256 threads:
@@ -821,9 +858,10 @@ template <> struct Vec4<double> {
 // backward launch reads accumulator (c0/256)&1 and clears the other one,
 // which the next (lower) block's reduction fills.  The inverse slice is
 // staged before the wait for the data earlier steps write.
-template <typename T, typename ACC, int DR = DMV_ROWS> constexpr size_t diag_mv_smem() {
+template <typename T, typename ACC, int DR = DMV_ROWS, int RG = RGn<ACC>::v>
+constexpr size_t diag_mv_smem() {
   return sizeof(T) * DR * SW +
-         sizeof(ACC) * ((256 / DR) * DR * (RGn<ACC>::v + 1) + SW * RGP<ACC>::v);
+         sizeof(ACC) * ((256 / DR) * DR * (RG + 1) + SW * RGP<ACC, RG>::v);
 }
 // MODE 0: one launch per step (programmatic dependent launch, two backward
 // accumulators per front used in turn); MODE 1: a task of a dataflow sweep
@@ -842,14 +880,14 @@ template <typename T> struct PSrc {
   int64_t ld = 0;
   bool writer = false;
 };
-template <typename T, typename ACC, bool BWD, int DR, int MODE, typename W>
+template <typename T, typename ACC, bool BWD, int DR, int MODE, int RG, typename W>
 __device__ __forceinline__ void diag_body(const LTask& t, int sub, const LsArgs<T, ACC>& a,
                                           unsigned char* dsm, const W& wait) {
-  constexpr int RG = RGn<ACC>::v, RS = RGP<ACC>::v;
+  constexpr int RS = RGP<ACC, RG>::v;
   // DR output rows per task; 256 / DR k-phases per row
   constexpr int NG = 256 / DR;
-  using V = typename Vec4<ACC>::V;
-  constexpr int VW = Vec4<ACC>::W;
+  using V = typename RhsVec<ACC, RG>::V;
+  constexpr int VW = RhsVec<ACC, RG>::W;
   T* Ms = reinterpret_cast<T*>(dsm);  // Ms[(k - klo)*DR + il] = M(i0 + il, k)
   ACC* part = reinterpret_cast<ACC*>(dsm + sizeof(T) * DR * SW);  // [NG][DR][RG + 1]
   ACC* vb = part + NG * DR * (RG + 1);                               // [SW][RG]
@@ -883,7 +921,7 @@ __device__ __forceinline__ void diag_body(const LTask& t, int sub, const LsArgs<
     __syncthreads();
     {
       // all loads of the slab issued before any is used (nk * RG <= 256 NL)
-      constexpr int NL = SW * RG / 256;
+      constexpr int NL = (SW * RG + 255) / 256;
       ACC v[NL];
 #pragma unroll
       for (int u = 0; u < NL; ++u) {
@@ -920,9 +958,11 @@ __device__ __forceinline__ void diag_body(const LTask& t, int sub, const LsArgs<
             acc[4 * q + 1] += l * x4.y;
             acc[4 * q + 2] += l * x4.z;
             acc[4 * q + 3] += l * x4.w;
-          } else {
+          } else if constexpr (VW == 2) {
             acc[2 * q + 0] += l * x4.x;
             acc[2 * q + 1] += l * x4.y;
+          } else {
+            acc[q] += l * x4;
           }
         }
       }
@@ -936,7 +976,9 @@ __device__ __forceinline__ void diag_body(const LTask& t, int sub, const LsArgs<
         ACC sum = ACC(0);
 #pragma unroll
         for (int gg = 0; gg < NG; ++gg) sum += part[(gg * DR + rr) * (RG + 1) + q];
-        ysl[(int64_t)(rg + q) * m + c0 + ii] = sum;
+        // (forward dataflow sweeps: y is final, nothing in the sweep reads it)
+        if (MODE == 1 && !BWD) a.x[(int64_t)(rg + q) * a.n + a.rlist[f.rl + c0 + ii]] = sum;
+        else ysl[(int64_t)(rg + q) * m + c0 + ii] = sum;
       }
     }
   }
@@ -948,17 +990,17 @@ __device__ __forceinline__ void diag_body(const LTask& t, int sub, const LsArgs<
 // NT threads, thread (row, column group g of 256 / (NT/32) columns).  The
 // 32 x 256 tile of L is staged in shared memory by one wave of asynchronous
 // copies; y is read as 16-byte vectors (one broadcast per warp).
-template <typename T, typename ACC, int NT> constexpr size_t upd_smem() {
+template <typename T, typename ACC, int NT, int RG = RGn<ACC>::v> constexpr size_t upd_smem() {
   return sizeof(T) * 32 * TW +
-         sizeof(ACC) * ((NT / 32) * 32 * (RGn<ACC>::v + 1) + TW * RGP<ACC>::v);
+         sizeof(ACC) * ((NT / 32) * 32 * (RG + 1) + TW * RGP<ACC, RG>::v);
 }
-template <typename T, typename ACC, int NT, int MODE, typename W>
+template <typename T, typename ACC, int NT, int MODE, int RG, typename W>
 __device__ __forceinline__ void upd_body(const LTask& t, const LsArgs<T, ACC>& a,
                                          unsigned char* dsm, const W& wait,
                                          const PSrc<T>& ps = PSrc<T>{}) {
-  constexpr int RG = RGn<ACC>::v, RS = RGP<ACC>::v, NGU = NT / 32, KPG = TW / NGU;
-  using V = typename Vec4<ACC>::V;
-  constexpr int VW = Vec4<ACC>::W;
+  constexpr int RS = RGP<ACC, RG>::v, NGU = NT / 32, KPG = TW / NGU;
+  using V = typename RhsVec<ACC, RG>::V;
+  constexpr int VW = RhsVec<ACC, RG>::W;
   T* Lt = reinterpret_cast<T*>(dsm);  // Lt[k*32 + rr] = L(r0 + rr, c0 + k)
   ACC* red = reinterpret_cast<ACC*>(dsm + sizeof(T) * 32 * TW);  // [NGU][32][RG + 1]
   ACC* yb = red + NGU * 32 * (RG + 1);                              // [TW][RG]
@@ -1012,7 +1054,7 @@ __device__ __forceinline__ void upd_body(const LTask& t, const LsArgs<T, ACC>& a
         }
       }
       {
-        constexpr int NL = TW * RG / NT;
+        constexpr int NL = (TW * RG + NT - 1) / NT;
         ACC v[NL];
 #pragma unroll
         for (int u = 0; u < NL; ++u) {
@@ -1022,7 +1064,7 @@ __device__ __forceinline__ void upd_body(const LTask& t, const LsArgs<T, ACC>& a
 #pragma unroll
         for (int u = 0; u < NL; ++u) {
           const int e = tid + NT * u;
-          yb[(e % TW) * RS + e / TW] = v[u];
+          if (e < TW * RG) yb[(e % TW) * RS + e / TW] = v[u];
         }
       }
       cp_async_wait_all();
@@ -1040,9 +1082,11 @@ __device__ __forceinline__ void upd_body(const LTask& t, const LsArgs<T, ACC>& a
             acc[4 * q + 1] += l * y4.y;
             acc[4 * q + 2] += l * y4.z;
             acc[4 * q + 3] += l * y4.w;
-          } else {
+          } else if constexpr (VW == 2) {
             acc[2 * q + 0] += l * y4.x;
             acc[2 * q + 1] += l * y4.y;
+          } else {
+            acc[q] += l * y4;
           }
         }
       }
@@ -1072,16 +1116,17 @@ __device__ __forceinline__ void upd_body(const LTask& t, const LsArgs<T, ACC>& a
 // memory.  Every task of a step adds into the same accumulator; the
 // contribution rows' share was put into tacc by k_rect_bwd and taken out by
 // the gather.
-template <typename T, typename ACC> constexpr size_t red_smem() {
-  return sizeof(T) * 32 * (TW + 1) + sizeof(ACC) * (TW * (RGn<ACC>::v + 1) + 32 * RGP<ACC>::v);
+template <typename T, typename ACC, int RG = RGn<ACC>::v> constexpr size_t red_smem() {
+  return sizeof(T) * 32 * (TW + 1) +
+         sizeof(ACC) * (TW * (RG + 1) + (32 * RGP<ACC, RG>::v + 1) / 2 * 2);
 }
-template <typename T, typename ACC, int NT, int MODE, typename W>
+template <typename T, typename ACC, int NT, int MODE, int RG, typename W>
 __device__ __forceinline__ void red_body(const LTask& t, const LsArgs<T, ACC>& a,
                                          unsigned char* dsm, const W& wait,
                                          const PSrc<T>& ps = PSrc<T>{}) {
-  constexpr int RG = RGn<ACC>::v, RS = RGP<ACC>::v, SR = 32, NH = NT / TW;
-  using V = typename Vec4<ACC>::V;
-  constexpr int VW = Vec4<ACC>::W;
+  constexpr int RS = RGP<ACC, RG>::v, SR = 32, NH = NT / TW;
+  using V = typename RhsVec<ACC, RG>::V;
+  constexpr int VW = RhsVec<ACC, RG>::W;
   T* Lt = reinterpret_cast<T*>(dsm);  // Lt[ii*(TW+1) + k] = L(s0 + ii, c0 + k)
   ACC* half = reinterpret_cast<ACC*>(dsm + sizeof(T) * SR * (TW + 1));  // [TW][RG + 1]
   ACC* xt = half + TW * (RG + 1);                                         // [SR][RG]
@@ -1124,7 +1169,7 @@ __device__ __forceinline__ void red_body(const LTask& t, const LsArgs<T, ACC>& a
             // z = u - t of the row's block (complete: the wait covered it)
             const int row = s0 + ii, jb = row / SW;
             z -= __ldcg(&a.tt[a.ttoff[t.f] + ((int64_t)jb * MAXR + rg + r) * SW + (row - jb * SW)]);
-            if (ps.writer) xs[xi] = z;
+            if (ps.writer) a.x[(int64_t)(rg + r) * a.n + a.rlist[f.rl + row]] = z;
           }
         }
         xt[ii * RS + r] = z;
@@ -1144,9 +1189,11 @@ __device__ __forceinline__ void red_body(const LTask& t, const LsArgs<T, ACC>& a
             acc[4 * q + 1] += l * x4.y;
             acc[4 * q + 2] += l * x4.z;
             acc[4 * q + 3] += l * x4.w;
-          } else {
+          } else if constexpr (VW == 2) {
             acc[2 * q + 0] += l * x4.x;
             acc[2 * q + 1] += l * x4.y;
+          } else {
+            acc[q] += l * x4;
           }
         }
       }
@@ -1165,23 +1212,23 @@ __device__ __forceinline__ void red_body(const LTask& t, const LsArgs<T, ACC>& a
   }
 }
 
-template <typename T, typename ACC, bool BWD>
+template <typename T, typename ACC, bool BWD, int RG>
 __global__ void __launch_bounds__(256) k_diag_mv(const LTask* __restrict__ tasks,
                                                  LsArgs<T, ACC> a) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  diag_body<T, ACC, BWD, DMV_ROWS, 0>(tasks[blockIdx.x], blockIdx.y, a, dsm, PdlWait{});
+  diag_body<T, ACC, BWD, DMV_ROWS, 0, RG>(tasks[blockIdx.x], blockIdx.y, a, dsm, PdlWait{});
 }
-template <typename T, typename ACC>
+template <typename T, typename ACC, int RG>
 __global__ void __launch_bounds__(512) k_fwd_upd3(const LTask* __restrict__ tasks,
                                                   LsArgs<T, ACC> a) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  upd_body<T, ACC, 512, 0>(tasks[blockIdx.x], a, dsm, PdlWait{});
+  upd_body<T, ACC, 512, 0, RG>(tasks[blockIdx.x], a, dsm, PdlWait{});
 }
-template <typename T, typename ACC>
+template <typename T, typename ACC, int RG>
 __global__ void __launch_bounds__(512) k_bwd_red3(const LTask* __restrict__ tasks,
                                                   LsArgs<T, ACC> a) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  red_body<T, ACC, 512, 0>(tasks[blockIdx.x], a, dsm, PdlWait{});
+  red_body<T, ACC, 512, 0, RG>(tasks[blockIdx.x], a, dsm, PdlWait{});
 }
 
 // ---------------------------------------------------------------------------
@@ -1239,7 +1286,6 @@ struct DfWait {
 template <typename T, typename ACC, typename W>
 __device__ __forceinline__ void fin_body(const LTask& t, const LsArgs<T, ACC>& a, const W& wait) {
   const FrontDesc f = a.fr[t.f];
-  ACC* xs = a.scratch + a.scr_off[t.f] * a.nrhs;
   const ACC* ysl = a.ys + a.scr_off[t.f] * a.nrhs;
   const ACC* tb = a.tt + a.ttoff[t.f];
   const int nrow = min(32, f.n - t.r0);
@@ -1247,13 +1293,13 @@ __device__ __forceinline__ void fin_body(const LTask& t, const LsArgs<T, ACC>& a
   for (int e = threadIdx.x; e < 32 * a.nrhs; e += blockDim.x) {
     const int ii = e % 32, r = e / 32, row = t.r0 + ii;
     if (ii < nrow) {
-      const int64_t xi = (int64_t)r * f.m + row;
-      xs[xi] = __ldcg(&ysl[xi]) - __ldcg(&tb[(int64_t)r * SW + row]);
+      a.x[(int64_t)r * a.n + a.rlist[f.rl + row]] =
+          __ldcg(&ysl[(int64_t)r * f.m + row]) - __ldcg(&tb[(int64_t)r * SW + row]);
     }
   }
 }
 
-template <typename T, typename ACC, bool BWD>
+template <typename T, typename ACC, bool BWD, int RG>
 __global__ void __launch_bounds__(256) k_chain(const DfTask* __restrict__ tasks, int ntask,
                                                LsArgs<T, ACC> a, unsigned* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1273,11 +1319,11 @@ __global__ void __launch_bounds__(256) k_chain(const DfTask* __restrict__ tasks,
     ps.ld = d.ldp;
     ps.writer = d.sub != 0;
     if (!BWD) {
-      if (d.kind == DF_DIAG_FWD) diag_body<T, ACC, false, DR, 1>(t, d.sub, a, dsm, w);
-      else upd_body<T, ACC, 256, 1>(t, a, dsm, w, ps);
+      if (d.kind == DF_DIAG_FWD) diag_body<T, ACC, false, DR, 1, RG>(t, d.sub, a, dsm, w);
+      else upd_body<T, ACC, 256, 1, RG>(t, a, dsm, w, ps);
     } else {
-      if (d.kind == DF_RED_BWD) red_body<T, ACC, 256, 1>(t, a, dsm, w, ps);
-      else if (d.kind == DF_DIAG_BWD) diag_body<T, ACC, true, DR, 1>(t, d.sub, a, dsm, w);
+      if (d.kind == DF_RED_BWD) red_body<T, ACC, 256, 1, RG>(t, a, dsm, w, ps);
+      else if (d.kind == DF_DIAG_BWD) diag_body<T, ACC, true, DR, 1, RG>(t, d.sub, a, dsm, w);
       else fin_body<T, ACC>(t, a, w);
     }
     // every thread's results visible device-wide before the count
@@ -1286,9 +1332,9 @@ __global__ void __launch_bounds__(256) k_chain(const DfTask* __restrict__ tasks,
     if (threadIdx.x == 0) atomicAdd(a.dfc + d.sig, 1);
   }
 }
-template <typename T, typename ACC> constexpr size_t chain_smem() {
-  constexpr size_t d = diag_mv_smem<T, ACC, DF_ROWS>(), u = upd_smem<T, ACC, 256>(),
-                   r = red_smem<T, ACC>();
+template <typename T, typename ACC, int RG> constexpr size_t chain_smem() {
+  constexpr size_t d = diag_mv_smem<T, ACC, DF_ROWS, RG>(), u = upd_smem<T, ACC, 256, RG>(),
+                   r = red_smem<T, ACC, RG>();
   return d > u ? (d > r ? d : r) : (u > r ? u : r);
 }
 
@@ -1334,7 +1380,7 @@ template <> struct Pair<double> {
 
 // Contribution rows (i >= n) of a front, forward: x(rls[i], :) -= L(i, c0:c0+bw)
 // y with y = x(rls[c0:c0+bw], :), the front's solved pivot rows, for the rows
-// [r0, r0 + 2 RECT_FWD_T) of the task (r0 divisible by 4; rows below n in
+// [r0, r0 + rect_fwd_rows) of the task (r0 divisible by 4; rows below n in
 // the first tile are skipped).  Thread t owns the adjacent rows r0 + 2t and
 // r0 + 2t + 1 and reads them from each column as one 8-byte (FP32) or
 // 16-byte (FP64) load straight into registers, the next RF_KU columns in
@@ -1346,23 +1392,28 @@ template <> struct Pair<double> {
 template <typename T, typename ACC, int RQ>
 __global__ void __launch_bounds__(RECT_FWD_T) k_rect_fwd(const LTask* __restrict__ tasks,
                                                          LsArgs<T, ACC> a) {
-  using V = typename Vec4<ACC>::V;
+  using V = typename RhsVec<ACC, RQ>::V;
   using P2 = typename Pair<T>::V;
-  constexpr int VW = Vec4<ACC>::W, KU = RF_KU;
-  static_assert(RQ % VW == 0, "right-hand sides per pass");
+  constexpr int VW = RhsVec<ACC, RQ>::W, KU = RF_KU;
+  // threads: row pair (NP of them) x column group (NK)
+  constexpr int NP = rect_fwd_rows(sizeof(T)) / 2, NK = RECT_FWD_T / NP;
   extern __shared__ __align__(16) unsigned char dsm[];
   int* rc = reinterpret_cast<int*>(dsm);        // [TW] pivot rows of the block
   ACC* yb = reinterpret_cast<ACC*>(rc + TW);   // [kpad][RQ]
   const LTask t = tasks[blockIdx.x];
   const FrontDesc f = a.fr[t.f];
   const int* rl = a.rlist + f.rl;
-  const int tid = threadIdx.x, bw = t.bw, i0 = t.r0 + 2 * tid;
+  const int tid = threadIdx.x, bw = t.bw, pr = tid % NP, i0 = t.r0 + 2 * pr;
   const bool live0 = i0 >= f.n && i0 < f.m, live1 = i0 + 1 >= f.n && i0 + 1 < f.m;
   const bool any = i0 < f.m;  // rows beyond m: padding of the column, never used
   const int dst0 = live0 ? rl[i0] : 0, dst1 = live1 ? rl[i0 + 1] : 0;
   const P2* Lp = reinterpret_cast<const P2*>(a.arena + f.off + (int64_t)t.c0 * f.ld + (any ? i0 : t.r0));
   const int64_t lds = f.ld / 2;  // column stride in pairs
   const int kpad = (bw + KU - 1) / KU * KU;
+  ACC* red = yb + kpad * RQ;  // [NK - 1][2 NP][RQ + 1], columns of groups 1 ..
+  // this group's columns [ka, ke)
+  const int kspan = (kpad / KU + NK - 1) / NK * KU, kg = tid / NP;
+  const int ka = min(kg * kspan, kpad), ke = min(ka + kspan, bw);
   for (int k = tid; k < bw; k += RECT_FWD_T) rc[k] = rl[t.c0 + k];
   for (int rg = 0; rg < a.nrhs; rg += RQ) {
     const int nr = min(RQ, a.nrhs - rg);
@@ -1374,20 +1425,20 @@ __global__ void __launch_bounds__(RECT_FWD_T) k_rect_fwd(const LTask* __restrict
     }
     P2 ln[KU];
 #pragma unroll
-    for (int u = 0; u < KU; ++u) ln[u] = (any && u < bw) ? Lp[u * lds] : P2{};
+    for (int u = 0; u < KU; ++u) ln[u] = (any && ka + u < ke) ? Lp[(int64_t)(ka + u) * lds] : P2{};
     cp_async_wait_all();
     __syncthreads();
     ACC acc0[RQ], acc1[RQ];
 #pragma unroll
     for (int q = 0; q < RQ; ++q) acc0[q] = acc1[q] = ACC(0);
-    for (int k0 = 0; k0 < bw; k0 += KU) {
+    for (int k0 = ka; k0 < ke; k0 += KU) {
       P2 lc[KU];
 #pragma unroll
       for (int u = 0; u < KU; ++u) lc[u] = ln[u];
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
         const int k = k0 + KU + u;
-        ln[u] = (any && k < bw) ? Lp[(int64_t)k * lds] : P2{};
+        ln[u] = (any && k < ke) ? Lp[(int64_t)k * lds] : P2{};
       }
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
@@ -1405,21 +1456,44 @@ __global__ void __launch_bounds__(RECT_FWD_T) k_rect_fwd(const LTask* __restrict
             acc1[4 * q + 1] += l1 * y4.y;
             acc1[4 * q + 2] += l1 * y4.z;
             acc1[4 * q + 3] += l1 * y4.w;
-          } else {
+          } else if constexpr (VW == 2) {
             acc0[2 * q + 0] += l0 * y4.x;
             acc0[2 * q + 1] += l0 * y4.y;
             acc1[2 * q + 0] += l1 * y4.x;
             acc1[2 * q + 1] += l1 * y4.y;
+          } else {
+            acc0[q] += l0 * y4;
+            acc1[q] += l1 * y4;
           }
         }
       }
     }
+    if constexpr (NK > 1) {
+      if (kg > 0) {
 #pragma unroll
-    for (int q = 0; q < RQ; ++q)
-      if (q < nr) {
-        if (live0) aadd(&a.x[(int64_t)(rg + q) * a.n + dst0], -acc0[q]);
-        if (live1) aadd(&a.x[(int64_t)(rg + q) * a.n + dst1], -acc1[q]);
+        for (int q = 0; q < RQ; ++q) {
+          red[((kg - 1) * 2 * NP + 2 * pr) * (RQ + 1) + q] = acc0[q];
+          red[((kg - 1) * 2 * NP + 2 * pr + 1) * (RQ + 1) + q] = acc1[q];
+        }
       }
+      __syncthreads();
+      if (kg == 0) {
+#pragma unroll
+        for (int g = 0; g < NK - 1; ++g)
+#pragma unroll
+          for (int q = 0; q < RQ; ++q) {
+            acc0[q] += red[(g * 2 * NP + 2 * pr) * (RQ + 1) + q];
+            acc1[q] += red[(g * 2 * NP + 2 * pr + 1) * (RQ + 1) + q];
+          }
+      }
+    }
+    if (kg == 0)
+#pragma unroll
+      for (int q = 0; q < RQ; ++q)
+        if (q < nr) {
+          if (live0) aadd(&a.x[(int64_t)(rg + q) * a.n + dst0], -acc0[q]);
+          if (live1) aadd(&a.x[(int64_t)(rg + q) * a.n + dst1], -acc1[q]);
+        }
   }
 }
 
@@ -1437,16 +1511,17 @@ __global__ void __launch_bounds__(RECT_FWD_T) k_rect_fwd(const LTask* __restrict
 template <typename T, typename ACC, int RQ>
 __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict__ tasks,
                                                          LsArgs<T, ACC> a) {
-  using V = typename Vec4<ACC>::V;
-  constexpr int VW = Vec4<ACC>::W, SR = RB_SR, KC = RECT_BWD_COLS, NT = RECT_BWD_T;
-  constexpr int NP = KC / 2, HR = SR / 2;  // column pairs; rows of a slice per half
+  using V = typename RhsVec<ACC, RQ>::V;
+  constexpr int VW = RhsVec<ACC, RQ>::W, SR = RB_SR, NT = RECT_BWD_T;
+  constexpr int KC = rect_bwd_cols(sizeof(T));
+  constexpr int NP = KC / 2, NH = NT / NP, HR = SR / NH;  // column pairs; row groups, rows each
   constexpr int NST = rb_nst<T>(), LP = rb_lp<T>(), CH = 16 / sizeof(T);
-  static_assert(RQ % VW == 0 && NT == 2 * NP && HR % CH == 0, "thread layout");
+  static_assert(NT == NH * NP && HR % CH == 0, "thread layout");
   extern __shared__ __align__(16) unsigned char dsm[];
   T* Ls = reinterpret_cast<T*>(dsm);                        // [NST][KC][LP]
   ACC* xt = reinterpret_cast<ACC*>(Ls + NST * KC * LP);     // [NST][SR][RQ]
-  ACC* half = xt + NST * SR * RQ;                           // [KC][RQ + 1]
-  int* rr = reinterpret_cast<int*>(half + KC * (RQ + 1));  // [RECT_BWD_ROWS]
+  ACC* part = xt + NST * SR * RQ;                           // [NH - 1][KC][RQ + 1]
+  int* rr = reinterpret_cast<int*>(part + (NH - 1) * KC * (RQ + 1));  // [RECT_BWD_ROWS]
   const LTask t = tasks[blockIdx.x];
   const FrontDesc f = a.fr[t.f];
   const T* Lc = a.arena + f.off + (int64_t)t.c0 * f.ld + t.r0;
@@ -1482,7 +1557,7 @@ __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict
     ACC acc0[RQ], acc1[RQ];
 #pragma unroll
     for (int q = 0; q < RQ; ++q) acc0[q] = acc1[q] = ACC(0);
-    unsigned long long pa0[RQ / 2], pa1[RQ / 2];  // FP32: packed pairs (fma.rn.f32x2)
+    unsigned long long pa0[(RQ + 1) / 2], pa1[(RQ + 1) / 2];  // FP32: packed pairs (fma.rn.f32x2)
 #pragma unroll
     for (int q = 0; q < RQ / 2; ++q) pa0[q] = pa1[q] = 0ull;
     for (int s = 0; s < nst; ++s) {
@@ -1520,6 +1595,9 @@ __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict
               pa1[2 * q] = f2fma(d1, x2.x, pa1[2 * q]);
               pa1[2 * q + 1] = f2fma(d1, x2.y, pa1[2 * q + 1]);
             }
+          } else if constexpr (VW == 1) {
+            acc0[0] += l0[u] * xv[0];
+            acc1[0] += l1[u] * xv[0];
           } else {
 #pragma unroll
             for (int q = 0; q < RQ / VW; ++q) {
@@ -1543,11 +1621,11 @@ __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict
       }
     }
     cp_async_wait<0>();
-    if (h == 1)
+    if (h > 0)
 #pragma unroll
       for (int q = 0; q < RQ; ++q) {
-        half[p * (RQ + 1) + q] = acc0[q];
-        half[(p + NP) * (RQ + 1) + q] = acc1[q];
+        part[((h - 1) * KC + p) * (RQ + 1) + q] = acc0[q];
+        part[((h - 1) * KC + p + NP) * (RQ + 1) + q] = acc1[q];
       }
     __syncthreads();
     if (h == 0) {
@@ -1558,9 +1636,12 @@ __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict
           const int64_t pr = rl[t.c0 + k];
 #pragma unroll
           for (int q = 0; q < RQ; ++q)
-            if (q < nr)
-              aadd(&a.tacc[(int64_t)(rg + q) * a.n + pr],
-                   (c == 0 ? acc0[q] : acc1[q]) + half[k * (RQ + 1) + q]);
+            if (q < nr) {
+              ACC sum = c == 0 ? acc0[q] : acc1[q];
+#pragma unroll
+              for (int g = 0; g < NH - 1; ++g) sum += part[(g * KC + k) * (RQ + 1) + q];
+              aadd(&a.tacc[(int64_t)(rg + q) * a.n + pr], sum);
+            }
         }
       }
     }
@@ -1571,13 +1652,16 @@ inline int nblocks(int64_t count, int bs) { return (int)((count + bs - 1) / bs);
 
 // dynamic shared memory of the contribution-row kernels
 template <typename T, typename ACC, int RQ> constexpr size_t rect_fwd_smem(int kpad) {
-  return sizeof(int) * TW + sizeof(ACC) * (size_t)kpad * RQ;
+  constexpr int NP = rect_fwd_rows(sizeof(T)) / 2, NK = RECT_FWD_T / NP;
+  return sizeof(int) * TW + sizeof(ACC) * ((size_t)kpad * RQ + (NK - 1) * 2 * NP * (RQ + 1));
 }
 template <typename T, typename ACC, int RQ> constexpr size_t rect_bwd_smem() {
-  return sizeof(T) * rb_nst<T>() * RECT_BWD_COLS * rb_lp<T>() +
-         sizeof(ACC) * (rb_nst<T>() * RB_SR * RQ + RECT_BWD_COLS * (RQ + 1)) +
+  constexpr int KC = rect_bwd_cols(sizeof(T)), NH = RECT_BWD_T / (KC / 2);
+  return sizeof(T) * rb_nst<T>() * KC * rb_lp<T>() +
+         sizeof(ACC) * (rb_nst<T>() * RB_SR * RQ + (NH - 1) * KC * (RQ + 1)) +
          sizeof(int) * RECT_BWD_ROWS;
 }
+
 }  // namespace
 
 template <typename T, typename ACC>
@@ -1664,6 +1748,38 @@ void launch_axpy_inplace(double* x, int ldx, const double* d, int n, int nrhs, c
   k_axpy<<<nblocks(c, 256), 256, 0, s>>>(x, ldx, d, n, nrhs);
 }
 
+// block steps (RG right-hand sides per pass) and contribution rows (RQ)
+template <typename T, typename ACC, int RG, int RQ>
+static void launch_products(int kind, const LTask* tasks, int ntask, LsArgs<T, ACC> a, int aux,
+                            cudaStream_t s) {
+  switch (kind) {
+    case LS_FWD_DIAG2:
+      launch_pdl(k_diag_mv<T, ACC, false, RG>, dim3(ntask, SW / DMV_ROWS), 256,
+                 diag_mv_smem<T, ACC, DMV_ROWS, RG>(), s, tasks, a);
+      break;
+    case LS_FWD_UPD2:
+      launch_pdl(k_fwd_upd3<T, ACC, RG>, dim3(ntask), 512, upd_smem<T, ACC, 512, RG>(), s, tasks,
+                 a);
+      break;
+    case LS_RECT_FWD: {
+      // aux: the widest task's columns rounded up to the pipeline slice
+      const int kpad = std::min(std::max(aux, RF_KU), TW);
+      k_rect_fwd<T, ACC, RQ><<<ntask, RECT_FWD_T, rect_fwd_smem<T, ACC, RQ>(kpad), s>>>(tasks, a);
+      break;
+    }
+    case LS_RECT_BWD:
+      k_rect_bwd<T, ACC, RQ><<<ntask, RECT_BWD_T, rect_bwd_smem<T, ACC, RQ>(), s>>>(tasks, a);
+      break;
+    case LS_BWD_RED2:
+      launch_pdl(k_bwd_red3<T, ACC, RG>, dim3(ntask), 512, red_smem<T, ACC, RG>(), s, tasks, a);
+      break;
+    case LS_BWD_DIAG2:
+      launch_pdl(k_diag_mv<T, ACC, true, RG>, dim3(ntask, SW / DMV_ROWS), 256,
+                 diag_mv_smem<T, ACC, DMV_ROWS, RG>(), s, tasks, a);
+      break;
+  }
+}
+
 template <typename T, typename ACC>
 void launch_lsolve(int kind, const LTask* tasks, int ntask, LsArgs<T, ACC> a, int aux,
                    cudaStream_t s) {
@@ -1676,51 +1792,44 @@ void launch_lsolve(int kind, const LTask* tasks, int ntask, LsArgs<T, ACC> a, in
       break;
     case LS_SCATTER_FWD:
     case LS_SCATTER_BWD:
-      k_lscatter<T, ACC><<<ntask, 256, 0, s>>>(tasks, a, kind == LS_SCATTER_FWD);
+      k_lscatter<T, ACC><<<ntask, 256, 0, s>>>(tasks, a);
       break;
-    case LS_FWD_DIAG2:
-      launch_pdl(k_diag_mv<T, ACC, false>, dim3(ntask, SW / DMV_ROWS), 256, diag_mv_smem<T, ACC>(), s,
-                 tasks, a);
-      break;
-    case LS_FWD_UPD2:
-      launch_pdl(k_fwd_upd3<T, ACC>, dim3(ntask), 512, upd_smem<T, ACC, 512>(), s, tasks, a);
-      break;
-    case LS_RECT_FWD: {
-      // aux: the widest task's columns rounded up to the pipeline slice
-      const int kpad = std::min(std::max(aux, RF_KU), TW);
-      if (a.nrhs <= 4)
-        k_rect_fwd<T, ACC, 4><<<ntask, RECT_FWD_T, rect_fwd_smem<T, ACC, 4>(kpad), s>>>(tasks, a);
-      else
-        k_rect_fwd<T, ACC, RQ_MID<ACC>>
-            <<<ntask, RECT_FWD_T, rect_fwd_smem<T, ACC, RQ_MID<ACC>>(kpad), s>>>(tasks, a);
-      break;
-    }
-    case LS_RECT_BWD:
-      if (a.nrhs <= 4)
-        k_rect_bwd<T, ACC, 4><<<ntask, RECT_BWD_T, rect_bwd_smem<T, ACC, 4>(), s>>>(tasks, a);
-      else
-        k_rect_bwd<T, ACC, RQ_MID<ACC>>
-            <<<ntask, RECT_BWD_T, rect_bwd_smem<T, ACC, RQ_MID<ACC>>(), s>>>(tasks, a);
-      break;
-    case LS_BWD_RED2:
-      launch_pdl(k_bwd_red3<T, ACC>, dim3(ntask), 512, red_smem<T, ACC>(), s, tasks, a);
-      break;
-    case LS_BWD_DIAG2:
-      launch_pdl(k_diag_mv<T, ACC, true>, dim3(ntask, SW / DMV_ROWS), 256, diag_mv_smem<T, ACC>(), s,
-                 tasks, a);
-      break;
+    default:
+      if constexpr (sizeof(ACC) == 8) {
+        switch (rhs_per_pass(a.nrhs, true)) {
+          case 1: return launch_products<T, ACC, 1, 1>(kind, tasks, ntask, a, aux, s);
+          case 2: return launch_products<T, ACC, 2, 2>(kind, tasks, ntask, a, aux, s);
+          case 4: return launch_products<T, ACC, 4, 4>(kind, tasks, ntask, a, aux, s);
+          case 6: return launch_products<T, ACC, 6, 6>(kind, tasks, ntask, a, aux, s);
+          default: return launch_products<T, ACC, 8, 8>(kind, tasks, ntask, a, aux, s);
+        }
+      } else {
+        if (rhs_per_pass(a.nrhs, false) == 4)
+          return launch_products<T, ACC, 4, 4>(kind, tasks, ntask, a, aux, s);
+        return launch_products<T, ACC, 16, 16>(kind, tasks, ntask, a, aux, s);
+      }
   }
 }
 
 // persistent CTAs of a dataflow sweep: resident CTAs per SM x SMs (set once)
-static int g_chain_ctas = 0;
+static int g_chain_ctas[2] = {0, 0};  // resident CTAs, 4 and 16 right-hand sides per pass
 
+template <int RG>
+static void launch_chain_rg(bool bwd, const DfTask* tasks, int ntask, LsArgs<float, float> a,
+                            unsigned* err, cudaStream_t s) {
+  const int grid = std::max(1, std::min(ntask, g_chain_ctas[RG == 16]));
+  constexpr size_t smem = chain_smem<float, float, RG>();
+  if (bwd) k_chain<float, float, true, RG><<<grid, 256, smem, s>>>(tasks, ntask, a, err);
+  else k_chain<float, float, false, RG><<<grid, 256, smem, s>>>(tasks, ntask, a, err);
+}
+
+// Four right-hand sides per pass when that is all: a task's slabs and sums are a
+// quarter of those of 16, and a task is what every block step waits for.
 void launch_chain(bool bwd, const DfTask* tasks, int ntask, LsArgs<float, float> a, unsigned* err,
                   cudaStream_t s) {
   if (ntask <= 0) return;
-  const int grid = std::max(1, std::min(ntask, g_chain_ctas));
-  if (bwd) k_chain<float, float, true><<<grid, 256, chain_smem<float, float>(), s>>>(tasks, ntask, a, err);
-  else k_chain<float, float, false><<<grid, 256, chain_smem<float, float>(), s>>>(tasks, ntask, a, err);
+  if (rhs_per_pass(a.nrhs, false) == 4) launch_chain_rg<4>(bwd, tasks, ntask, a, err, s);
+  else launch_chain_rg<16>(bwd, tasks, ntask, a, err, s);
   SG_CUDA(cudaGetLastError());
 }
 
@@ -1731,42 +1840,60 @@ void launch_inv_diag(const T* arena, const FrontDesc* fr, const LTask* tasks, in
   k_inv_diag<T><<<ntask, 4 * LB, 0, s>>>(arena, fr, tasks, inv, inv_off, unit);
 }
 
-template <typename T, int RQ>
-void set_rect_smem() {
-  SG_CUDA(cudaFuncSetAttribute(k_rect_fwd<T, T, RQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rect_fwd_smem<T, T, RQ>(TW)));
-  SG_CUDA(cudaFuncSetAttribute(k_rect_bwd<T, T, RQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rect_bwd_smem<T, T, RQ>()));
+template <typename T, int RG>
+void set_product_smem() {
+  SG_CUDA(cudaFuncSetAttribute(k_rect_fwd<T, T, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)rect_fwd_smem<T, T, RG>(TW)));
+  SG_CUDA(cudaFuncSetAttribute(k_rect_bwd<T, T, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)rect_bwd_smem<T, T, RG>()));
+  SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, false, RG>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)diag_mv_smem<T, T, DMV_ROWS, RG>()));
+  SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, true, RG>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)diag_mv_smem<T, T, DMV_ROWS, RG>()));
+  SG_CUDA(cudaFuncSetAttribute(k_fwd_upd3<T, T, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)upd_smem<T, T, 512, RG>()));
+  SG_CUDA(cudaFuncSetAttribute(k_bwd_red3<T, T, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)red_smem<T, T, RG>()));
+}
+
+template <int RG>
+void set_chain_attributes() {
+  constexpr int cs = (int)chain_smem<float, float, RG>();
+  auto kf = k_chain<float, float, false, RG>;
+  auto kb = k_chain<float, float, true, RG>;
+  SG_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
+  SG_CUDA(cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
+  int dev = 0, nsm = 0, per0 = 0, per1 = 0;
+  SG_CUDA(cudaGetDevice(&dev));
+  SG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per0, kf, 256, cs));
+  SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, kb, 256, cs));
+  g_chain_ctas[RG == 16] = std::max(1, nsm * std::max(1, std::min(per0, per1)));
 }
 
 template <typename T>
 void prepare_solve_kernels() {
   SG_CUDA(cudaFuncSetAttribute(k_inv_block<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)inv_block_smem<T>()));
-  SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_mv_smem<T, T>()));
-  SG_CUDA(cudaFuncSetAttribute(k_diag_mv<T, T, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_mv_smem<T, T>()));
   SG_CUDA(cudaFuncSetAttribute(k_tri<T, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)TRI_SMEM));
   SG_CUDA(cudaFuncSetAttribute(k_tri<T, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)TRI_SMEM));
-  set_rect_smem<T, 4>();
-  set_rect_smem<T, RQ_MID<T>>();
-  SG_CUDA(cudaFuncSetAttribute(k_fwd_upd3<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)upd_smem<T, T, 512>()));
-  SG_CUDA(cudaFuncSetAttribute(k_bwd_red3<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)red_smem<T, T>()));
+  if constexpr (sizeof(T) == 8) {
+    set_product_smem<T, 1>();
+    set_product_smem<T, 2>();
+    set_product_smem<T, 4>();
+    set_product_smem<T, 6>();
+    set_product_smem<T, 8>();
+  } else {
+    set_product_smem<T, 4>();
+    set_product_smem<T, 16>();
+  }
   if constexpr (std::is_same<T, float>::value) {
-    const int cs = (int)chain_smem<T, T>();
-    SG_CUDA(cudaFuncSetAttribute(k_chain<T, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
-    SG_CUDA(cudaFuncSetAttribute(k_chain<T, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
-    int dev = 0, nsm = 0, per0 = 0, per1 = 0;
-    SG_CUDA(cudaGetDevice(&dev));
-    SG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per0, k_chain<T, T, false>, 256, cs));
-    SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, k_chain<T, T, true>, 256, cs));
-    g_chain_ctas = std::max(1, nsm * std::max(1, std::min(per0, per1)));
+    set_chain_attributes<4>();
+    set_chain_attributes<16>();
   }
 }
 

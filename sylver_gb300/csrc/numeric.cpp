@@ -1132,8 +1132,8 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
     // kernels skip the first tile's rows below n)
     auto rect = [&](std::vector<SOp>& ops, bool fwd) {
       int64_t a = (int64_t)htasks.size();
-      const int cw = fwd ? RECT_FWD_COLS : RECT_BWD_COLS;
-      const int rh = fwd ? 2 * RECT_FWD_T : RECT_BWD_ROWS;
+      const int cw = fwd ? RECT_FWD_COLS : rect_bwd_cols(elem);
+      const int rh = fwd ? rect_fwd_rows(elem) : RECT_BWD_ROWS;
       int wmax = 0;
       for (int f = 0; f < v.nfront; ++f) {
         const FrontDesc& d = hfr[L.f0 + f];
@@ -1270,7 +1270,7 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
         rows(v.bwd, LS_GATHER_BWD);
         // backward: u_b = X_b^T x_b for every block; then from the last
         // block: z_j = u_j - t_j and t_b += P_jb^T z_j (the block before
-        // first: the chain; its tasks store z_j); z_0 = u_0 - t_0
+        // first: the chain; its tasks store z_j in x); z_0 = u_0 - t_0
         a = (int64_t)hdf.size();
         for (int f = v.nsmall; f < v.nfront; ++f)
           for (int b = 0; b < nbk[f]; ++b)
@@ -1298,13 +1298,11 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
           step(v.fwd, LS_FWD_DIAG2, b, true);
           step(v.fwd, LS_FWD_UPD2, b, false);
         }
-        rows(v.fwd, LS_SCATTER_FWD);
         rows(v.bwd, LS_GATHER_BWD);
         for (int b = maxb2 - 1; b >= 0; --b) {
           step(v.bwd, LS_BWD_RED2, b, false);
           step(v.bwd, LS_BWD_DIAG2, b, true);
         }
-        rows(v.bwd, LS_SCATTER_BWD);
       }
     }
     rect(v.fwd, true);
@@ -1406,7 +1404,7 @@ void SolvePlan::run(bool fwd, const T* arena, const FrontDesc* dfr, const int* r
                      dataflow ? dfcnt.as<int>() + v.dfc_base : nullptr,
                      dataflow ? dfo.as<int2>() + v.f0 : nullptr,
                      dataflow ? ttoff.as<int64_t>() + v.f0 : nullptr,
-                     dataflow ? static_cast<const T*>(pmat.p) : nullptr, dataflow ? 1 : 0};
+                     dataflow ? static_cast<const T*>(pmat.p) : nullptr};
     const std::vector<SOp>& ops = fwd ? v.fwd : v.bwd;
     for (size_t k = 0; k < ops.size(); ++k) {
       const SOp& op = ops[k];
