@@ -138,6 +138,7 @@ struct UpdTask {
 // most BLK_W columns (a multiple of BLK_B by schedule choice).
 constexpr int BLK_B = 64;
 constexpr int BLK_W = 256;
+constexpr int BLK_FEW_CTAS = 608;  // four CTAs of the fused panel kernel per SM
 // k per pipeline stage of the tensor-core update (BF16 elements); stacked
 // panel pitches are multiples of it
 constexpr int TC_KCHUNK = 64;
@@ -151,11 +152,13 @@ constexpr int TC_KCHUNK = 64;
 // later update reads the panel.  cbbase >= 0: the front's contribution
 // rows (>= n) are also written, at K columns [c, c + panel width) clipped to
 // n rounded up to 64, to the contribution-block operand planes (pitch
-// cbpitch), stacked row cbbase for front row n.
+// cbpitch), stacked row cbbase for front row n.  Panels of 64 columns take one
+// kernel for the diagonal block and rows [r0, r1); there xi >= 0 is the block's
+// place in the level's store, base still belongs to row pend.
 struct BlkTask {
   int64_t off;
   int ld, m, c, bw, pend, r0, xi, base;
-  int n, cbbase, cbpitch;
+  int n, cbbase, cbpitch, r1;
 };
 
 #if defined(__CUDACC__)
@@ -242,11 +245,19 @@ void launch_diag_chol(T* arena, const PanelTask* t, int ntask, unsigned* status,
                       cudaStream_t s);
 template <typename T>
 void launch_panel_trsm(T* arena, const PanelTask* t, int ntask, cudaStream_t s);
+// tile: rows and columns of a task, Tiles<T>::TM or (FP64) half of it
 template <typename T>
 void launch_update(T* arena, const T* abuf, const UpdTask* t, int ntask, int tile,
                    cudaStream_t s);
 
-// Launchers (kernels_blocked.cu), FP32 only.  xinv holds one 64 x 64
+// Launchers (kernels_blocked.cu), FP32 only.  64-column panels: the whole panel
+// step, and the level's diagonal blocks from the store into the fronts.
+void launch_blk_fused(float* arena, const BlkTask* t, int ntask, float* dstore, uint16_t* planes,
+                      int64_t pstride, int pitch, uint16_t* cbplanes, int64_t cbpstride,
+                      unsigned* status, cudaStream_t s);
+void launch_diag_store32(float* arena, const BlkTask* t, int ntask, const float* dstore,
+                         cudaStream_t s);
+// Wider panels.  xinv holds one 64 x 64
 // inverse per diagonal-block task of the launch.
 void prepare_blocked_kernels();
 void launch_blk_diag(float* arena, const BlkTask* t, int ntask, float* xinv, unsigned* status,

@@ -41,10 +41,18 @@ constexpr int PROWS = 64;         // rows of one panel-kernel CTA
 constexpr int PTHREADS = 2 * PROWS;
 constexpr int ALD = PROWS + 1;
 
-// start of column j of a packed lower triangle with PW rows
-__device__ __forceinline__ int pcol(int j) { return j * PW - (j * (j - 1)) / 2; }
-// (i, j), i >= j, of the packed lower triangle
-__device__ __forceinline__ int pidx(int i, int j) { return pcol(j) + i - j; }
+// Storage of a panel's diagonal block in shared memory, (i, j) with i >= j:
+// a packed lower triangle with PW rows, or (64-column panels) full columns of
+// 64 + 4 so that 16-byte reads down a column stay aligned.
+struct PackedTri {
+  __device__ __forceinline__ static int col(int j) { return j * PW - (j * (j - 1)) / 2 - j; }
+  __device__ __forceinline__ int operator()(int i, int j) const { return col(j) + i; }
+};
+constexpr int FLD = BLK_B + 4;
+struct DenseTri {
+  __device__ __forceinline__ static int col(int j) { return j * FLD; }
+  __device__ __forceinline__ int operator()(int i, int j) const { return col(j) + i; }
+};
 
 // One warp: Cholesky of the 16 x 16 diagonal sub-block at (q, q) of the
 // packed triangle Lp, in registers (lane i < 16 holds row i; lanes 16..31
@@ -54,12 +62,15 @@ __device__ __forceinline__ int pidx(int i, int j) { return pcol(j) + i - j; }
 // (tt[k*16 + i] = L(i, k), 16-byte aligned) and X = L^-1 to xs and xg (both
 // xs[k*16 + i] = X(i, k)).  A non-positive pivot is replaced by one and
 // reported when its column is below bwreal.
+// xg may be null.
+template <typename Tri>
 __device__ __noinline__ void warp_chol16(float* __restrict__ Lp, int q, int bwreal,
                                          const float* __restrict__ bk, float* __restrict__ tt,
                                          float* __restrict__ xs, float* __restrict__ xg,
                                          unsigned* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const int li = lane & (SB - 1);
+  const Tri pidx;
   float a[SB], rinv[SB];
 #pragma unroll
   for (int k = 0; k < SB; ++k) a[k] = (k <= li) ? Lp[pidx(q + li, q + k)] : 0.f;
@@ -134,36 +145,23 @@ __device__ __noinline__ void warp_chol16(float* __restrict__ Lp, int q, int bwre
     for (int i = 0; i < SB; i += 4) {
       const float4 x4 = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
       *reinterpret_cast<float4*>(&xs[li * SB + i]) = x4;
-      *reinterpret_cast<float4*>(&xg[li * SB + i]) = x4;
+      if (xg != nullptr) *reinterpret_cast<float4*>(&xg[li * SB + i]) = x4;
     }
   }
 }
 
-__global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena,
-                                                       const BlkTask* __restrict__ tasks,
-                                                       float* __restrict__ xinv,
-                                                       unsigned* __restrict__ status) {
-  extern __shared__ __align__(16) float sm[];
-  float* Xs = sm;                      // inverse of the current sub-block, Xs[k*16 + j] = X(j, k)
-  float* Bk = Xs + SB * SB;            // Bk[m*16 + i] = L(c1 + i, q0 + m), the next sub-block's rows
-  float* Tt = Bk + SB * SB;            // dense copy of the factorised sub-block (warp 0)
-  float* Lp = Tt + SB * SB;            // packed lower triangle, PW rows
-  const BlkTask t = tasks[blockIdx.x];
-  float* a = arena + t.off;
-  const int64_t ld = t.ld;
-  const int k0 = t.c, w = t.bw, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wp = (w + SB - 1) / SB * SB;  // rows/cols beyond w: identity
-  float* xg = xinv + (int64_t)t.xi * XSZ;
-  for (int j = warp; j < wp; j += DTHREADS / 32) {
-    float* col = Lp + pcol(j) - j;
-    for (int i = j + lane; i < wp; i += 32) {
-      if (i < w && j < w) cp_async(&col[i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
-      else col[i] = (i == j) ? 1.f : 0.f;
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  if (warp == 0) warp_chol16(Lp, 0, w, nullptr, Tt, Xs, xg, status);
+// Cholesky of the wp x wp diagonal block in Lp (wp a multiple of 16, identity
+// beyond w) by NT threads, NT / 32 a multiple of four.  Inverse of sub-block q at
+// Xs + q XSTEP (XSTEP 0: the current one only) and, unless null, at
+// xg + q * 256; Bk and Tt: 16 x 16 scratch each.
+template <typename Tri, int NT, int XSTEP>
+__device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int wp,
+                                             float* __restrict__ Xs, float* __restrict__ Bk,
+                                             float* __restrict__ Tt, float* __restrict__ xg,
+                                             unsigned* __restrict__ status) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const Tri pidx;
+  if (warp == 0) warp_chol16<Tri>(Lp, 0, w, nullptr, Tt, Xs, xg, status);
   __syncthreads();
   // Per 16-column sub-block q0: (b) all threads solve the rows below it with
   // its inverse; then warp 0 updates the next diagonal sub-block by it and
@@ -178,7 +176,7 @@ __global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena
     // (b) L(r, q0 + j) = sum_k A(r, q0 + k) X(j, k) for rows r >= c1; four
     // lanes per row, lane group g owning columns 4g .. 4g + 3
     const int nb = (wp - c1) * 4;
-    for (int e0 = 0; e0 < nb; e0 += DTHREADS) {
+    for (int e0 = 0; e0 < nb; e0 += NT) {
       const int e = e0 + tid;
       const int r = c1 + (e >> 2), g = e & 3;
       float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -186,7 +184,7 @@ __global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena
 #pragma unroll
         for (int k = 0; k < SB; ++k) {
           const float vk = Lp[pidx(r, q0 + k)];
-          const float4 x4 = *reinterpret_cast<const float4*>(&Xs[k * SB + 4 * g]);
+          const float4 x4 = *reinterpret_cast<const float4*>(&Xs[q0 / SB * XSTEP + k * SB + 4 * g]);
           o[0] = fmaf(vk, x4.x, o[0]);
           o[1] = fmaf(vk, x4.y, o[1]);
           o[2] = fmaf(vk, x4.z, o[2]);
@@ -204,11 +202,12 @@ __global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena
     }
     __syncthreads();
     if (warp == 0) {
-      warp_chol16(Lp, c1, w, Bk, Tt, Xs, xg + (c1 / SB) * SB * SB, status);
+      warp_chol16<Tri>(Lp, c1, w, Bk, Tt, Xs + (c1 / SB) * XSTEP,
+                       xg == nullptr ? xg : xg + (c1 / SB) * SB * SB, status);
     } else if (warp & 3) {
-      // the 12 update warps, numbered 0..11
+      // the update warps, numbered from 0
       const int uw = warp - 1 - (warp >> 2), utid = uw * 32 + lane;
-      constexpr int UTHREADS = DTHREADS / 32 * 3 / 4 * 32;
+      constexpr int UTHREADS = NT / 32 * 3 / 4 * 32;
       // (c1) rows [c1 + 16, wp) x columns [c1, c1 + 16): lane group g of a
       // row updates columns c1 + 4g .. + 3
       const int c2s = c1 + SB;
@@ -245,7 +244,7 @@ __global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena
         const int rl = lane & 7, cl = lane >> 3;
 #pragma unroll 4
         for (int k = 0; k < SB; ++k) {
-          const float* colk = Lp + pcol(q0 + k) - (q0 + k);
+          const float* colk = Lp + Tri::col(q0 + k);
           float rv[2], cv[4];
 #pragma unroll
           for (int u = 0; u < 2; ++u) rv[u] = colk[r0 + rl + 8 * u];
@@ -267,8 +266,35 @@ __global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena
     }
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena,
+                                                       const BlkTask* __restrict__ tasks,
+                                                       float* __restrict__ xinv,
+                                                       unsigned* __restrict__ status) {
+  extern __shared__ __align__(16) float sm[];
+  float* Xs = sm;                      // inverse of the current sub-block, Xs[k*16 + j] = X(j, k)
+  float* Bk = Xs + SB * SB;            // Bk[m*16 + i] = L(c1 + i, q0 + m), the next sub-block's rows
+  float* Tt = Bk + SB * SB;            // dense copy of the factorised sub-block (warp 0)
+  float* Lp = Tt + SB * SB;            // packed lower triangle, PW rows
+  const BlkTask t = tasks[blockIdx.x];
+  float* a = arena + t.off;
+  const int64_t ld = t.ld;
+  const int k0 = t.c, w = t.bw, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wp = (w + SB - 1) / SB * SB;  // rows/cols beyond w: identity
+  float* xg = xinv + (int64_t)t.xi * XSZ;
+  for (int j = warp; j < wp; j += DTHREADS / 32) {
+    float* col = Lp + PackedTri::col(j);
+    for (int i = j + lane; i < wp; i += 32) {
+      if (i < w && j < w) cp_async(&col[i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
+      else col[i] = (i == j) ? 1.f : 0.f;
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  factor_block<PackedTri, DTHREADS, 0>(Lp, w, wp, Xs, Bk, Tt, xg, status);
   for (int j = warp; j < w; j += DTHREADS / 32) {
-    const float* col = Lp + pcol(j) - j;
+    const float* col = Lp + PackedTri::col(j);
     for (int i = j + lane; i < w; i += 32) a[(int64_t)(k0 + j) * ld + k0 + i] = col[i];
   }
 }
@@ -296,47 +322,22 @@ __device__ __forceinline__ void put_split4(const float* __restrict__ Ar, int rr,
 // of rows 16q .. 16q + 15) starts at lw_off(q), 16 values per k.
 __host__ __device__ constexpr int lw_off(int q) { return 128 * q * (q - 1); }
 
-// Rows [r0, r0 + 64) below the panel [k0, k0 + w): L_R L_WW^T = A_R by block
-// forward substitution over 16-column sub-blocks.  Each row is solved by two
-// lanes of one warp (lane & 15 picks the row, lane >> 4 the half of the
-// sub-block's columns); rows never depend on one another, so after the block
-// rows of L_WW and the sub-block inverses are staged once, the sub-steps need
-// no block-wide barrier.
-__global__ void __launch_bounds__(PTHREADS) k_blk_panel(float* __restrict__ arena,
-                                                        const BlkTask* __restrict__ tasks,
-                                                        const float* __restrict__ xinv,
-                                                        uint16_t* __restrict__ planes,
-                                                        int64_t pstride, int pw, int pitch,
-                                                        uint16_t* __restrict__ cbplanes,
-                                                        int64_t cbpstride) {
-  extern __shared__ __align__(16) float sm[];
-  float* Ar = sm;                          // Ar[k*ALD + r] = A(r0 + r, k0 + k), then L
-  float* Lw = Ar + pw * ALD;               // block rows of L_WW (lw_off layout)
-  float* Xs = Lw + lw_off(pw / SB);        // Xs[q*256 + k*16 + j] = X_q(j, k)
-  const BlkTask t = tasks[blockIdx.x];
-  float* a = arena + t.off;
+// Rows r0 .. r0 + nr - 1 of the panel (Ar[k * ALD + row]): L_R L_WW^T = A_R by block
+// forward substitution over 16-column sub-blocks, by PTHREADS threads; the
+// result to the front and, where later updates read it, to the operand planes.
+// Each row is solved by two lanes of one warp (lane & 15 picks the row, lane >> 4
+// the half of the sub-block's columns); rows never depend on one another, so
+// the sub-steps need no block-wide barrier.  lrow(q, k): the 16 values L(16q ..
+// 16q + 15, k) of the diagonal block.
+template <typename LRow>
+__device__ __forceinline__ void solve_rows(const BlkTask& t, float* __restrict__ a, int r0, int nr,
+                                           int nsb, int pw, float* __restrict__ Ar, LRow lrow,
+                                           const float* __restrict__ Xs,
+                                           uint16_t* __restrict__ planes, int64_t pstride,
+                                           int pitch, uint16_t* __restrict__ cbplanes,
+                                           int64_t cbpstride) {
+  const int k0 = t.c, w = t.bw, tid = threadIdx.x;
   const int64_t ld = t.ld;
-  const int k0 = t.c, w = t.bw, r0 = t.r0, tid = threadIdx.x;
-  const int nr = min(PROWS, t.m - r0);
-  const int nsb = (w + SB - 1) / SB, wp = nsb * SB;
-  const float* xg = xinv + (int64_t)t.xi * XSZ;
-  for (int e = tid; e < PROWS * wp; e += PTHREADS) {
-    const int r = e % PROWS, k = e / PROWS;
-    if (r < nr && k < w) cp_async(&Ar[k * ALD + r], &a[(int64_t)(k0 + k) * ld + r0 + r]);
-    else Ar[k * ALD + r] = 0.f;
-  }
-  for (int q = 1; q < nsb; ++q) {
-    float* dst = Lw + lw_off(q);
-    const int q0 = q * SB;
-    for (int e = tid; e < SB * q0; e += PTHREADS) {
-      const int jj = e % SB, k = e / SB;
-      if (q0 + jj < w) cp_async(&dst[e], &a[(int64_t)(k0 + k) * ld + k0 + q0 + jj]);
-      else dst[e] = 0.f;
-    }
-  }
-  for (int e = tid; e < nsb * SB * SB; e += PTHREADS) cp_async(&Xs[e], &xg[e]);
-  cp_async_wait_all();
-  __syncthreads();
   const int lane = tid & 31, h = lane >> 4;
   const int r = (tid >> 5) * 16 + (lane & 15);
   for (int q = 0; q < nsb; ++q) {
@@ -346,12 +347,12 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_panel(float* __restrict__ aren
     float v[8];
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) v[jj] = Ar[(c0 + jj) * ALD + r];
-    const float* lq = Lw + lw_off(q) + 8 * h;
 #pragma unroll 4
     for (int k = 0; k < q0; ++k) {
       const float ar = Ar[k * ALD + r];
-      const float4 la = *reinterpret_cast<const float4*>(lq + k * SB);
-      const float4 lb = *reinterpret_cast<const float4*>(lq + k * SB + 4);
+      const float* lq = lrow(q, k) + 8 * h;
+      const float4 la = *reinterpret_cast<const float4*>(lq);
+      const float4 lb = *reinterpret_cast<const float4*>(lq + 4);
       v[0] = fmaf(-ar, la.x, v[0]);
       v[1] = fmaf(-ar, la.y, v[1]);
       v[2] = fmaf(-ar, la.z, v[2]);
@@ -423,6 +424,128 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_panel(float* __restrict__ aren
   }
 }
 
+// Rows [r0, r0 + 64) below a panel wider than 64 columns, with the diagonal
+// block's factor and sub-block inverses from k_blk_diag.
+__global__ void __launch_bounds__(PTHREADS) k_blk_panel(float* __restrict__ arena,
+                                                        const BlkTask* __restrict__ tasks,
+                                                        const float* __restrict__ xinv,
+                                                        uint16_t* __restrict__ planes,
+                                                        int64_t pstride, int pw, int pitch,
+                                                        uint16_t* __restrict__ cbplanes,
+                                                        int64_t cbpstride) {
+  extern __shared__ __align__(16) float sm[];
+  float* Ar = sm;                          // Ar[k*ALD + r] = A(r0 + r, k0 + k), then L
+  float* Lw = Ar + pw * ALD;               // block rows of L_WW (lw_off layout)
+  float* Xs = Lw + lw_off(pw / SB);        // Xs[q*256 + k*16 + j] = X_q(j, k)
+  const BlkTask t = tasks[blockIdx.x];
+  float* a = arena + t.off;
+  const int64_t ld = t.ld;
+  const int k0 = t.c, w = t.bw, r0 = t.r0, tid = threadIdx.x;
+  const int nr = min(PROWS, t.m - r0);
+  const int nsb = (w + SB - 1) / SB, wp = nsb * SB;
+  const float* xg = xinv + (int64_t)t.xi * XSZ;
+  for (int e = tid; e < PROWS * wp; e += PTHREADS) {
+    const int r = e % PROWS, k = e / PROWS;
+    if (r < nr && k < w) cp_async(&Ar[k * ALD + r], &a[(int64_t)(k0 + k) * ld + r0 + r]);
+    else Ar[k * ALD + r] = 0.f;
+  }
+  for (int q = 1; q < nsb; ++q) {
+    float* dst = Lw + lw_off(q);
+    const int q0 = q * SB;
+    for (int e = tid; e < SB * q0; e += PTHREADS) {
+      const int jj = e % SB, k = e / SB;
+      if (q0 + jj < w) cp_async(&dst[e], &a[(int64_t)(k0 + k) * ld + k0 + q0 + jj]);
+      else dst[e] = 0.f;
+    }
+  }
+  for (int e = tid; e < nsb * SB * SB; e += PTHREADS) cp_async(&Xs[e], &xg[e]);
+  cp_async_wait_all();
+  __syncthreads();
+  solve_rows(t, a, r0, nr, nsb, pw, Ar, [&](int q, int k) { return Lw + lw_off(q) + k * SB; }, Xs,
+             planes, pstride, pitch, cbplanes, cbpstride);
+}
+
+// A 64-column panel in one launch: every CTA factorises the diagonal block for
+// itself, then solves rows [r0, r1) below it, 64 at a time.  A panel is latency
+// (four 16-column pivot chains, then four substitution steps), and a separate
+// launch for the diagonal block added its own start, a round trip of the block
+// and its inverses through memory, and the gap between the two (18 + 18 us a
+// panel at 80^3; see launch_blk_fused).  The CTA with xi >= 0 leaves the factor in
+// dstore; k_diag_store32 moves it into the front when no CTA reads the
+// assembled block any more.
+__global__ void __launch_bounds__(PTHREADS) k_blk_fused(float* __restrict__ arena,
+                                                        const BlkTask* __restrict__ tasks,
+                                                        float* __restrict__ dstore,
+                                                        uint16_t* __restrict__ planes,
+                                                        int64_t pstride, int pitch,
+                                                        uint16_t* __restrict__ cbplanes,
+                                                        int64_t cbpstride,
+                                                        unsigned* __restrict__ status) {
+  constexpr int W = BLK_B;
+  extern __shared__ __align__(16) float sm[];
+  float* D = sm;                        // D[k * FLD + i] = L(k0 + i, k0 + k)
+  float* Ar = D + W * FLD;              // Ar[k * ALD + r] = A(r0 + r, k0 + k), then L
+  float* Xs = Ar + ((W * ALD + 3) & ~3);  // inverses of the four sub-blocks
+  float* Bk = Xs + (W / SB) * SB * SB;
+  float* Tt = Bk + SB * SB;
+  BlkTask t = tasks[blockIdx.x];
+  float* a = arena + t.off;
+  const int64_t ld = t.ld;
+  const int k0 = t.c, w = t.bw, tid = threadIdx.x;
+  const int nsb = (w + SB - 1) / SB, wp = nsb * SB;
+  auto load_rows = [&](int r0, int nr) {
+    for (int e = tid; e < PROWS * wp; e += PTHREADS) {
+      const int r = e % PROWS, k = e / PROWS;
+      if (r < nr && k < w) cp_async(&Ar[k * ALD + r], &a[(int64_t)(k0 + k) * ld + r0 + r]);
+      else Ar[k * ALD + r] = 0.f;
+    }
+    cp_async_commit();
+  };
+  for (int e = tid; e < wp * W; e += PTHREADS) {
+    const int i = e % W, j = e / W;
+    if (i < j || i >= wp) continue;
+    if (i < w) cp_async(&D[j * FLD + i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
+    else D[j * FLD + i] = (i == j) ? 1.f : 0.f;
+  }
+  cp_async_commit();
+  if (t.r0 < t.r1) load_rows(t.r0, min(PROWS, t.r1 - t.r0));
+  cp_async_wait<1>();
+  if (t.r0 >= t.r1) cp_async_wait<0>();
+  __syncthreads();
+  factor_block<DenseTri, PTHREADS, SB * SB>(D, w, wp, Xs, Bk, Tt, nullptr, status);
+  __syncthreads();
+  if (t.xi >= 0) {
+    float* o = dstore + (int64_t)t.xi * (W * W);
+    for (int e = tid; e < w * W; e += PTHREADS) {
+      const int i = e % W, j = e / W;
+      if (i >= j && i < w) o[e] = D[j * FLD + i];
+    }
+  }
+  for (int r0 = t.r0; r0 < t.r1; r0 += PROWS) {
+    const int nr = min(PROWS, t.r1 - r0);
+    if (r0 > t.r0) {
+      __syncthreads();  // the previous rows are no longer read
+      load_rows(r0, nr);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    solve_rows(t, a, r0, nr, nsb, W, Ar,
+               [&](int q, int k) { return D + k * FLD + q * SB; }, Xs, planes, pstride, pitch,
+               cbplanes, cbpstride);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_diag_store32(float* __restrict__ arena,
+                                                      const BlkTask* __restrict__ tasks,
+                                                      const float* __restrict__ dstore) {
+  const BlkTask t = tasks[blockIdx.x];
+  const float* o = dstore + (int64_t)t.xi * (BLK_B * BLK_B);
+  for (int e = threadIdx.x; e < t.bw * BLK_B; e += 256) {
+    const int i = e % BLK_B, j = e / BLK_B;
+    if (i >= j && i < t.bw) arena[t.off + (int64_t)(t.c + j) * t.ld + t.c + i] = o[e];
+  }
+}
+
 constexpr size_t diag_smem() {
   return sizeof(float) * ((size_t)PW * (PW + 1) / 2 + 3 * SB * SB);
 }
@@ -430,9 +553,16 @@ constexpr size_t panel_smem(int pitch) {
   return sizeof(float) * ((size_t)pitch * ALD + lw_off(pitch / SB) + (size_t)pitch * SB);
 }
 
+constexpr size_t fused_smem() {
+  return sizeof(float) * ((size_t)BLK_B * FLD + ((BLK_B * ALD + 3) & ~3) +
+                          (BLK_B / SB + 2) * SB * SB);
+}
+
 }  // namespace
 
 void prepare_blocked_kernels() {
+  SG_CUDA(cudaFuncSetAttribute(k_blk_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)fused_smem()));
   SG_CUDA(cudaFuncSetAttribute(k_blk_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)diag_smem()));
   SG_CUDA(cudaFuncSetAttribute(k_blk_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -451,6 +581,20 @@ void launch_blk_panel(float* arena, const BlkTask* t, int ntask, const float* xi
   if (ntask <= 0) return;
   k_blk_panel<<<ntask, PTHREADS, panel_smem(pw), s>>>(arena, t, xinv, planes, pstride, pw,
                                                        pitch, cbplanes, cbpstride);
+}
+
+void launch_blk_fused(float* arena, const BlkTask* t, int ntask, float* dstore, uint16_t* planes,
+                      int64_t pstride, int pitch, uint16_t* cbplanes, int64_t cbpstride,
+                      unsigned* status, cudaStream_t s) {
+  if (ntask <= 0) return;
+  k_blk_fused<<<ntask, PTHREADS, fused_smem(), s>>>(arena, t, dstore, planes, pstride, pitch,
+                                                    cbplanes, cbpstride, status);
+}
+
+void launch_diag_store32(float* arena, const BlkTask* t, int ntask, const float* dstore,
+                         cudaStream_t s) {
+  if (ntask <= 0) return;
+  k_diag_store32<<<ntask, 256, 0, s>>>(arena, t, dstore);
 }
 
 }  // namespace sylver_gb300

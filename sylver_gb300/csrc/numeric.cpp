@@ -572,6 +572,7 @@ void FKeep::plan_cholesky() {
       const int GW = G * PW;
       int maxn = 0;
       for (int s : large) maxn = std::max(maxn, st.ncol[s]);
+      const int64_t bd0 = (int64_t)blkd.size();
       for (int g0 = 0; g0 < maxn; g0 += GW) {
         // rows [g0 + PW, m) of fronts with fully-summed columns past the
         // group's first panel are stacked (transposed, 3xBF16 split, K
@@ -616,23 +617,35 @@ void FKeep::plan_cholesky() {
         for (int g = 0; g < G; ++g) {
           const int k0 = g0 + g * PW;
           if (k0 >= maxn) break;
-          // the panel's diagonal block (one CTA per front), then the rows
-          // below it (one CTA per 64 rows)
+          // the panel's diagonal block and the rows below it: one launch for
+          // 64-column panels (the blocks go to a store until the level's
+          // end), else one CTA per front, then one per 64 rows
+          const bool fused = PW == BLK_B;
           const int64_t d0 = (int64_t)blkd.size(), p0 = (int64_t)blkp.size();
+          // rows per CTA of the fused kernel: all SMs busy, then as few
+          // repeats of the diagonal block as that allows
+          int64_t below = 0;
+          for (int s : large)
+            if (k0 < st.ncol[s]) below += st.nrow[s] - std::min(k0 + PW, st.ncol[s]);
+          const int rt = fused ? std::max(64, std::min(512, (int)(below / BLK_FEW_CTAS) / 64 * 64))
+                               : 64;
           for (int s : large) {
             const int m = st.nrow[s], n = st.ncol[s];
             if (k0 >= n) continue;
             const int pend = std::min(k0 + PW, n);
-            const int xi = (int)((int64_t)blkd.size() - d0);
+            const int xi = (int)((int64_t)blkd.size() - (fused ? bd0 : d0));
             // stacked row of row pend: only when a later update of this
             // group reads the panel (columns remain past it)
             const int pb = (pend < n) ? base[s] + (pend - q) : -1;
-            blkd.push_back({off[s], ld[s], m, k0, pend - k0, pend, 0, xi, -1, n, -1, 0});
-            for (int r0 = pend; r0 < m; r0 += 64)
-              blkp.push_back({off[s], ld[s], m, k0, pend - k0, pend, r0, xi, pb, n,
-                              r0 + 64 > n ? cbb[s] : -1, cb_pitch});
+            blkd.push_back({off[s], ld[s], m, k0, pend - k0, pend, 0, xi, -1, n, -1, 0, 0});
+            for (int r0 = pend; r0 < m || (fused && r0 == pend); r0 += rt) {
+              const int r1 = std::min(r0 + rt, m);
+              blkp.push_back({off[s], ld[s], m, k0, pend - k0, pend, r0,
+                              fused && r0 > pend ? -1 : xi, pb, n, r1 > n ? cbb[s] : -1, cb_pitch,
+                              r1});
+            }
           }
-          if ((int64_t)blkd.size() > d0) {
+          if (!fused && (int64_t)blkd.size() > d0) {
             ops.push_back({Op::BDIAG, d0, (int64_t)blkd.size(), 0});
             blkinv_count = std::max(blkinv_count, (int64_t)blkd.size() - d0);
           }
@@ -643,6 +656,10 @@ void FKeep::plan_cholesky() {
         }
         // the trailing fully-summed columns, by the whole group
         if (lvl >= 0) tc_update(GW, -1, 0, GW / TC_KCHUNK);
+      }
+      if (PW == BLK_B && (int64_t)blkd.size() > bd0) {
+        ops.push_back({Op::BDIAG, bd0, (int64_t)blkd.size(), 0});
+        dstore_blocks = std::max(dstore_blocks, (int64_t)blkd.size() - bd0);
       }
     } else {
       for (int s : large) maxsteps = std::max(maxsteps, (st.ncol[s] + NB - 1) / NB);
@@ -859,7 +876,8 @@ void FKeep::upload_static(cudaStream_t s) {
     if (splan.dataflow && splan.p_elems > 0) splan.pmat.ensure((size_t)splan.p_elems * sizeof(float));
   }
   tcerr.ensure(sizeof(unsigned));
-  if (dstore_blocks > 0) dstore64.ensure((size_t)dstore_blocks * 32 * 32 * sizeof(double));
+  if (dstore_blocks > 0)
+    dstore.ensure((size_t)dstore_blocks * (precision == 1 ? BLK_B * BLK_B * sizeof(float) : 32 * 32 * sizeof(double)));
   if (blkinv_count > 0) blkinv.ensure((size_t)blkinv_count * BLK_B * BLK_B * sizeof(float));
   if (!tclev.empty() && precision != 1) {
     // one buffer of seven digit planes and row exponents for all launches
@@ -929,14 +947,14 @@ void FKeep::run_ops(cudaStream_t s) {
         if constexpr (std::is_same<T, float>::value)
           launch_diag_chol<T>(A, diagt.as<PanelTask>() + op.a, (int)cnt, stp, s);
         else
-          launch_diag_store64(A, diagst64.as<P64Task>() + op.a, (int)cnt, dstore64.as<double>(),
+          launch_diag_store64(A, diagst64.as<P64Task>() + op.a, (int)cnt, dstore.as<double>(),
                               s);
         break;
       case Op::PANEL:
         if constexpr (std::is_same<T, float>::value)
           launch_panel_trsm<T>(A, panel.as<PanelTask>() + op.a, (int)cnt, s);
         else
-          launch_panel64(A, panel64.as<P64Task>() + op.a, (int)cnt, op.rows, dstore64.as<double>(),
+          launch_panel64(A, panel64.as<P64Task>() + op.a, (int)cnt, op.rows, dstore.as<double>(),
                          tcplanes.as<uint16_t>(), plane_stride,
                          op.aux >= 0 ? tclev[op.aux].pitch : 0, ozexp.as<int>(), stp, s);
         break;
@@ -957,13 +975,21 @@ void FKeep::run_ops(cudaStream_t s) {
         break;
       case Op::BDIAG:
         if constexpr (std::is_same<T, float>::value)
-          launch_blk_diag(A, blkdiag.as<BlkTask>() + op.a, (int)cnt, blkinv.as<float>(), stp, s);
+          if (blk_pw == BLK_B)
+            launch_diag_store32(A, blkdiag.as<BlkTask>() + op.a, (int)cnt, dstore.as<float>(), s);
+          else
+            launch_blk_diag(A, blkdiag.as<BlkTask>() + op.a, (int)cnt, blkinv.as<float>(), stp, s);
         break;
       case Op::BPANEL:
         if constexpr (std::is_same<T, float>::value)
-          launch_blk_panel(A, blkpanel.as<BlkTask>() + op.a, (int)cnt, blkinv.as<float>(),
-                           tcplanes.as<uint16_t>(), plane_stride, blk_pw, op.aux,
-                           cbplanes.as<uint16_t>(), cb_stride, s);
+          if (blk_pw == BLK_B)
+            launch_blk_fused(A, blkpanel.as<BlkTask>() + op.a, (int)cnt, dstore.as<float>(),
+                             tcplanes.as<uint16_t>(), plane_stride, op.aux,
+                             cbplanes.as<uint16_t>(), cb_stride, stp, s);
+          else
+            launch_blk_panel(A, blkpanel.as<BlkTask>() + op.a, (int)cnt, blkinv.as<float>(),
+                             tcplanes.as<uint16_t>(), plane_stride, blk_pw, op.aux,
+                             cbplanes.as<uint16_t>(), cb_stride, s);
         break;
       case Op::TCUPD:
         if constexpr (std::is_same<T, float>::value)
@@ -1266,7 +1292,6 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
           }
         }
         v.fwd.push_back({LS_CHAIN_FWD, a, (int64_t)hdf.size()});
-        rows(v.fwd, LS_SCATTER_FWD);
         rows(v.bwd, LS_GATHER_BWD);
         // backward: u_b = X_b^T x_b for every block; then from the last
         // block: z_j = u_j - t_j and t_b += P_jb^T z_j (the block before
@@ -1292,17 +1317,18 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
             hdf.push_back({DF_FIN_BWD, f, 0, bw_of(f, 0), r0, 0, nred_ctr(f, 0), 1,
                            nred_of(f, 0), zdone(f, 0), NSUB, ready(f, 0), 0, 0, 0});
         v.bwd.push_back({LS_CHAIN_BWD, a, (int64_t)hdf.size()});
-        rows(v.bwd, LS_SCATTER_BWD);
       } else {
         for (int b = 0; b < maxb2; ++b) {
           step(v.fwd, LS_FWD_DIAG2, b, true);
           step(v.fwd, LS_FWD_UPD2, b, false);
         }
+        rows(v.fwd, LS_SCATTER_FWD);
         rows(v.bwd, LS_GATHER_BWD);
         for (int b = maxb2 - 1; b >= 0; --b) {
           step(v.bwd, LS_BWD_RED2, b, false);
           step(v.bwd, LS_BWD_DIAG2, b, true);
         }
+        rows(v.bwd, LS_SCATTER_BWD);
       }
     }
     rect(v.fwd, true);

@@ -226,9 +226,10 @@ struct FKeep {
   std::vector<TcLevel> tclev;
   std::vector<CUtensorMap> tmaps;   // three per tensor-core launch (one per BF16 plane)
   DevMem tcsplit, tctask, tcplanes, tcerr;
-  // FP64: digit splits and row scale exponents; panel and diagonal-store
-  // tasks, and the factorised diagonal blocks of a level's panels
-  DevMem ozsplit, ozexp, panel64, diagst64, dstore64;
+  // FP64: digit splits and row scale exponents; panel and diagonal-store tasks
+  DevMem ozsplit, ozexp, panel64, diagst64;
+  // the factorised diagonal blocks of a level's panels, until its end
+  DevMem dstore;
   int64_t dstore_blocks = 0;
   int64_t plane_stride = 0;        // elements between the BF16 planes
   DevMem cbplanes;                 // contribution-block operands written by the panel kernel
