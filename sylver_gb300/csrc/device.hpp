@@ -346,15 +346,18 @@ constexpr int LSOLVE_TW = 256;   // columns of the L tiles of the update and red
 constexpr int LSOLVE_UPD_ROWS = 32;  // rows per forward-update CTA
 constexpr int LSOLVE_RED_ROWS = 64;  // rows per backward-reduction CTA
 // Contribution-row tasks: LS_RECT_FWD takes rect_fwd_rows x RECT_FWD_COLS of L,
-// LS_RECT_BWD RECT_BWD_ROWS x rect_bwd_cols.  FP64 tasks have a quarter of the
-// rows (columns): one SM's FP64 pipe takes 38 us for 256 x 128 entries times 4
-// right-hand sides, and a level may have fewer tasks than SMs.  The side that is
+// LS_RECT_BWD RECT_BWD_ROWS x rect_bwd_cols.  FP64 tasks and those of calls with
+// few right-hand sides (at most 4) are short: one SM's FP64 pipe takes 38 us for
+// 256 x 128 entries times 4 right-hand sides, and with few columns a task is the
+// latency of its columns one after another (64^3, FP32, one right-hand side: 24
+// us a level in 256-row tasks, 16 us in 64-row ones; with 16 right-hand sides
+// the long ones win, 0.69 against 0.92 ms a sweep at 80^3).  The side that is
 // summed over stays long, so that each row (column) takes as few additions.
 constexpr int RECT_FWD_T = 128, RECT_BWD_T = 128;  // threads
 constexpr int RECT_FWD_COLS = 128;
 constexpr int RECT_BWD_ROWS = 256;
-constexpr int rect_fwd_rows(size_t elem) { return elem == 8 ? 64 : 256; }
-constexpr int rect_bwd_cols(size_t elem) { return elem == 8 ? 32 : 128; }
+constexpr int rect_fwd_rows(size_t elem, bool few) { return elem == 8 || few ? 64 : 256; }
+constexpr int rect_bwd_cols(size_t elem, bool few) { return elem == 8 ? 32 : few ? 64 : 128; }
 // Large fronts are swept block by block over their fully-summed rows only.
 // The contribution rows (>= n) of every front of a level are one separate
 // launch per direction: forward after the pivot rows are solved (x(cb) -=

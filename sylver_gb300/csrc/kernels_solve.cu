@@ -392,15 +392,18 @@ __global__ void k_scale_vals(double* __restrict__ val, const int* __restrict__ r
   val[k] = (scale[r] * val[k]) * scale[col[k]];
 }
 
+// res = b - A x (FP64), one row per thread, RR right-hand sides per pass; the
+// row's entries are taken four at a time so that 4 RR loads of x are in flight.
+// RR is the fewest that need no more passes: the multiply-adds of columns the
+// call does not have cost as much as real ones (the FP64 pipe bounds this
+// kernel: 64^3 27-point with one right-hand side, 268 us with 16 per pass).
+template <int RR>
 __global__ void __launch_bounds__(128) k_residual(const int64_t* __restrict__ rowptr,
                                                   const int* __restrict__ col,
                                                   const double* __restrict__ a, int n,
                                                   const double* __restrict__ x, int ldx,
                                                   const double* __restrict__ b, int ldb,
                                                   double* __restrict__ res, int nrhs) {
-  // one row per thread, up to 16 right-hand sides per pass; the row's
-  // entries are taken four at a time so that 64 loads of x are in flight
-  constexpr int RR = 16;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t p0 = rowptr[i], p1 = rowptr[i + 1];
@@ -421,7 +424,8 @@ __global__ void __launch_bounds__(128) k_residual(const int64_t* __restrict__ ro
       for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int q = 0; q < RR; ++q)
-          if (r0 + q < nrhs) acc[q] = fma(v[u], x[(int64_t)(r0 + q) * ldx + j[u]], acc[q]);
+          if (RR == 1 || r0 + q < nrhs)
+            acc[q] = fma(v[u], x[(int64_t)(r0 + q) * ldx + j[u]], acc[q]);
     }
 #pragma unroll
     for (int q = 0; q < RR; ++q)
@@ -443,18 +447,24 @@ __global__ void __launch_bounds__(256) k_maxnorms(const double* __restrict__ res
   // range, reduced in the block before one atomic per value (a few hundred
   // blocks per right-hand side; per-warp atomics on the same three words were
   // the bottleneck)
-  __shared__ double red[3][8];
+  __shared__ unsigned long long red[3][8];
   const int r = blockIdx.y;
-  double mr = 0.0, mx = 0.0, mb = 0.0;
+  // magnitudes as integers, which order alike (NaN counts as nothing, as with
+  // fmax): comparisons in FP64 would run on its pipe
+  unsigned long long mr = 0, mx = 0, mb = 0;
+  auto take = [](unsigned long long& m, double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+    if (u > m && u <= 0x7ff0000000000000ull) m = u;
+  };
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    mr = fmax(mr, fabs(res[(int64_t)r * n + i]));
-    mx = fmax(mx, fabs(x[(int64_t)r * ldx + i]));
-    mb = fmax(mb, fabs(b[(int64_t)r * ldb + i]));
+    take(mr, res[(int64_t)r * n + i]);
+    take(mx, x[(int64_t)r * ldx + i]);
+    take(mb, b[(int64_t)r * ldb + i]);
   }
   for (int o = 16; o > 0; o >>= 1) {
-    mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    mb = fmax(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, o));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) {
@@ -464,9 +474,9 @@ __global__ void __launch_bounds__(256) k_maxnorms(const double* __restrict__ res
   }
   __syncthreads();
   if (threadIdx.x < 3) {
-    double m = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[threadIdx.x][w]);
-    atomic_max_nonneg(&norms[3 * r + threadIdx.x], m);
+    unsigned long long m = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = max(m, red[threadIdx.x][w]);
+    atomicMax(reinterpret_cast<unsigned long long*>(&norms[3 * r + threadIdx.x]), m);
   }
 }
 
@@ -1396,7 +1406,7 @@ __global__ void __launch_bounds__(RECT_FWD_T) k_rect_fwd(const LTask* __restrict
   using P2 = typename Pair<T>::V;
   constexpr int VW = RhsVec<ACC, RQ>::W, KU = RF_KU;
   // threads: row pair (NP of them) x column group (NK)
-  constexpr int NP = rect_fwd_rows(sizeof(T)) / 2, NK = RECT_FWD_T / NP;
+  constexpr int NP = rect_fwd_rows(sizeof(T), RQ <= 4) / 2, NK = RECT_FWD_T / NP;
   extern __shared__ __align__(16) unsigned char dsm[];
   int* rc = reinterpret_cast<int*>(dsm);        // [TW] pivot rows of the block
   ACC* yb = reinterpret_cast<ACC*>(rc + TW);   // [kpad][RQ]
@@ -1513,7 +1523,7 @@ __global__ void __launch_bounds__(RECT_BWD_T) k_rect_bwd(const LTask* __restrict
                                                          LsArgs<T, ACC> a) {
   using V = typename RhsVec<ACC, RQ>::V;
   constexpr int VW = RhsVec<ACC, RQ>::W, SR = RB_SR, NT = RECT_BWD_T;
-  constexpr int KC = rect_bwd_cols(sizeof(T));
+  constexpr int KC = rect_bwd_cols(sizeof(T), RQ <= 4);
   constexpr int NP = KC / 2, NH = NT / NP, HR = SR / NH;  // column pairs; row groups, rows each
   constexpr int NST = rb_nst<T>(), LP = rb_lp<T>(), CH = 16 / sizeof(T);
   static_assert(NT == NH * NP && HR % CH == 0, "thread layout");
@@ -1652,11 +1662,11 @@ inline int nblocks(int64_t count, int bs) { return (int)((count + bs - 1) / bs);
 
 // dynamic shared memory of the contribution-row kernels
 template <typename T, typename ACC, int RQ> constexpr size_t rect_fwd_smem(int kpad) {
-  constexpr int NP = rect_fwd_rows(sizeof(T)) / 2, NK = RECT_FWD_T / NP;
+  constexpr int NP = rect_fwd_rows(sizeof(T), RQ <= 4) / 2, NK = RECT_FWD_T / NP;
   return sizeof(int) * TW + sizeof(ACC) * ((size_t)kpad * RQ + (NK - 1) * 2 * NP * (RQ + 1));
 }
 template <typename T, typename ACC, int RQ> constexpr size_t rect_bwd_smem() {
-  constexpr int KC = rect_bwd_cols(sizeof(T)), NH = RECT_BWD_T / (KC / 2);
+  constexpr int KC = rect_bwd_cols(sizeof(T), RQ <= 4), NH = RECT_BWD_T / (KC / 2);
   return sizeof(T) * rb_nst<T>() * KC * rb_lp<T>() +
          sizeof(ACC) * (rb_nst<T>() * RB_SR * RQ + (NH - 1) * KC * (RQ + 1)) +
          sizeof(int) * RECT_BWD_ROWS;
@@ -1714,7 +1724,10 @@ void launch_residual(const int64_t* rowptr, const int* col, const double* aval, 
                      const double* x, int ldx, const double* b, int ldb, double* r, int nrhs,
                      cudaStream_t s) {
   if (n == 0) return;
-  k_residual<<<nblocks(n, 128), 128, 0, s>>>(rowptr, col, aval, n, x, ldx, b, ldb, r, nrhs);
+  const int np = (nrhs + 15) / 16, need = (nrhs + np - 1) / np;
+  auto kern = need <= 1 ? k_residual<1> : need <= 2 ? k_residual<2> : need <= 4 ? k_residual<4>
+              : need <= 8 ? k_residual<8> : k_residual<16>;
+  kern<<<nblocks(n, 128), 128, 0, s>>>(rowptr, col, aval, n, x, ldx, b, ldb, r, nrhs);
 }
 
 void launch_maxnorms(const double* res, const double* x, int ldx, const double* b, int ldb,

@@ -1157,22 +1157,33 @@ void SolvePlan::build_tasks(const std::vector<FrontDesc>& hfr, const std::vector
     // (tiles start on a row divisible by 4, for 16-byte copies of L; the
     // kernels skip the first tile's rows below n)
     auto rect = [&](std::vector<SOp>& ops, bool fwd) {
-      int64_t a = (int64_t)htasks.size();
-      const int cw = fwd ? RECT_FWD_COLS : rect_bwd_cols(elem);
-      const int rh = fwd ? rect_fwd_rows(elem) : RECT_BWD_ROWS;
       int wmax = 0;
-      for (int f = 0; f < v.nfront; ++f) {
-        const FrontDesc& d = hfr[L.f0 + f];
-        if (d.m <= d.n) continue;
-        for (int c0 = 0; c0 < d.n; c0 += cw) {
-          const int bw = std::min(cw, d.n - c0);
-          wmax = std::max(wmax, bw);
-          for (int r0 = d.n & ~3; r0 < d.m; r0 += rh) htasks.push_back({f, c0, bw, r0, 0, 0});
+      auto tasks_of = [&](bool few) {
+        const int cw = fwd ? RECT_FWD_COLS : rect_bwd_cols(elem, few);
+        const int rh = fwd ? rect_fwd_rows(elem, few) : RECT_BWD_ROWS;
+        for (int f = 0; f < v.nfront; ++f) {
+          const FrontDesc& d = hfr[L.f0 + f];
+          if (d.m <= d.n) continue;
+          for (int c0 = 0; c0 < d.n; c0 += cw) {
+            const int bw = std::min(cw, d.n - c0);
+            wmax = std::max(wmax, bw);
+            for (int r0 = d.n & ~3; r0 < d.m; r0 += rh) htasks.push_back({f, c0, bw, r0, 0, 0});
+          }
         }
+      };
+      SOp op{fwd ? LS_RECT_FWD : LS_RECT_BWD, (int64_t)htasks.size(), 0};
+      tasks_of(true);
+      op.b = (int64_t)htasks.size();
+      if (op.b == op.a) return;
+      op.a_many = op.a;
+      op.b_many = op.b;
+      if (elem == 4) {
+        op.a_many = op.b;
+        tasks_of(false);
+        op.b_many = (int64_t)htasks.size();
       }
-      push(ops, fwd ? LS_RECT_FWD : LS_RECT_BWD, a);
-      if (!ops.empty() && ops.back().kind == (fwd ? LS_RECT_FWD : LS_RECT_BWD))
-        ops.back().aux = round_up(wmax, 16);
+      op.aux = round_up(wmax, 16);
+      ops.push_back(op);
     };
     rect(v.bwd, false);
     if (v.nsmall > 0) {
@@ -1447,7 +1458,9 @@ void SolvePlan::run(bool fwd, const T* arena, const FrontDesc* dfr, const int* r
         if (prof) mark(fwd ? 0 : 1, s);
         continue;
       }
-      launch_lsolve<T, ACC>(op.kind, tasks.as<LTask>() + op.a, (int)(op.b - op.a), a, op.aux, s);
+      const bool many = nrhs > 4 && (op.kind == LS_RECT_FWD || op.kind == LS_RECT_BWD);
+      const int64_t t0 = many ? op.a_many : op.a, t1 = many ? op.b_many : op.b;
+      launch_lsolve<T, ACC>(op.kind, tasks.as<LTask>() + t0, (int)(t1 - t0), a, op.aux, s);
       if (prof) mark(2 + op.kind, s);
     }
   };

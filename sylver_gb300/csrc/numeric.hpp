@@ -140,6 +140,8 @@ struct SolvePlan {
     int kind;      // LsKind
     int64_t a, b;  // task range
     int aux = 0;   // LS_RECT_FWD: widest task's columns, rounded up to 16
+    // LS_RECT_*: FP32 tasks for calls with more than 4 right-hand sides
+    int64_t a_many = 0, b_many = 0;
   };
   struct Lv {
     int f0 = 0, nsmall = 0, nfront = 0;
