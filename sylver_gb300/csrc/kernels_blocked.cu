@@ -26,7 +26,7 @@
 // solves multiply by the explicit inverses of 16 x 16 diagonal sub-blocks
 // (a block forward substitution), which keeps their error at the level of
 // a plain substitution.
-#include "device.hpp"
+#include "pivot.cuh"
 
 namespace sylver_gb300 {
 
@@ -41,18 +41,10 @@ constexpr int PROWS = 64;         // rows of one panel-kernel CTA
 constexpr int PTHREADS = 2 * PROWS;
 constexpr int ALD = PROWS + 1;
 
-// Storage of a panel's diagonal block in shared memory, (i, j) with i >= j:
-// a packed lower triangle with PW rows, or (64-column panels) full columns of
-// 64 + 4 so that 16-byte reads down a column stay aligned.
-struct PackedTri {
-  __device__ __forceinline__ static int col(int j) { return j * PW - (j * (j - 1)) / 2 - j; }
-  __device__ __forceinline__ int operator()(int i, int j) const { return col(j) + i; }
-};
-constexpr int FLD = BLK_B + 4;
-struct DenseTri {
-  __device__ __forceinline__ static int col(int j) { return j * FLD; }
-  __device__ __forceinline__ int operator()(int i, int j) const { return col(j) + i; }
-};
+// start of column j of a packed lower triangle with PW rows
+__device__ __forceinline__ int pcol(int j) { return j * PW - (j * (j - 1)) / 2; }
+// (i, j), i >= j, of the packed lower triangle
+__device__ __forceinline__ int pidx(int i, int j) { return pcol(j) + i - j; }
 
 // One warp: Cholesky of the 16 x 16 diagonal sub-block at (q, q) of the
 // packed triangle Lp, in registers (lane i < 16 holds row i; lanes 16..31
@@ -62,15 +54,12 @@ struct DenseTri {
 // (tt[k*16 + i] = L(i, k), 16-byte aligned) and X = L^-1 to xs and xg (both
 // xs[k*16 + i] = X(i, k)).  A non-positive pivot is replaced by one and
 // reported when its column is below bwreal.
-// xg may be null.
-template <typename Tri>
 __device__ __noinline__ void warp_chol16(float* __restrict__ Lp, int q, int bwreal,
                                          const float* __restrict__ bk, float* __restrict__ tt,
                                          float* __restrict__ xs, float* __restrict__ xg,
                                          unsigned* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const int li = lane & (SB - 1);
-  const Tri pidx;
   float a[SB], rinv[SB];
 #pragma unroll
   for (int k = 0; k < SB; ++k) a[k] = (k <= li) ? Lp[pidx(q + li, q + k)] : 0.f;
@@ -145,23 +134,36 @@ __device__ __noinline__ void warp_chol16(float* __restrict__ Lp, int q, int bwre
     for (int i = 0; i < SB; i += 4) {
       const float4 x4 = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
       *reinterpret_cast<float4*>(&xs[li * SB + i]) = x4;
-      if (xg != nullptr) *reinterpret_cast<float4*>(&xg[li * SB + i]) = x4;
+      *reinterpret_cast<float4*>(&xg[li * SB + i]) = x4;
     }
   }
 }
 
-// Cholesky of the wp x wp diagonal block in Lp (wp a multiple of 16, identity
-// beyond w) by NT threads, NT / 32 a multiple of four.  Inverse of sub-block q at
-// Xs + q XSTEP (XSTEP 0: the current one only) and, unless null, at
-// xg + q * 256; Bk and Tt: 16 x 16 scratch each.
-template <typename Tri, int NT, int XSTEP>
-__device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int wp,
-                                             float* __restrict__ Xs, float* __restrict__ Bk,
-                                             float* __restrict__ Tt, float* __restrict__ xg,
-                                             unsigned* __restrict__ status) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Tri pidx;
-  if (warp == 0) warp_chol16<Tri>(Lp, 0, w, nullptr, Tt, Xs, xg, status);
+__global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena,
+                                                       const BlkTask* __restrict__ tasks,
+                                                       float* __restrict__ xinv,
+                                                       unsigned* __restrict__ status) {
+  extern __shared__ __align__(16) float sm[];
+  float* Xs = sm;                      // inverse of the current sub-block, Xs[k*16 + j] = X(j, k)
+  float* Bk = Xs + SB * SB;            // Bk[m*16 + i] = L(c1 + i, q0 + m), the next sub-block's rows
+  float* Tt = Bk + SB * SB;            // dense copy of the factorised sub-block (warp 0)
+  float* Lp = Tt + SB * SB;            // packed lower triangle, PW rows
+  const BlkTask t = tasks[blockIdx.x];
+  float* a = arena + t.off;
+  const int64_t ld = t.ld;
+  const int k0 = t.c, w = t.bw, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wp = (w + SB - 1) / SB * SB;  // rows/cols beyond w: identity
+  float* xg = xinv + (int64_t)t.xi * XSZ;
+  for (int j = warp; j < wp; j += DTHREADS / 32) {
+    float* col = Lp + pcol(j) - j;
+    for (int i = j + lane; i < wp; i += 32) {
+      if (i < w && j < w) cp_async(&col[i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
+      else col[i] = (i == j) ? 1.f : 0.f;
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  if (warp == 0) warp_chol16(Lp, 0, w, nullptr, Tt, Xs, xg, status);
   __syncthreads();
   // Per 16-column sub-block q0: (b) all threads solve the rows below it with
   // its inverse; then warp 0 updates the next diagonal sub-block by it and
@@ -176,7 +178,7 @@ __device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int 
     // (b) L(r, q0 + j) = sum_k A(r, q0 + k) X(j, k) for rows r >= c1; four
     // lanes per row, lane group g owning columns 4g .. 4g + 3
     const int nb = (wp - c1) * 4;
-    for (int e0 = 0; e0 < nb; e0 += NT) {
+    for (int e0 = 0; e0 < nb; e0 += DTHREADS) {
       const int e = e0 + tid;
       const int r = c1 + (e >> 2), g = e & 3;
       float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -184,7 +186,7 @@ __device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int 
 #pragma unroll
         for (int k = 0; k < SB; ++k) {
           const float vk = Lp[pidx(r, q0 + k)];
-          const float4 x4 = *reinterpret_cast<const float4*>(&Xs[q0 / SB * XSTEP + k * SB + 4 * g]);
+          const float4 x4 = *reinterpret_cast<const float4*>(&Xs[k * SB + 4 * g]);
           o[0] = fmaf(vk, x4.x, o[0]);
           o[1] = fmaf(vk, x4.y, o[1]);
           o[2] = fmaf(vk, x4.z, o[2]);
@@ -202,12 +204,11 @@ __device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int 
     }
     __syncthreads();
     if (warp == 0) {
-      warp_chol16<Tri>(Lp, c1, w, Bk, Tt, Xs + (c1 / SB) * XSTEP,
-                       xg == nullptr ? xg : xg + (c1 / SB) * SB * SB, status);
+      warp_chol16(Lp, c1, w, Bk, Tt, Xs, xg + (c1 / SB) * SB * SB, status);
     } else if (warp & 3) {
-      // the update warps, numbered from 0
+      // the 12 update warps, numbered 0..11
       const int uw = warp - 1 - (warp >> 2), utid = uw * 32 + lane;
-      constexpr int UTHREADS = NT / 32 * 3 / 4 * 32;
+      constexpr int UTHREADS = DTHREADS / 32 * 3 / 4 * 32;
       // (c1) rows [c1 + 16, wp) x columns [c1, c1 + 16): lane group g of a
       // row updates columns c1 + 4g .. + 3
       const int c2s = c1 + SB;
@@ -244,7 +245,7 @@ __device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int 
         const int rl = lane & 7, cl = lane >> 3;
 #pragma unroll 4
         for (int k = 0; k < SB; ++k) {
-          const float* colk = Lp + Tri::col(q0 + k);
+          const float* colk = Lp + pcol(q0 + k) - (q0 + k);
           float rv[2], cv[4];
 #pragma unroll
           for (int u = 0; u < 2; ++u) rv[u] = colk[r0 + rl + 8 * u];
@@ -266,35 +267,8 @@ __device__ __forceinline__ void factor_block(float* __restrict__ Lp, int w, int 
     }
     __syncthreads();
   }
-}
-
-__global__ void __launch_bounds__(DTHREADS) k_blk_diag(float* __restrict__ arena,
-                                                       const BlkTask* __restrict__ tasks,
-                                                       float* __restrict__ xinv,
-                                                       unsigned* __restrict__ status) {
-  extern __shared__ __align__(16) float sm[];
-  float* Xs = sm;                      // inverse of the current sub-block, Xs[k*16 + j] = X(j, k)
-  float* Bk = Xs + SB * SB;            // Bk[m*16 + i] = L(c1 + i, q0 + m), the next sub-block's rows
-  float* Tt = Bk + SB * SB;            // dense copy of the factorised sub-block (warp 0)
-  float* Lp = Tt + SB * SB;            // packed lower triangle, PW rows
-  const BlkTask t = tasks[blockIdx.x];
-  float* a = arena + t.off;
-  const int64_t ld = t.ld;
-  const int k0 = t.c, w = t.bw, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wp = (w + SB - 1) / SB * SB;  // rows/cols beyond w: identity
-  float* xg = xinv + (int64_t)t.xi * XSZ;
-  for (int j = warp; j < wp; j += DTHREADS / 32) {
-    float* col = Lp + PackedTri::col(j);
-    for (int i = j + lane; i < wp; i += 32) {
-      if (i < w && j < w) cp_async(&col[i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
-      else col[i] = (i == j) ? 1.f : 0.f;
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  factor_block<PackedTri, DTHREADS, 0>(Lp, w, wp, Xs, Bk, Tt, xg, status);
   for (int j = warp; j < w; j += DTHREADS / 32) {
-    const float* col = Lp + PackedTri::col(j);
+    const float* col = Lp + pcol(j) - j;
     for (int i = j + lane; i < w; i += 32) a[(int64_t)(k0 + j) * ld + k0 + i] = col[i];
   }
 }
@@ -465,6 +439,123 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_panel(float* __restrict__ aren
              planes, pstride, pitch, cbplanes, cbpstride);
 }
 
+constexpr int FLD = BLK_B + 4;  // column stride of the fused kernel's block: 16-byte aligned
+
+// Cholesky of the 64 x 64 block D[k * FLD + i] = A(i, k) (identity beyond w) by
+// PTHREADS threads, in blocks of eight columns: warp 0 factorises a block with
+// two rows per lane in registers (its pivots reach the other lanes by shuffles,
+// no barrier), then 4 x 4 register tiles apply it to the triangle behind it.
+// Afterwards each warp inverts one 16 x 16 sub-block into Xs[q * 256 + k * 16 + i]
+// = X_q(i, k).  rinv: 64 floats of scratch.
+__device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __restrict__ Xs,
+                                         float* __restrict__ rinv,
+                                         unsigned* __restrict__ status) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int CB = 8, W = BLK_B;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll 1
+  for (int b = 0; b < W; b += CB) {
+    if (b >= w) {  // identity columns: only their reciprocals are missing
+      if (tid < CB) rinv[b + tid] = 1.f;
+      continue;
+    }
+    if (warp == 0) {
+      const int i0 = b + lane, i1 = i0 + 32;
+      float c[CB], e[CB];
+#pragma unroll
+      for (int u = 0; u < CB; ++u) {
+        c[u] = (lane >= u && i0 < W) ? D[(b + u) * FLD + i0] : 0.f;
+        e[u] = i1 < W ? D[(b + u) * FLD + i1] : 0.f;
+      }
+      bool bad = false;
+#pragma unroll
+      for (int k = 0; k < CB; ++k) {
+        float d = __shfl_sync(FULL, c[k], k);
+        if (!(d > 0.f)) {
+          bad = true;
+          d = 1.f;
+        }
+        const float r = pivot_rsqrt(d);
+        const float l = lane > k ? c[k] * r : 0.f;
+        e[k] *= r;
+#pragma unroll
+        for (int u = k + 1; u < CB; ++u) {
+          const float lu = __shfl_sync(FULL, l, u);
+          c[u] = fmaf(-l, lu, c[u]);
+          e[u] = fmaf(-e[k], lu, e[u]);
+        }
+        c[k] = lane == k ? d * r : l;
+        if (lane == k) rinv[b + k] = r;
+      }
+      if (bad && lane == 0) atomicOr(status, ST_NOT_POSDEF);
+#pragma unroll
+      for (int u = 0; u < CB; ++u) {
+        if (lane >= u && i0 < W) D[(b + u) * FLD + i0] = c[u];
+        if (i1 < W) D[(b + u) * FLD + i1] = e[u];
+      }
+    }
+    __syncthreads();
+    const int o = b + CB, nt = (W - o) / 4;
+#pragma unroll 1
+    for (int x = tid; x < nt * (nt + 1) / 2; x += PTHREADS) {
+      int q = (int)((sqrtf(8.f * (float)x + 1.f) - 1.f) * 0.5f);
+      if (q * (q + 1) / 2 > x) --q;
+      else if ((q + 1) * (q + 2) / 2 <= x) ++q;
+      const int tj = nt - 1 - q, ti = nt - 1 - (x - q * (q + 1) / 2);
+      const int r0 = o + 4 * ti, c0 = o + 4 * tj;
+      float acc[4][4];  // acc[column][row]
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const float4 y = *reinterpret_cast<const float4*>(&D[(c0 + v) * FLD + r0]);
+        acc[v][0] = y.x; acc[v][1] = y.y; acc[v][2] = y.z; acc[v][3] = y.w;
+      }
+#pragma unroll
+      for (int k = 0; k < CB; ++k) {
+        const float4 ra = *reinterpret_cast<const float4*>(&D[(b + k) * FLD + r0]);
+        const float4 cb = *reinterpret_cast<const float4*>(&D[(b + k) * FLD + c0]);
+        const float rv[4] = {ra.x, ra.y, ra.z, ra.w}, cv[4] = {cb.x, cb.y, cb.z, cb.w};
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc[v][u] = fmaf(-rv[u], cv[v], acc[v][u]);
+      }
+      // (entries above the diagonal of a diagonal tile are never used)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        *reinterpret_cast<float4*>(&D[(c0 + v) * FLD + r0]) =
+            make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  // column li of X_q by substitution, x(k) final before it is subtracted
+  const int q0 = warp * SB, li = lane & (SB - 1);
+  if (q0 < w) {
+    float x[SB];
+#pragma unroll
+    for (int i = 0; i < SB; ++i) x[i] = i == li ? 1.f : 0.f;
+#pragma unroll
+    for (int k = 0; k < SB; ++k) {
+      x[k] *= rinv[q0 + k];
+#pragma unroll
+      for (int i4 = (k + 1) & ~3; i4 < SB; i4 += 4) {
+        const float4 l4 = *reinterpret_cast<const float4*>(&D[(q0 + k) * FLD + q0 + i4]);
+        const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i4 + u > k) x[i4 + u] = fmaf(-lv[u], x[k], x[i4 + u]);
+      }
+    }
+    if (lane < SB) {
+#pragma unroll
+      for (int i = 0; i < SB; i += 4)
+        *reinterpret_cast<float4*>(&Xs[warp * SB * SB + li * SB + i]) =
+            make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+    }
+  }
+  __syncthreads();
+}
+
 // A 64-column panel in one launch: every CTA factorises the diagonal block for
 // itself, then solves rows [r0, r1) below it, 64 at a time.  A panel is latency
 // (four 16-column pivot chains, then four substitution steps), and a separate
@@ -486,9 +577,8 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_fused(float* __restrict__ aren
   float* D = sm;                        // D[k * FLD + i] = L(k0 + i, k0 + k)
   float* Ar = D + W * FLD;              // Ar[k * ALD + r] = A(r0 + r, k0 + k), then L
   float* Xs = Ar + ((W * ALD + 3) & ~3);  // inverses of the four sub-blocks
-  float* Bk = Xs + (W / SB) * SB * SB;
-  float* Tt = Bk + SB * SB;
-  BlkTask t = tasks[blockIdx.x];
+  float* rinv = Xs + (W / SB) * SB * SB;
+  const BlkTask t = tasks[blockIdx.x];
   float* a = arena + t.off;
   const int64_t ld = t.ld;
   const int k0 = t.c, w = t.bw, tid = threadIdx.x;
@@ -501,10 +591,9 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_fused(float* __restrict__ aren
     }
     cp_async_commit();
   };
-  for (int e = tid; e < wp * W; e += PTHREADS) {
+  for (int e = tid; e < W * W; e += PTHREADS) {
     const int i = e % W, j = e / W;
-    if (i < j || i >= wp) continue;
-    if (i < w) cp_async(&D[j * FLD + i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
+    if (i >= j && i < w) cp_async(&D[j * FLD + i], &a[(int64_t)(k0 + j) * ld + k0 + i]);
     else D[j * FLD + i] = (i == j) ? 1.f : 0.f;
   }
   cp_async_commit();
@@ -512,8 +601,7 @@ __global__ void __launch_bounds__(PTHREADS) k_blk_fused(float* __restrict__ aren
   cp_async_wait<1>();
   if (t.r0 >= t.r1) cp_async_wait<0>();
   __syncthreads();
-  factor_block<DenseTri, PTHREADS, SB * SB>(D, w, wp, Xs, Bk, Tt, nullptr, status);
-  __syncthreads();
+  factor64(D, w, Xs, rinv, status);
   if (t.xi >= 0) {
     float* o = dstore + (int64_t)t.xi * (W * W);
     for (int e = tid; e < w * W; e += PTHREADS) {
@@ -555,7 +643,7 @@ constexpr size_t panel_smem(int pitch) {
 
 constexpr size_t fused_smem() {
   return sizeof(float) * ((size_t)BLK_B * FLD + ((BLK_B * ALD + 3) & ~3) +
-                          (BLK_B / SB + 2) * SB * SB);
+                          (BLK_B / SB) * SB * SB + BLK_B);
 }
 
 }  // namespace
