@@ -37,9 +37,11 @@ constexpr int OZ_A_BYTES = OZ_DIGITS * OZ_A_TILE;
 constexpr int OZ_B_BYTES = OZ_DIGITS * OZ_B_TILE;
 constexpr int OZ_STAGE_BYTES = OZ_A_BYTES + OZ_B_BYTES;  // 84 KiB
 constexpr int OZ_GROUPS = OZ_DIGITS;               // s = 2 .. 8
+constexpr int OZ_HALF = 4;                         // groups 0 .. 3 and 4 .. 6 change hands
 constexpr int OZ_DRAIN = 2;                        // k chunks summed in an accumulator
 constexpr int OZ_EPI_WARP0 = 2;
-constexpr int OZ_EPI_WARPS = 8;
+constexpr int OZ_EPI_WARPS = 16;
+constexpr int OZ_EC = ON / (OZ_EPI_WARPS / 4);       // columns per epilogue warp
 constexpr int OZ_THREADS = 32 * (OZ_EPI_WARP0 + OZ_EPI_WARPS);
 constexpr int OZ_TMEM_COLS = 512;                  // seven accumulators of 64 columns
 
@@ -92,30 +94,49 @@ __device__ __noinline__ double extreme_scale(int e) {
   return __longlong_as_double((long long)(1023 + max(-1000, min(1000, r))) << 52);
 }
 
-// fixed-point sum += G * 2^(62 - (9 s - 2)) for group s = G + 2
+// fixed-point sum += round(v) * 2^(62 - (9 s - 2)) for group s = G + 2.  The
+// hardware conversion runs at 16 per clock and SM; groups 0 and 1 (below 2^20 by
+// the row norms, 64 columns) are rounded by adding 1.5 2^23, groups 5 and 6, whose
+// unit is 2^-61 and less, by adding 1.5 2^26 (to a multiple of eight: 2^-59 of the
+// norms at most).  What the added constants leave in the sum is
+// group_bias() per call of each.
+constexpr float OZ_MAGIC23 = 12582912.f, OZ_MAGIC26 = 100663296.f;
 template <int G>
-__device__ __forceinline__ void add_group(long long& acc, int v) {
+__device__ __forceinline__ void add_group(unsigned long long& acc, float v) {
   constexpr int SH = 46 - 9 * G;  // 46, 37, 28, 19, 10, 1, -8
-  if constexpr (SH >= 32) {
-    const unsigned hi = (unsigned)((unsigned long long)acc >> 32) + ((unsigned)v << (SH - 32));
-    acc = (long long)(((unsigned long long)hi << 32) | (unsigned)acc);
-  } else if constexpr (SH >= 0) {
-    acc += (long long)v * (long long)(1 << SH);
-  } else {
-    acc += (long long)((v + (1 << (-SH - 1))) >> (-SH));
+  if constexpr (G < 2) {
+    const unsigned u = __float_as_uint(v + OZ_MAGIC23);
+    const unsigned hi = (unsigned)(acc >> 32) + (u << (SH - 32));
+    acc = ((unsigned long long)hi << 32) | (unsigned)acc;
+  } else if constexpr (G < 5) {
+    acc += (unsigned long long)((long long)__float2int_rn(v) * (long long)(1 << SH));
+  } else if constexpr (G == 5) {
+    acc += (unsigned long long)__float_as_uint(v + OZ_MAGIC26) * (8u << SH);
+  } else {  // one is 8 units: >> 5 in all
+    acc += (__float_as_uint(v + OZ_MAGIC26) + 16) >> 5;
   }
+}
+// (modulo 2^64, as the sum is until its constants are out)
+__device__ __forceinline__ unsigned long long group_bias() {
+  constexpr unsigned B23 = 0x4b400000u, B26 = 0x4cc00000u;
+  return ((unsigned long long)((B23 << 14) + (B23 << 5)) << 32) + (unsigned long long)B26 * 16 +
+         (B26 >> 5);
 }
 
 // Persistent: CTA b processes tiles b, b + gridDim.x, ...
 //   warp 0 lane 0 : TMA producer (one 3D load of all seven digit tiles per
 //                   operand and 32-wide k chunk),
-//   warp 1 lane 0 : MMA issuer; the seven groups have an accumulator each,
-//                   which sums two k chunks before the epilogue takes it; group
-//                   after group, so that its reads overlap the MMAs of the
-//                   other groups; tiles narrower than 64 columns take narrower
-//                   MMAs,
-//   warps 2..9    : epilogue; each thread keeps the fixed-point sums of one
-//                   row and 32 columns in registers and reads the next group's
+//   warp 1 lane 0 : MMA issuer; the seven groups have neighbouring accumulators of
+//                   64 columns, and the digit tiles of B lie one after another
+//                   in shared memory, so one MMA multiplies a digit of A by up
+//                   to four of B (N = 256) into as many groups; an MMA takes
+//                   about 90 clocks for any N up to 128, and one per digit pair
+//                   made 28 instead of 11 per 16 columns of k.  The
+//                   accumulators sum two k chunks; groups 0 .. 3 and 4 .. 6
+//                   change hands separately, so that the epilogue reads one half
+//                   while the MMAs fill the other,
+//   warps 2..17   : epilogue; each thread keeps the fixed-point sums of one
+//                   row and 16 columns in registers and reads the next group's
 //                   accumulator while it adds the current one.
 // Seven accumulators fill the tensor memory at 64 columns; with 128 columns
 // and four accumulators in turn each k chunk had to be drained by itself, and the
@@ -128,8 +149,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                   unsigned* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[OZ_STAGES], empty[OZ_STAGES], acc_full[OZ_GROUPS],
-      acc_empty[OZ_GROUPS], done;
+  __shared__ uint64_t full[OZ_STAGES], empty[OZ_STAGES], acc_full[2], acc_empty[2], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   volatile int* abortp = &abort_flag;
@@ -137,13 +157,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(tasks + blockIdx.x) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapa) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapb) : "memory");
     for (int s = 0; s < OZ_STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int a = 0; a < OZ_GROUPS; ++a) {
+    for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], OZ_EPI_WARPS);
     }
@@ -193,8 +214,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       bool ok = true;
       for (int ti = blockIdx.x; ti < ntask && ok; ti += gridDim.x) {
         const int nk = tasks[ti].nk;
-        const uint32_t idesc =
-            oz_idesc(min(ON, (tasks[ti].colEnd - tasks[ti].col0 + 15) & ~15));
         for (int kc = 0; kc < nk && ok; ++kc, ++g) {
           const int s = g % OZ_STAGES;
           const bool first = kc % OZ_DRAIN == 0;
@@ -206,25 +225,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t ad = sw64_desc(su32(smem + s * OZ_STAGE_BYTES));
           const uint64_t bd = sw64_desc(su32(smem + s * OZ_STAGE_BYTES + OZ_A_BYTES));
-          for (int gr = 0; gr < OZ_GROUPS; ++gr) {
-            // the epilogue has read this accumulator's previous sum
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            // the epilogue has read this half's previous sums
             if (first && it > 0) {
-              if (!mbar_wait_or_abort(&acc_empty[gr], (it - 1) & 1, err, abortp)) {
+              if (!mbar_wait_or_abort(&acc_empty[half], (it - 1) & 1, err, abortp)) {
                 ok = false;
                 break;
               }
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
-            const uint32_t d = tmem + (uint32_t)(gr * ON);
-            for (int p = 0; p <= gr; ++p) {
+            // digit p of A times digits q0, q0 + 1, ... of B: groups g0 .. gl
+            const int gl = half ? OZ_GROUPS - 1 : OZ_HALF - 1;
+#pragma unroll
+            for (int p = 0; p <= gl; ++p) {
+              const int g0 = max(p, half ? OZ_HALF : 0), q0 = g0 - p;
               const uint64_t ap = ad + (uint64_t)(p * (OZ_A_TILE >> 4));
-              const uint64_t bq = bd + (uint64_t)((gr - p) * (OZ_B_TILE >> 4));
+              const uint64_t bq = bd + (uint64_t)(q0 * (OZ_B_TILE >> 4));
 #pragma unroll
               for (int kk = 0; kk < OZ_KC / 16; ++kk)
-                mma_bf16(d, ap + 2 * kk, bq + 2 * kk, idesc,
-                         (first && p == 0 && kk == 0) ? 0u : 1u);
+                mma_bf16(tmem + (uint32_t)(g0 * ON), ap + 2 * kk, bq + 2 * kk,
+                         oz_idesc((gl - g0 + 1) * ON),
+                         (p > 0 || kk > 0) ? 1u : (first ? 0u : 1u));
             }
-            if (last) mma_commit(&acc_full[gr]);
+            if (last) mma_commit(&acc_full[half]);
           }
           if (last) ++it;
           if (ok) mma_commit(&empty[s]);
@@ -234,35 +258,37 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       mma_commit(&done);
     }
   } else {
-    // TMEM lanes [32q, 32q + 32) are this warp's, and columns [32h, 32h + 32)
-    // of each tile
-    // (of a tile of at most 32 columns: [16h, 16h + 16))
+    // TMEM lanes [32q, 32q + 32) are this warp's, and columns [16h, 16h + 16)
+    // of each tile (of a tile of at most 32 columns: [8h, 8h + 8))
     const int q = warp & 3, h = (warp - OZ_EPI_WARP0) >> 2;
     int it = 0;
     bool ok = true;
     uint32_t ta = 0;  // this warp's columns of accumulator 0
     // wait for group gr's accumulator and start its read into v (warp-uniform:
     // tcgen05.ld is a warp-collective instruction)
-    auto fetch = [&](int gr, uint32_t (&v)[32]) {
+    auto fetch = [&](int gr, uint32_t (&v)[OZ_EC]) {
       int ready = 0;
-      if (lane == 0) ready = mbar_wait_or_abort(&acc_full[gr], it & 1, err, abortp);
+      if (lane == 0)
+        ready = mbar_wait_or_abort(&acc_full[gr >= OZ_HALF], it & 1, err, abortp);
       ready = __shfl_sync(0xffffffffu, ready, 0);
       if (!ready) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      tmem_ld32_async(ta + (uint32_t)(gr * ON), v);
+      tmem_ld16_async(ta + (uint32_t)(gr * ON), v);
       return true;
     };
-    // the read of group gr has landed: hand the accumulator back
-    auto landed = [&](int gr, uint32_t (&v)[32]) {
+    // the read of group gr has landed: hand a half's accumulators back after
+    // its last group
+    auto landed = [&](int gr, uint32_t (&v)[OZ_EC]) {
       tmem_ld_wait(v);
+      if (gr != OZ_HALF - 1 && gr != OZ_GROUPS - 1) return;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[gr]);
+      if (lane == 0) mbar_arrive(&acc_empty[gr >= OZ_HALF]);
     };
     for (int ti = blockIdx.x; ti < ntask && ok; ti += gridDim.x) {
       const TcTask t = tasks[ti];
       const int rt = q * 32 + lane, row = t.row0 + rt;
-      const int hw = t.colEnd - t.col0 <= 32 ? 16 : 32;
+      const int hw = t.colEnd - t.col0 <= ON / 2 ? OZ_EC / 2 : OZ_EC;
       ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * hw);
       const int c0 = t.col0 + h * hw, ce = min(t.colEnd, c0 + hw);
       const bool on = c0 < ce;  // warp-uniform
@@ -270,24 +296,28 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       // row exponent; lane j holds column c0 + j's
       const int ei = has ? sexp[t.a_row + rt] : 0;
       const int ejl = c0 + lane < ce ? sexp[t.b_row + h * hw + lane] : 0;
-      long long acc[32];
+      // (what the rounding constants will have added is taken out beforehand)
+      unsigned long long acc[OZ_EC];
+      const unsigned long long bias = ((t.nk + OZ_DRAIN - 1) / OZ_DRAIN) * group_bias();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = 0;
+      for (int j = 0; j < OZ_EC; ++j) acc[j] = 0ull - bias;
       for (int kc = 0; kc < t.nk; kc += OZ_DRAIN) {
-        uint32_t va[32], vb[32];
-        auto add = [&](auto gc, uint32_t (&v)[32]) {
+        uint32_t va[OZ_EC], vb[OZ_EC];
+        auto add = [&](auto gc, uint32_t (&v)[OZ_EC]) {
           if (on) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              add_group<decltype(gc)::value>(acc[j], __float2int_rn(__uint_as_float(v[j])));
+            for (int j = 0; j < OZ_EC; ++j)
+              add_group<decltype(gc)::value>(acc[j], __uint_as_float(v[j]));
           }
         };
-        auto step = [&](auto gc, uint32_t (&cur)[32], uint32_t (&nxt)[32]) {
+        auto step = [&](auto gc, uint32_t (&cur)[OZ_EC], uint32_t (&nxt)[OZ_EC]) {
           constexpr int G = decltype(gc)::value;
           if (!ok) return;
           landed(G, cur);
+          // (the other half's groups may have to be waited for: add first)
+          if constexpr (G + 1 == OZ_HALF) add(gc, cur);
           if constexpr (G + 1 < OZ_GROUPS) ok = fetch(G + 1, nxt);
-          add(gc, cur);
+          if constexpr (G + 1 != OZ_HALF) add(gc, cur);
         };
         ok = fetch(0, va);
         step(std::integral_constant<int, 0>{}, va, vb);
@@ -307,30 +337,25 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const bool safe = __all_sync(0xffffffffu, abs(ei) <= OZ_EXP_SAFE / 2 &&
                                                     abs(ejl) <= OZ_EXP_SAFE / 2);
       double* cp = arena + t.c_off + row + (int64_t)c0 * t.ldc;
-      double cv[2][8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) cv[0][j] = c0 + j < cend ? cp[(int64_t)j * t.ldc] : 0.0;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
+      for (int b = 0; b < OZ_EC / 8; ++b) {
         if (c0 + 8 * b >= ce) break;  // warp-uniform
-        if (b < 3) {
+        double cv[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            cv[(b + 1) & 1][j] =
-                c0 + 8 * b + 8 + j < cend ? cp[(int64_t)(8 * b + 8 + j) * t.ldc] : 0.0;
-        }
+        for (int j = 0; j < 8; ++j)
+          cv[j] = c0 + 8 * b + j < cend ? cp[(int64_t)(8 * b + j) * t.ldc] : 0.0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int jj = 8 * b + j;
           const int e = ei + __shfl_sync(0xffffffffu, ejl, jj);
           double d;
           if (safe) {
-            d = fixed_to_double(acc[jj], e);
+            d = fixed_to_double((long long)acc[jj], e);
           } else {
-            d = fixed_to_double(acc[jj], max(-OZ_EXP_SAFE, min(OZ_EXP_SAFE, e)));
+            d = fixed_to_double((long long)acc[jj], max(-OZ_EXP_SAFE, min(OZ_EXP_SAFE, e)));
             d *= extreme_scale(e);
           }
-          if (c0 + jj < cend) cp[(int64_t)jj * t.ldc] = cv[b & 1][j] - d;
+          if (c0 + jj < cend) cp[(int64_t)jj * t.ldc] = cv[j] - d;
         }
       }
     }

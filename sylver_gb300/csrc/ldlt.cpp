@@ -36,7 +36,45 @@
 
 namespace sylver_gb300 {
 
+// Pinned host memory for the tables a level uploads, handed out front to back.
+// reset() once every copy out of it has completed; a request beyond the
+// capacity moves to a larger block, the old one is kept until the reset.
+struct PinnedStage {
+  char* p = nullptr;
+  size_t cap = 0, used = 0, want = 0;
+  std::vector<void*> old;
+  PinnedStage() = default;
+  PinnedStage(const PinnedStage&) = delete;
+  PinnedStage& operator=(const PinnedStage&) = delete;
+  ~PinnedStage() {
+    reset();
+    if (p) cudaFreeHost(p);
+  }
+  void reset() {
+    for (void* q : old) cudaFreeHost(q);
+    old.clear();
+    used = want = 0;
+  }
+  void* take(size_t bytes) {
+    bytes = (bytes + 63) / 64 * 64;
+    want += bytes;
+    if (used + bytes > cap) {
+      const size_t nc = std::max(2 * cap, std::max<size_t>(2 * want, 1 << 20));
+      void* np = nullptr;
+      SG_CUDA(cudaMallocHost(&np, nc));
+      if (p) old.push_back(p);
+      p = static_cast<char*>(np);
+      cap = nc;
+      used = 0;
+    }
+    void* q = p + used;
+    used += bytes;
+    return q;
+  }
+};
+
 struct LdltState {
+  PinnedStage stage;  // reset after each level's host synchronisation
   // per front (original index)
   std::vector<int> m, n, nelim, ld, var_off;
   std::vector<int64_t> off, d_off;
@@ -93,11 +131,18 @@ void grow(DevMem& d, size_t bytes, cudaStream_t s) {
   d.bytes = nb;
 }
 
+// Upload through pinned memory: a copy from pageable memory makes the host wait
+// for the work queued before it (on the shifted 7-point 48^3 matrix about 20 of
+// the factorization's 48 ms), so the next level's tables were not prepared while
+// this level's contribution blocks ran.
 template <typename V>
-void put(DevMem& d, const std::vector<V>& v, cudaStream_t s) {
-  d.ensure(std::max<size_t>(1, v.size()) * sizeof(V));
-  if (!v.empty())
-    SG_CUDA(cudaMemcpyAsync(d.p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, s));
+void put(LdltState& L, DevMem& d, const std::vector<V>& v, cudaStream_t s, size_t off = 0) {
+  d.ensure((off + std::max<size_t>(1, v.size())) * sizeof(V));
+  if (v.empty()) return;
+  void* h = L.stage.take(v.size() * sizeof(V));
+  std::memcpy(h, v.data(), v.size() * sizeof(V));
+  SG_CUDA(cudaMemcpyAsync(static_cast<V*>(d.p) + off, h, v.size() * sizeof(V),
+                          cudaMemcpyHostToDevice, s));
 }
 
 }  // namespace
@@ -184,6 +229,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
   L.var_used = L.d_used = 0;
   L.alloc.reset();
   L.pending.clear();
+  if (L.stage.used) SG_CUDA(cudaStreamSynchronize(s));
+  L.stage.reset();
   // fronts kept in place unless their blocks would take more than half of
   // the device memory that way; then the factor columns are copied out to a
   // compact store after each level and whole blocks are given back
@@ -270,9 +317,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     T* A = fk.arena.as<T>();
     int* dvar = L.dvar.as<int>();
     if (!hvar_lvl.empty())
-      SG_CUDA(cudaMemcpyAsync(dvar + L.var_off[F[0]], hvar_lvl.data(),
-                              hvar_lvl.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    put(L.zspans, zsp, s);
+      put(L, L.dvar, hvar_lvl, s, (size_t)L.var_off[F[0]]);
+    put(L, L.zspans, zsp, s);
     launch_zero_spans<T>(A, L.zspans.as<ZeroSpan>(), (int)zsp.size(), s);
     SG_CUDA(cudaMemsetAsync(L.dall.as<double>() + L.d_off[F[0]], 0,
                             (size_t)(L.d_used - L.d_off[F[0]]) * sizeof(double), s));
@@ -293,8 +339,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
           prev = dest;
         }
       }
-      put(L.am_src, asrc, s);
-      put(L.am_dst, adst, s);
+      put(L, L.am_src, asrc, s);
+      put(L, L.am_dst, adst, s);
       launch_init_a<T>(A, fk.val.as<double>(), L.am_src.as<int64_t>(), L.am_dst.as<int64_t>(),
                        (int64_t)asrc.size(), atomic, s);
       launches++;
@@ -343,9 +389,9 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       }
       rank_item0[maxkids] = (int64_t)items.size();
       if (!items.empty()) {
-        put(L.ea_cd, cds, s);
-        put(L.ea_items, items, s);
-        put(L.ea_maps, maps, s);
+        put(L, L.ea_cd, cds, s);
+        put(L, L.ea_items, items, s);
+        put(L, L.ea_maps, maps, s);
         for (int r = 0; r < maxkids; ++r) {
           int cnt = (int)(rank_item0[r + 1] - rank_item0[r]);
           if (cnt <= 0) continue;
@@ -386,7 +432,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     if (L.sc.bytes < (size_t)std::max<int64_t>(scr, 1) * sizeof(T))
       L.sc.ensure((size_t)std::max<int64_t>(scr, 1) * sizeof(T));
     L.mvvar.ensure((size_t)std::max<int64_t>(ivar, 1) * sizeof(int));
-    put(L.fr, fr, s);
+    put(L, L.fr, fr, s);
     // per-step CTA maps: diag, apply, commit, update, move
     std::vector<CtaMap> maps;
     struct StepMaps { int64_t o[5]; int n[5]; };
@@ -416,7 +462,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
         sm[k].n[kind] = (int)((int64_t)maps.size() - sm[k].o[kind]);
       }
     }
-    put(L.cmap, maps, s);
+    put(L, L.cmap, maps, s);
     // per-slot step buffers and state (p/nf ping-pong, p_final)
     L.blk.ensure((size_t)std::max(nslot, 1) * LDLT_BW * (LDLT_BW + 1) * sizeof(double));
     L.bdinv.ensure((size_t)std::max(nslot, 1) * 2 * LDLT_BW * sizeof(double));
@@ -461,7 +507,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     for (int q = 0; q < nslot; ++q)
       if (st.sparent[F[q]] - 1 >= ns) roots.push_back(fr[q]);
     if (!roots.empty()) {
-      put(L.fr2, roots, s);
+      put(L, L.fr2, roots, s);
       launch_ldlt_tpp<T>(A, L.fr2.as<LdltFront>(), (int)roots.size(), stp, kRootU, tpp1, tpp2,
                          s);
       launches++;
@@ -469,18 +515,19 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     launches += 1;
     // ---- the level's one host synchronisation: eliminated counts and the
     // (pivoted) variable lists for the parents' maps
-    std::vector<int> h(3 * nslot);
-    SG_CUDA(cudaMemcpyAsync(h.data(), p_final, nslot * sizeof(int), cudaMemcpyDeviceToHost, s));
-    SG_CUDA(cudaMemcpyAsync(h.data() + nslot, tpp1, 2 * nslot * sizeof(int),
-                            cudaMemcpyDeviceToHost, s));
+    int* h = static_cast<int*>(L.stage.take(3 * nslot * sizeof(int)));
+    int* hv = static_cast<int*>(
+        L.stage.take(std::max<size_t>(hvar_lvl.size(), 1) * sizeof(int)));
+    SG_CUDA(cudaMemcpyAsync(h, p_final, nslot * sizeof(int), cudaMemcpyDeviceToHost, s));
+    SG_CUDA(cudaMemcpyAsync(h + nslot, tpp1, 2 * nslot * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (!hvar_lvl.empty())
-      SG_CUDA(cudaMemcpyAsync(hvar_lvl.data(), dvar + L.var_off[F[0]],
-                              hvar_lvl.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+      SG_CUDA(cudaMemcpyAsync(hv, dvar + L.var_off[F[0]], hvar_lvl.size() * sizeof(int),
+                              cudaMemcpyDeviceToHost, s));
     SG_CUDA(cudaStreamSynchronize(s));
     {
       size_t o = 0;
       for (int s2 : F) {
-        std::copy(hvar_lvl.begin() + o, hvar_lvl.begin() + o + L.m[s2], L.var[s2].begin());
+        std::copy(hv + o, hv + o + L.m[s2], L.var[s2].begin());
         o += L.m[s2];
       }
     }
@@ -498,6 +545,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       }
       fk.num_delay += nn - t2;
     }
+    L.stage.reset();  // every copy out of it, and h and hv, are done with
     // ---- copy-out: the level's factor columns to the compact store (the
     // blocks are given back whole once the parents have assembled them)
     if (L.copyout) {
@@ -511,7 +559,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       }
       if ((size_t)L.fused * sizeof(T) > fk.fstore.bytes)
         grow(fk.fstore, (size_t)L.fused * sizeof(T), s);
-      put(L.cspans, cs, s);
+      put(L, L.cspans, cs, s);
       launch_copy_spans<T>(fk.fstore.as<T>(), fk.arena.as<T>(), L.cspans.as<CopySpan>(),
                            (int)cs.size(), s);
     }
@@ -577,13 +625,13 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       if (!cfr.empty()) {
         if (L.sc2.bytes < (size_t)std::max<int64_t>(cscr, 1) * sizeof(T))
           L.sc2.ensure((size_t)std::max<int64_t>(cscr, 1) * sizeof(T));
-        put(L.fr2, cfr, s);
-        put(L.cmap2, cm, s);
+        put(L, L.fr2, cfr, s);
+        put(L, L.cmap2, cm, s);
         launch_ldlt_calc_ld<T>(A, L.sc2.as<T>(), L.fr2.as<LdltFront>(), L.cmap2.as<CtaMap>(),
                                (int)cm.size(), stp, s);
         launches++;
         if (!ut.empty()) {
-          put(L.up, ut, s);
+          put(L, L.up, ut, s);
           launch_update<T>(A, L.sc2.as<T>(), L.up.as<UpdTask>(), (int)ut.size(), UT, s);
           launches++;
         }
@@ -596,8 +644,8 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
             uint16_t* planes = L.tcplanes.as<uint16_t>();
             std::vector<TcSplit> all(spl);
             all.insert(all.end(), spd.begin(), spd.end());
-            put(L.tcsplit, all, s);
-            put(L.tctask, tct, s);
+            put(L, L.tcsplit, all, s);
+            put(L, L.tctask, tct, s);
             launch_split_t(A, L.tcsplit.as<TcSplit>(), (int)spl.size(), max_rows, planes,
                            pstride, pitch, s);
             launch_split_t(L.sc2.as<float>(), L.tcsplit.as<TcSplit>() + spl.size(),
@@ -680,9 +728,9 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     L.scratch_rows = std::max(L.scratch_rows, acc);
   }
   fk.clear_solve_graphs();
-  put(L.sfr, L.hsfr, s);
-  put(L.sscr, L.hsscr, s);
-  put(L.sdoff, L.hsdoff, s);
+  put(L, L.sfr, L.hsfr, s);
+  put(L, L.sscr, L.hsscr, s);
+  put(L, L.sdoff, L.hsdoff, s);
   // per-step launches unless asked for: on the shifted 7-point 48^3 matrix (4
   // right-hand sides, five corrections) the dataflow sweeps measured slower
   // (refined solve 23.0-24.2 ms against 21.0-22.4 ms)
