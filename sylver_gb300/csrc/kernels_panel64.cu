@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(P64_THREADS)
     k_panel64(double* __restrict__ arena, const P64Task* __restrict__ tasks,
               double* __restrict__ dstore, uint16_t* __restrict__ planes, int64_t pstride,
               int pitch, int* __restrict__ sexp, unsigned* __restrict__ status) {
-  constexpr int CB = 8;               // columns of a diagonal sub-block
+  constexpr int CB = 4;               // columns of a diagonal sub-block
   constexpr int RW = 32 / NG;         // rows per warp
   constexpr int RC = 4 * RW;          // rows per tile of the CTA
   constexpr int NC = PB / NG;         // columns per lane
