@@ -188,8 +188,9 @@ struct ChildDesc {
 };
 struct EaItem {
   int child;  // index into ChildDesc array
-  int col;    // CB column
+  int col;    // CB column (launch_extend_add: the first of up to EA_COLS)
 };
+constexpr int EA_COLS = 8;
 
 // ---------------------------------------------------------------------------
 // Launchers (kernels_factor.cu)

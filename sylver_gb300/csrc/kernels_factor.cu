@@ -155,14 +155,17 @@ __device__ __forceinline__ void ea_column(T* __restrict__ arena, const ChildDesc
   }
 }
 
+// One CTA per item (up to EA_COLS columns of one child), a warp per column.
 template <typename T>
-__global__ void k_extend_add(T* __restrict__ arena, const ChildDesc* __restrict__ cd,
-                             const EaItem* __restrict__ items, const int* __restrict__ maps,
-                             int nitems, bool atomic) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= nitems) return;
-  const EaItem it = items[warp];
-  ea_column<T>(arena, cd[it.child], maps, it.col, threadIdx.x & 31, atomic);
+__global__ void __launch_bounds__(32 * EA_COLS) k_extend_add(T* __restrict__ arena,
+                                                             const ChildDesc* __restrict__ cd,
+                                                             const EaItem* __restrict__ items,
+                                                             const int* __restrict__ maps,
+                                                             bool atomic) {
+  const EaItem it = items[blockIdx.x];
+  const ChildDesc c = cd[it.child];
+  const int j = it.col + (threadIdx.x >> 5);
+  if (j < c.mc) ea_column<T>(arena, c, maps, j, threadIdx.x & 31, atomic);
 }
 
 // One warp per parent column: the CB columns of the front's children that
@@ -539,8 +542,7 @@ template <typename T>
 void launch_extend_add(T* arena, const ChildDesc* cd, const EaItem* items, const int* maps,
                        int nitems, cudaStream_t s, bool atomic) {
   if (nitems <= 0) return;
-  int blocks = (nitems + 7) / 8;
-  k_extend_add<T><<<blocks, 256, 0, s>>>(arena, cd, items, maps, nitems, atomic);
+  k_extend_add<T><<<nitems, 32 * EA_COLS, 0, s>>>(arena, cd, items, maps, atomic);
 }
 
 template <typename T>

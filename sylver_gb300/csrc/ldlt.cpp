@@ -75,6 +75,10 @@ struct PinnedStage {
 
 struct LdltState {
   PinnedStage stage;  // reset after each level's host synchronisation
+  // front row and column of every original entry (order of nlist / 2), and
+  // whether a front has two entries for one place; fixed by the analysis
+  std::vector<int> ent_row, ent_col;
+  std::vector<char> ent_dup;
   // per front (original index)
   std::vector<int> m, n, nelim, ld, var_off;
   std::vector<int64_t> off, d_off;
@@ -131,6 +135,17 @@ void grow(DevMem& d, size_t bytes, cudaStream_t s) {
   d.bytes = nb;
 }
 
+// Pinned room for a table of n entries, and its upload.
+template <typename V>
+V* staged(LdltState& L, size_t n) {
+  return static_cast<V*>(L.stage.take(n * sizeof(V)));
+}
+template <typename V>
+void send(DevMem& d, const V* h, size_t n, cudaStream_t s) {
+  d.ensure(std::max<size_t>(1, n) * sizeof(V));
+  if (n) SG_CUDA(cudaMemcpyAsync(d.p, h, n * sizeof(V), cudaMemcpyHostToDevice, s));
+}
+
 // Upload through pinned memory: a copy from pageable memory makes the host wait
 // for the work queued before it (on the shifted 7-point 48^3 matrix about 20 of
 // the factorization's 48 ms), so the next level's tables were not prepared while
@@ -174,6 +189,20 @@ void plan_ldlt(FKeep& fk) {
   // whole blocks given back (factor columns copied out) for fronts that
   // would not fit that way.
   LdltState& L = *fk.ldlt;
+  L.ent_row.resize(st.nlist.size() / 2);
+  L.ent_col.resize(st.nlist.size() / 2);
+  L.ent_dup.assign(ns, 0);
+  for (int s = 0; s < ns; ++s) {
+    const int64_t nrow = st.nrow[s];
+    int64_t prev = -1;
+    for (int64_t k = st.nptr[s] - 1; k < st.nptr[s + 1] - 1; ++k) {
+      const int64_t dest = st.nlist[2 * k + 1] - 1;
+      L.ent_col[k] = (int)(dest / nrow);
+      L.ent_row[k] = (int)(dest % nrow);
+      if (dest == prev) L.ent_dup[s] = 1;
+      prev = dest;
+    }
+  }
   for (int whole = 0; whole < 2; ++whole) {
     ArenaAlloc sim;
     std::vector<int64_t> soff(ns, 0);
@@ -281,6 +310,11 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     L.pending.clear();
     std::vector<ZeroSpan> zsp;
     std::vector<int> hvar_lvl;
+    {
+      size_t rows = 0;  // delayed columns come on top
+      for (int s2 : F) rows += st.nrow[s2];
+      hvar_lvl.reserve(rows + rows / 8);
+    }
     for (int s2 : F) {
       int sncol = st.ncol[s2], snrow = st.nrow[s2];
       int ndin = 0;
@@ -298,12 +332,13 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
       L.var_off[s2] = (int)L.var_used;
       L.var_used += L.m[s2];
       auto& v = L.var[s2];
-      v.clear();
+      v.resize(L.m[s2]);
       const int* rl = &st.rlist[st.rptr[s2] - 1];
-      for (int i = 0; i < sncol; ++i) v.push_back(rl[i] - 1);
+      int* vp = v.data();
+      for (int i = 0; i < sncol; ++i) *vp++ = rl[i] - 1;
       for (int c : st.children[s2])
-        for (int jj = L.nelim[c]; jj < L.n[c]; ++jj) v.push_back(L.var[c][jj]);
-      for (int i = sncol; i < snrow; ++i) v.push_back(rl[i] - 1);
+        for (int jj = L.nelim[c]; jj < L.n[c]; ++jj) *vp++ = L.var[c][jj];
+      for (int i = sncol; i < snrow; ++i) *vp++ = rl[i] - 1;
       hvar_lvl.insert(hvar_lvl.end(), v.begin(), v.end());
       fk.maxfront = std::max(fk.maxfront, L.m[s2]);
     }
@@ -324,25 +359,26 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
                             (size_t)(L.d_used - L.d_off[F[0]]) * sizeof(double), s));
     // ---- original entries (rows below the own columns shift by ndelay_in)
     {
-      std::vector<int64_t> asrc, adst;
       bool atomic = false;
+      size_t cnt = 0;
+      for (int s2 : F) cnt += st.nptr[s2 + 1] - st.nptr[s2];
+      int64_t* asrc = staged<int64_t>(L, cnt);
+      int64_t* adst = staged<int64_t>(L, cnt);
+      size_t w = 0;
       for (int s2 : F) {
-        int snrow = st.nrow[s2], sncol = st.ncol[s2], ndin = L.n[s2] - sncol;
-        int64_t prev = -1;
-        for (int64_t k = st.nptr[s2] - 1; k < st.nptr[s2 + 1] - 1; ++k) {
-          int64_t src = st.nlist[2 * k] - 1, dest = st.nlist[2 * k + 1] - 1;
-          int64_t c = dest / snrow, r = dest % snrow;
-          if (r >= sncol) r += ndin;
-          asrc.push_back(src);
-          adst.push_back(L.off[s2] + c * L.ld[s2] + r);
-          if (dest == prev) atomic = true;
-          prev = dest;
+        const int sncol = st.ncol[s2], ndin = L.n[s2] - sncol;
+        const int64_t base = L.off[s2], ldf = L.ld[s2];
+        atomic = atomic || L.ent_dup[s2];
+        for (int64_t k = st.nptr[s2] - 1; k < st.nptr[s2 + 1] - 1; ++k, ++w) {
+          const int r = L.ent_row[k];
+          asrc[w] = st.nlist[2 * k] - 1;
+          adst[w] = base + L.ent_col[k] * ldf + (r >= sncol ? r + ndin : r);
         }
       }
-      put(L, L.am_src, asrc, s);
-      put(L, L.am_dst, adst, s);
+      send(L.am_src, asrc, cnt, s);
+      send(L.am_dst, adst, cnt, s);
       launch_init_a<T>(A, fk.val.as<double>(), L.am_src.as<int64_t>(), L.am_dst.as<int64_t>(),
-                       (int64_t)asrc.size(), atomic, s);
+                       (int64_t)cnt, atomic, s);
       launches++;
     }
     // ---- children: delayed columns and contribution blocks, one launch per
@@ -351,53 +387,55 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
     {
       int maxkids = 0;
       for (int p2 : F) maxkids = std::max(maxkids, (int)st.children[p2].size());
-      std::vector<ChildDesc> cds;
-      std::vector<EaItem> items;
-      std::vector<int> maps;
-      std::vector<int64_t> rank_item0(maxkids + 1, 0);
-      std::vector<std::vector<int>> pmaps(F.size());
-      for (size_t k = 0; k < F.size(); ++k) {
-        int p2 = F[k];
-        for (int i = 0; i < L.m[p2]; ++i) pos[L.var[p2][i]] = i;
-        auto& pm = pmaps[k];
-        for (int c : st.children[p2])
-          for (int i = L.nelim[c]; i < L.m[c]; ++i) pm.push_back(pos[L.var[c][i]]);
-      }
-      for (int r = 0; r < maxkids; ++r) {
-        rank_item0[r] = (int64_t)items.size();
-        for (size_t k = 0; k < F.size(); ++k) {
-          int p2 = F[k];
-          const auto& kids = st.children[p2];
-          if (r >= (int)kids.size()) continue;
-          int moff = 0;
-          for (int rr = 0; rr < r; ++rr) moff += L.m[kids[rr]] - L.nelim[kids[rr]];
-          int c = kids[r];
-          int mc = L.m[c] - L.nelim[c];
+      // child descriptors and row maps by rank, front by front; items of up
+      // to EA_COLS columns of one child
+      std::vector<size_t> cd0(maxkids + 1, 0), map0(maxkids + 1, 0), item0(maxkids + 1, 0);
+      for (int p2 : F) {
+        const auto& kids = st.children[p2];
+        for (size_t r = 0; r < kids.size(); ++r) {
+          const int mc = L.m[kids[r]] - L.nelim[kids[r]];
           if (mc <= 0) continue;
-          ChildDesc cd;
-          cd.cb_off = L.off[c] + (int64_t)L.nelim[c] * L.ld[c] + L.nelim[c];
-          cd.p_off = L.off[p2];
-          cd.ld_c = L.ld[c];
-          cd.ld_p = L.ld[p2];
-          cd.mc = mc;
-          cd.map_off = (int)maps.size();
-          maps.insert(maps.end(), pmaps[k].begin() + moff, pmaps[k].begin() + moff + mc);
-          int ci = (int)cds.size();
-          cds.push_back(cd);
-          for (int jj = 0; jj < mc; ++jj) items.push_back({ci, jj});
+          cd0[r + 1] += 1;
+          map0[r + 1] += mc;
+          item0[r + 1] += ceil_div(mc, EA_COLS);
         }
       }
-      rank_item0[maxkids] = (int64_t)items.size();
-      if (!items.empty()) {
-        put(L, L.ea_cd, cds, s);
-        put(L, L.ea_items, items, s);
-        put(L, L.ea_maps, maps, s);
+      for (int r = 0; r < maxkids; ++r) {
+        cd0[r + 1] += cd0[r];
+        map0[r + 1] += map0[r];
+        item0[r + 1] += item0[r];
+      }
+      if (cd0[maxkids] > 0) {
+        ChildDesc* cds = staged<ChildDesc>(L, cd0[maxkids]);
+        EaItem* items = staged<EaItem>(L, item0[maxkids]);
+        int* maps = staged<int>(L, map0[maxkids]);
+        std::vector<size_t> cd(cd0), mp(map0), im(item0);
+        for (int p2 : F) {
+          const auto& kids = st.children[p2];
+          if (kids.empty()) continue;
+          const int* pv = L.var[p2].data();
+          for (int i = 0; i < L.m[p2]; ++i) pos[pv[i]] = i;
+          for (size_t r = 0; r < kids.size(); ++r) {
+            const int c = kids[r], ne = L.nelim[c], mc = L.m[c] - ne;
+            if (mc <= 0) continue;
+            cds[cd[r]] = {L.off[c] + (int64_t)ne * L.ld[c] + ne, L.off[p2], L.ld[c], L.ld[p2], mc,
+                          (int)mp[r]};
+            const int* cv = L.var[c].data() + ne;
+            int* mo = maps + mp[r];
+            for (int i = 0; i < mc; ++i) mo[i] = pos[cv[i]];
+            mp[r] += mc;
+            for (int j = 0; j < mc; j += EA_COLS) items[im[r]++] = {(int)cd[r], j};
+            ++cd[r];
+          }
+        }
+        send(L.ea_cd, cds, cd0[maxkids], s);
+        send(L.ea_items, items, item0[maxkids], s);
+        send(L.ea_maps, maps, map0[maxkids], s);
         for (int r = 0; r < maxkids; ++r) {
-          int cnt = (int)(rank_item0[r + 1] - rank_item0[r]);
+          const int cnt = (int)(item0[r + 1] - item0[r]);
           if (cnt <= 0) continue;
-          launch_extend_add<T>(A, L.ea_cd.as<ChildDesc>(),
-                               L.ea_items.as<EaItem>() + rank_item0[r], L.ea_maps.as<int>(),
-                               cnt, s, /*atomic=*/false);
+          launch_extend_add<T>(A, L.ea_cd.as<ChildDesc>(), L.ea_items.as<EaItem>() + item0[r],
+                               L.ea_maps.as<int>(), cnt, s, /*atomic=*/false);
           launches++;
         }
       }

@@ -486,7 +486,7 @@ void FKeep::plan_cholesky() {
         cds.push_back(cd);
         if ((int)by_rank.size() <= rank) by_rank.resize(rank + 1);
         for (int j = 0; j < mc; ++j) {
-          by_rank[rank].push_back({ci, j});
+          if (j % EA_COLS == 0) by_rank[rank].push_back({ci, j});
           dests.push_back({k, maps[cd.map_off + j], rank, {ci, j}});
           if (j > 0 && maps[cd.map_off + j] <= maps[cd.map_off + j - 1]) ordered = false;
         }
