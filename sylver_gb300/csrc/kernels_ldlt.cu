@@ -518,6 +518,122 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
   if (tid == 0 && fail < nd) atomicMin(&st.npass_raw[q], fail);
 }
 
+// The same for FP64, four lanes per row (128 threads for 32 rows), lane group c
+// holding columns c, c + 4, ...: an FP64 instruction keeps a scheduler's pipe for
+// 65 clocks however many lanes it has, so a row per lane left 3/4 of the SM's
+// pipes idle wherever a launch has fewer rows than the chip has warps.  Every
+// entry keeps its operations and their order.  14^3 saddle point: 30 -> 16 us per
+// launch.
+constexpr int R4 = 32, T4 = 128, NC4 = BW / 4, RW4 = 8;  // rows, threads, columns a lane, rows a warp
+// the row's values in columns k - 1 and k + 1, k = 4 u + c
+__device__ __forceinline__ void neighbours4(const double (&x)[NC4], int u, int rl, int c,
+                                            double& prev, double& next) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const double n0 = __shfl_sync(FULL, x[u], rl + ((c + 1) & 3) * RW4);
+  const double n1 = u + 1 < NC4 ? __shfl_sync(FULL, x[u + 1 < NC4 ? u + 1 : u], rl) : 0.0;
+  const double p0 = __shfl_sync(FULL, x[u], rl + ((c + 3) & 3) * RW4);
+  const double p1 = u > 0 ? __shfl_sync(FULL, x[u > 0 ? u - 1 : 0], rl + 3 * RW4) : 0.0;
+  next = c < 3 ? n0 : n1;
+  prev = c > 0 ? p0 : p1;
+}
+
+__global__ void __launch_bounds__(T4) k_app_apply64(const double* __restrict__ arena,
+                                                    double* __restrict__ scratch,
+                                                    const LdltFront* __restrict__ fr,
+                                                    const CtaMap* __restrict__ cm, LdltStep st) {
+  __shared__ double L[BW][BW + 2];  // zero past the ndiag pivots
+  __shared__ double dv[2 * BW];
+  __shared__ int perm[BW], kind[BW];
+  __shared__ int fail, has2;
+  const CtaMap c = cm[blockIdx.x];
+  const LdltFront F = fr[c.f];
+  const int q = F.fidx, w = block_width(F, st.k), e = extra_rows(F, w);
+  const int p = st.p_cur[q], nd = st.ndiag[q];
+  if (nd == 0) return;
+  const double* A = arena + F.off;
+  const int64_t ld = F.ld, pm = F.m;
+  const int tid = threadIdx.x, lane = tid & 31, rl = lane % RW4, cg = lane / RW4;
+  const double* blk = st.blk + (int64_t)q * BW * LDB;
+  for (int idx = tid; idx < BW * BW; idx += T4) {
+    const int j = idx / BW, k = idx % BW;
+    L[j][k] = (j < nd && k < nd) ? blk[j * LDB + k] : 0.0;
+  }
+  if (tid < 2 * BW) dv[tid] = st.bdinv[q * 2 * BW + tid];
+  if (tid < BW) perm[tid] = st.lperm[q * BW + tid];
+  if (tid == 0) fail = nd;
+  __syncthreads();
+  if (tid < BW) {
+    kind[tid] = pivot_kind(dv, tid, nd);
+    const unsigned two = __ballot_sync(0xffffffffu, kind[tid] == PV_FIRST && tid < nd);
+    if (tid == 0) has2 = two != 0;
+  }
+  __syncthreads();
+  const BelowRows br{p + w, F.n, e, F.m};
+  const int nrow = br.count();
+  const double lim = 1.0 / st.u;
+  double* pan = scratch + F.pan_off;
+  for (int t0 = c.local * R4; t0 < nrow; t0 += c.count * R4) {
+    const int ci = t0 + (tid >> 5) * RW4 + rl;
+    const bool has = ci < nrow;
+    const int r = has ? br.row(ci) : 0;
+    double x[NC4];
+#pragma unroll
+    for (int u = 0; u < NC4; ++u) {
+      const int k = 4 * u + cg;
+      x[u] = has && k < nd ? A[(p + perm[k]) * ld + r] : 0.0;
+    }
+    // x L^T = a  (unit lower L)
+#pragma unroll
+    for (int u0 = 0; u0 < NC4; ++u0) {
+      for (int jj = 0; jj < 4 && 4 * u0 + jj < nd; ++jj) {
+        const double xj = -__shfl_sync(0xffffffffu, x[u0], rl + jj * RW4);
+        const double* lj = &L[4 * u0 + jj][cg];
+        if (cg > jj) x[u0] = fma_(xj, lj[4 * u0], x[u0]);
+#pragma unroll
+        for (int u = u0 + 1; u < NC4; ++u) x[u] = fma_(xj, lj[4 * u], x[u]);
+      }
+    }
+    // times D^-1 (apply_pivot OP_N)
+    double y[NC4];
+#pragma unroll
+    for (int u = 0; u < NC4; ++u) {
+      const int k = 4 * u + cg;
+      double xp = 0.0, xn = 0.0;
+      if (has2) neighbours4(x, u, rl, cg, xp, xn);
+      double v = x[u];
+      if (k < nd) {
+        const int kd = kind[k];
+        if (kd == PV_ONE) {
+          v = mul_(x[u], dv[2 * k]);
+        } else if (kd == PV_FIRST && k + 1 < BW) {
+          v = fma_(dv[2 * k], x[u], mul_(dv[2 * k + 1], xn));
+        } else if (kd == PV_SECOND && k > 0 && kind[k - 1] == PV_FIRST) {
+          v = fma_(dv[2 * k - 1], xp, mul_(dv[2 * k + 1], x[u]));
+        } else if (kd == PV_ZERO) {
+          v = (fabs(x[u]) < st.small) ? 0.0 : dinf() * x[u];
+        }
+      }
+      y[u] = v;
+    }
+    if (has) {
+      int first = nd;
+#pragma unroll
+      for (int u = NC4 - 1; u >= 0; --u) {
+        const int k = 4 * u + cg;
+        if (k < nd && above(y[u], lim)) first = k;
+      }
+      if (first < nd) atomicMin(&fail, first);
+#pragma unroll
+      for (int u = 0; u < NC4; ++u) {
+        const int k = 4 * u + cg;
+        if (k < nd) pan[k * pm + r] = y[u];
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0 && fail < nd) atomicMin(&st.npass_raw[q], fail);
+}
+
 // ---------------------------------------------------------------------------
 // Commit over rows [p, m): passed columns get L (and L*D of the rows from
 // p + npass on, for the trailing update), failed columns get back their
@@ -641,6 +757,127 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
   }
   if (c.local == 0) {
     for (int k = tid; k < 2 * np; k += RT) st.dall[F.d_off + 2 * p + k] = dv[k];
+    if (tid == 0) {
+      const int nf = st.nf_cur[q];
+      st.npass[q] = np;
+      st.p_next[q] = p + np;
+      st.nf_next[q] = nf + (w - np);
+      if (st.k == F.nblk - 1) st.p_final[q] = p + np;
+    }
+  }
+}
+
+// The same for FP64, four lanes per row as in k_app_apply64 (a row's 32 FP64
+// divisions were half of the launch): 22 -> 13 us per launch on the 14^3 saddle
+// point.
+__global__ void __launch_bounds__(T4) k_app_commit64(double* __restrict__ arena,
+                                                     double* __restrict__ scratch,
+                                                     const LdltFront* __restrict__ fr,
+                                                     const CtaMap* __restrict__ cm, LdltStep st) {
+  __shared__ double L[BW][LDB];
+  __shared__ double dv[2 * BW];
+  __shared__ double dca[BW], dcb[BW];  // D of a 2x2 pair's two columns
+  __shared__ int perm[BW], kind[BW];
+  __shared__ int has2;
+  const CtaMap c = cm[blockIdx.x];
+  const LdltFront F = fr[c.f];
+  const int q = F.fidx, w = block_width(F, st.k);
+  const int p = st.p_cur[q], nd = st.ndiag[q];
+  double* A = arena + F.off;
+  const int64_t ld = F.ld, pm = F.m;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rl = lane % RW4, cg = lane / RW4;
+  const double* blk = st.blk + (int64_t)q * BW * LDB;
+  // only the tile of the block's own rows reads L (the rest come from apply)
+  if (c.local == 0)
+    for (int idx = tid; idx < BW * LDB; idx += T4) (&L[0][0])[idx] = blk[idx];
+  if (tid < 2 * BW) dv[tid] = st.bdinv[q * 2 * BW + tid];
+  if (tid < BW) perm[tid] = st.lperm[q * BW + tid];
+  __syncthreads();
+  // the block's permutation on its rows of the eliminated columns [0, p)
+  {
+    constexpr int PU = 4;
+    const int pl = perm[lane];
+    if (__any_sync(0xffffffffu, lane < w && pl != lane))
+      for (int c0 = (c.local * (T4 / 32) + warp) * PU; c0 < p; c0 += c.count * (T4 / 32) * PU) {
+        double v[PU];
+#pragma unroll
+        for (int u = 0; u < PU; ++u)
+          v[u] = (lane < w && c0 + u < p) ? A[(c0 + u) * ld + p + pl] : 0.0;
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < PU; ++u)
+          if (lane < w && c0 + u < p) A[(c0 + u) * ld + p + lane] = v[u];
+      }
+  }
+  // Column::adjust: drop the first half of a 2x2 pivot split by the test
+  int np = min(st.npass_raw[q], nd);
+  if (np > 0 && isfinite(dv[2 * (np - 1)]) && dv[2 * (np - 1) + 1] != 0.0) np--;
+  if (tid < BW) {
+    const int kd = pivot_kind(dv, tid, np);
+    kind[tid] = kd;
+    if (kd == PV_FIRST || (kd == PV_SECOND && tid < np)) {
+      const int k = kd == PV_FIRST ? tid : tid - 1;
+      const double a = dv[2 * k], b = dv[2 * k + 1], cc = dv[2 * k + 3];
+      const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
+      dca[tid] = kd == PV_FIRST ? cc / det : -b / det;
+      dcb[tid] = kd == PV_FIRST ? -b / det : a / det;
+    }
+    const unsigned two = __ballot_sync(0xffffffffu, kd == PV_FIRST || kd == PV_SECOND);
+    if (tid == 0) has2 = two != 0;
+  }
+  __syncthreads();
+  const double* pan = scratch + F.pan_off;
+  double* ldp = scratch + F.ldp_off;
+  for (int t0 = p + c.local * R4; t0 < F.m; t0 += c.count * R4) {
+    const int r = t0 + warp * RW4 + rl;
+    const bool has = r < F.m, in_blk = r < p + w;
+    const int i = r - p;
+    // phase 1: L of the passed columns, the values failed columns keep
+    // (in-block rows all belong to the tile that starts at p, so no other
+    // CTA writes what this one reads)
+    double l[NC4];
+#pragma unroll
+    for (int u = 0; u < NC4; ++u) {
+      const int k = 4 * u + cg;
+      double v = 0.0;
+      if (has && !in_blk) {
+        v = k < np ? pan[k * pm + r] : k < w ? A[(p + perm[k]) * ld + r] : 0.0;
+      } else if (has) {
+        if (k < np) {
+          v = (i > k) ? L[k][i] : (i == k ? 1.0 : 0.0);
+        } else if (k < w && i >= k) {
+          const int ai = perm[i], ak = perm[k];
+          v = A[(p + min(ai, ak)) * ld + p + max(ai, ak)];
+        }
+      }
+      l[u] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NC4; ++u) {
+      const int k = 4 * u + cg;
+      double lp = 0.0, ln = 0.0;
+      if (has2) neighbours4(l, u, rl, cg, lp, ln);
+      if (!has) continue;
+      if (k < w && !(in_blk && i < k)) A[(p + k) * ld + r] = l[u];
+      if (r >= p + np && k < np) {
+        const int kd = kind[k];
+        double v = 0.0;
+        if (kd == PV_ONE) {
+          v = l[u] / dv[2 * k];
+        } else if (kd == PV_FIRST) {
+          if (k + 1 < BW) v = fma_(l[u], dca[k], mul_(ln, dcb[k]));
+        } else if (kd == PV_SECOND) {
+          if (k > 0) v = fma_(lp, dca[k], mul_(l[u], dcb[k]));
+        }
+        ldp[k * pm + r] = v;
+      }
+    }
+    __syncthreads();
+  }
+  if (c.local == 0) {
+    for (int k = tid; k < 2 * np; k += T4) st.dall[F.d_off + 2 * p + k] = dv[k];
     if (tid == 0) {
       const int nf = st.nf_cur[q];
       st.npass[q] = np;
@@ -1010,12 +1247,16 @@ void launch_app_diag(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm
 template <typename T>
 void launch_app_apply(const T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                       LdltStep st, cudaStream_t s) {
-  if (ncta > 0) k_app_apply<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
+  if (ncta <= 0) return;
+  if constexpr (sizeof(T) == 8) k_app_apply64<<<ncta, T4, 0, s>>>(arena, scratch, fr, cm, st);
+  else k_app_apply<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_commit(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                        LdltStep st, cudaStream_t s) {
-  if (ncta > 0) k_app_commit<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
+  if (ncta <= 0) return;
+  if constexpr (sizeof(T) == 8) k_app_commit64<<<ncta, T4, 0, s>>>(arena, scratch, fr, cm, st);
+  else k_app_commit<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_move(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
