@@ -42,6 +42,7 @@
 #include <type_traits>
 
 #include "ldlt_dev.hpp"
+#include "pivot.cuh"
 #include "tile_update.cuh"
 
 namespace sylver_gb300 {
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(DG_T) k_app_diag(T* __restrict__ arena, T* __r
   };
   // 1x1 pivot at position s (label l, its column in col1)
   auto elim1 = [&](int s, int l) {
-    const C di = C(1) / dg[l];
+    const C di = quot(C(1), dg[l]);
     update(s, [&](C x, int i, int j) { return fma_(-col1[i], mul_(col1[j], di), x); });
     if (warp == DG_W - 1) {
       if (lane < R && mp > s) Ls[s][lane] = mul_(col1[lane], di);
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(DG_T) k_app_diag(T* __restrict__ arena, T* __r
   auto elim2 = [&](int s, int l1, int l2) {
     const double a11 = dg[l1], a21 = col1[l2], a22 = dg[l2];
     const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
-    const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+    const double i11 = quot(a22, det), i12 = quot(-a21, det), i22 = quot(a11, det);
     update(s + 1, [&](C x, int i, int j) {
       const double w1 = col1[j], w2 = col2[j];
       const C x1 = (C)fma_(i11, w1, mul_(i12, w2)), x2 = (C)fma_(i12, w1, mul_(i22, w2));
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(DG_T) k_app_diag(T* __restrict__ arena, T* __r
     }
   } else {
     // ---- threshold partial pivoting over the w candidates (ldlt_tpp_factor)
-    const double lim = 1.0 / st.u;
+    const double lim = quot(1.0, st.u);
     while (s < w) {
       int decided = 0, piv = -1, tpiv = -1, lc = -1, lt = -1;
       for (int c = s; c < w && !decided; ++c) {
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(DG_T) k_app_diag(T* __restrict__ arena, T* __r
           const double a11 = dg[lc], a22 = dg[lt], a21 = col1[lt];
           const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
           if (fabs(det) > st.small && isfinite(det)) {
-            const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+            const double i11 = quot(a22, det), i12 = quot(-a21, det), i22 = quot(a11, det);
             if (fma_(fabs(i11), ap2, mul_(fabs(i12), at2)) <= lim &&
                 fma_(fabs(i12), ap2, mul_(fabs(i22), at2)) <= lim) {
               decided = 2; piv = c; tpiv = tm;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
   __syncthreads();
   const BelowRows br{p + w, F.n, e, F.m};
   const int nrow = br.count();
-  const double lim = 1.0 / st.u;
+  const double lim = quot(1.0, st.u);
   T* pan = scratch + F.pan_off;
   for (int t0 = c.local * RT; t0 < nrow; t0 += c.count * RT) {
     const int ci = t0 + tid;
@@ -570,7 +571,7 @@ __global__ void __launch_bounds__(T4) k_app_apply64(const double* __restrict__ a
   __syncthreads();
   const BelowRows br{p + w, F.n, e, F.m};
   const int nrow = br.count();
-  const double lim = 1.0 / st.u;
+  const double lim = quot(1.0, st.u);
   double* pan = scratch + F.pan_off;
   for (int t0 = c.local * R4; t0 < nrow; t0 += c.count * R4) {
     const int ci = t0 + (tid >> 5) * RW4 + rl;
@@ -699,8 +700,8 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
       const int k = kd == PV_FIRST ? tid : tid - 1;
       const double a = dv[2 * k], b = dv[2 * k + 1], cc = dv[2 * k + 3];
       const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
-      dca[tid] = kd == PV_FIRST ? cc / det : -b / det;
-      dcb[tid] = kd == PV_FIRST ? -b / det : a / det;
+      dca[tid] = quot(kd == PV_FIRST ? cc : -b, det);
+      dcb[tid] = quot(kd == PV_FIRST ? -b : a, det);
     }
   }
   __syncthreads();
@@ -820,8 +821,8 @@ __global__ void __launch_bounds__(T4) k_app_commit64(double* __restrict__ arena,
       const int k = kd == PV_FIRST ? tid : tid - 1;
       const double a = dv[2 * k], b = dv[2 * k + 1], cc = dv[2 * k + 3];
       const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
-      dca[tid] = kd == PV_FIRST ? cc / det : -b / det;
-      dcb[tid] = kd == PV_FIRST ? -b / det : a / det;
+      dca[tid] = quot(kd == PV_FIRST ? cc : -b, det);
+      dcb[tid] = quot(kd == PV_FIRST ? -b : a, det);
     }
     const unsigned two = __ballot_sync(0xffffffffu, kd == PV_FIRST || kd == PV_SECOND);
     if (tid == 0) has2 = two != 0;
@@ -1045,7 +1046,7 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
     __syncthreads();
     return fmax(res, 0.0);
   };
-  const double lim = 1.0 / u;
+  const double lim = quot(1.0, u);
   int ne = pstart[F.fidx];
   while (ne < n) {
     int decided = 0, piv = -1, tpiv = -1;
@@ -1062,7 +1063,7 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
         double a11 = sym(c, c), a22 = sym(t, t), a21 = sym(t, c);
         double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
         if (fabs(det) > st.small && isfinite(det)) {
-          double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+          double i11 = quot(a22, det), i12 = quot(-a21, det), i22 = quot(a11, det);
           if (fma_(fabs(i11), ap2, mul_(fabs(i12), at2)) <= lim &&
               fma_(fabs(i12), ap2, mul_(fabs(i22), at2)) <= lim) {
             decided = 2; piv = c; tpiv = t;
@@ -1088,7 +1089,7 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
     } else if (decided == 1) {
       swap_xy(ne, piv);
       const int k = ne;
-      const double di = 1.0 / (double)at(k, k);
+      const double di = quot(1.0, (double)at(k, k));
       const int wdt = n - k - 1;
       for (int e = tid; e < wdt * (m - k - 1); e += nt) {
         int j = k + 1 + e % wdt, rr = k + 1 + e / wdt;
@@ -1110,7 +1111,7 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
       swap_xy(k + 1, (tpiv == k) ? piv : tpiv);
       const double a11 = at(k, k), a21 = at(k + 1, k), a22 = at(k + 1, k + 1);
       const double det = __dsub_rn(mul_(a11, a22), mul_(a21, a21));
-      const double i11 = a22 / det, i12 = -a21 / det, i22 = a11 / det;
+      const double i11 = quot(a22, det), i12 = quot(-a21, det), i22 = quot(a11, det);
       const int wdt = n - k - 2;
       for (int e = tid; wdt > 0 && e < wdt * (m - k - 2); e += nt) {
         int j = k + 2 + e % wdt, rr = k + 2 + e / wdt;
@@ -1146,11 +1147,10 @@ __global__ void __launch_bounds__(256) k_ldlt_tpp(T* __restrict__ arena,
 // ---------------------------------------------------------------------------
 // L*D of contribution rows [n, m) over columns [0, nelim) (F.p = nelim).
 // A slice's CTAs stride over tiles of LDLT_RT rows x CLD columns, one row per
-// thread, CLD_U loads in flight.  (With all nelim columns on the thread of a
-// row the kernel was one latency chain: 39 us per launch on the shifted
-// 7-point 48^3 matrix, 51 us in FP64 on a 14^3 saddle point.)  Each column is
-// independent: the 2x2 coefficients are formed once per tile, and every
-// element keeps its operations, so the results keep their bits.
+// thread, a tile's loads all in flight.  Bound by the latency of a tile's batches,
+// one after another: on the 14^3 saddle point (FP64) 51 us per launch with all
+// nelim columns on the thread of a row, 28 us in tiles of 32 columns, 11 us in
+// tiles of 8.
 constexpr int CLD = LDLT_CLD, CLD_U = 8;
 template <typename T>
 __global__ void __launch_bounds__(LDLT_RT) k_ldlt_calc_ld(const T* __restrict__ arena,
@@ -1182,8 +1182,8 @@ __global__ void __launch_bounds__(LDLT_RT) k_ldlt_calc_ld(const T* __restrict__ 
         const double a = D[2 * p], b = D[2 * p + 1], cc = D[2 * p + 3];
         const double det = __dsub_rn(mul_(a, cc), mul_(b, b));
         kind[tid] = second ? 2 : 1;
-        ca[tid] = second ? -b / det : cc / det;
-        cb[tid] = second ? a / det : -b / det;
+        ca[tid] = quot(second ? -b : cc, det);
+        cb[tid] = quot(second ? a : -b, det);
       } else {
         kind[tid] = D[2 * k] == 0.0 ? 3 : 0;
         ca[tid] = D[2 * k];

@@ -7,7 +7,7 @@ namespace sylver_gb300 {
 
 constexpr int LDLT_BW = 32;   // block width of the a-posteriori pivoting
 constexpr int LDLT_RT = 128;  // rows per CTA tile in calc_ld
-constexpr int LDLT_CLD = 32;  // columns per CTA tile in calc_ld
+constexpr int LDLT_CLD = 8;   // columns per CTA tile in calc_ld (one batch of loads in flight)
 // Rows per CTA tile in apply / commit and the square tile of
 // the block steps' update.  FP64 takes the smallest: its multiply-adds run at
 // 2 per clock and SM, so a launch ends soonest with its rows over every SM

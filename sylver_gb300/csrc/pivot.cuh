@@ -1,5 +1,6 @@
 // Reciprocal square roots of Cholesky pivots without IEEE square root and
-// division, which cost several times as long on the chain of pivots.
+// division, which cost several times as long on the chain of pivots, and an FP64
+// quotient off the FP64 pipe.
 #pragma once
 
 #include <cfloat>
@@ -36,6 +37,48 @@ __device__ __forceinline__ double rsqrt64(double d) {
   const unsigned long long r = (unsigned long long)(y + (1 << 9)) >> 10;  // 53 bits
   return __longlong_as_double((long long)(((unsigned long long)(1021 - q) << 52) + r));
 }
+
+// a / b rounded to nearest even, bit for bit the IEEE quotient, in integer
+// arithmetic: a reciprocal of b's mantissa from the FP32 estimate y0 and y0 (1 + e +
+// e^2), e = 1 - f y0, a quotient within one unit, and the exact remainder.  About
+// 45 integer instructions; the FP64 pipe takes a dozen instructions of 65 clocks.
+// Operands or results without a normal exponent take the division itself.
+__device__ __noinline__ double div64_slow(double a, double b) { return a / b; }
+__device__ __forceinline__ double div64(double a, double b) {
+  const unsigned long long ab = (unsigned long long)__double_as_longlong(a);
+  const unsigned long long bb = (unsigned long long)__double_as_longlong(b);
+  const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff;
+  const int e = ea - eb + 1023;
+  if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff || e < 2 || e > 2045)
+    return div64_slow(a, b);
+  const unsigned long long ma = (ab & 0xfffffffffffffull) | (1ull << 52);
+  const unsigned long long mb = (bb & 0xfffffffffffffull) | (1ull << 52);
+  const float f = __uint_as_float(0x3f800000u | (unsigned)((mb >> 29) & 0x7fffff));
+  const unsigned Y = min((unsigned)(__fdividef(1.f, f) * 16777216.f), 16777215u);
+  // e in units of 2^-76 (2^76 - mb Y fits 64 bits), then e + e^2
+  const long long e76 = (long long)(0ull - mb * Y);
+  const long long h = e76 >> 24;
+  const long long d76 = e76 + ((h * h) >> 28);
+  // 2^63 / f and the quotient in units of 2^-62
+  const unsigned long long r63 =
+      ((unsigned long long)Y << 39) + (unsigned long long)(((long long)Y * (d76 >> 17)) >> 20);
+  const unsigned long long q62 = __umul64hi(ma << 11, r63);
+  const int lt = ma < mb;  // the quotient of the mantissas is below one
+  unsigned long long q = q62 >> (10 - lt);
+  long long rem = (long long)((ma << (52 + lt)) - q * mb);
+  if (rem < 0) {
+    --q;
+    rem += (long long)mb;
+  } else if (rem >= (long long)mb) {
+    ++q;
+    rem -= (long long)mb;
+  }
+  if (2 * rem > (long long)mb || (2 * rem == (long long)mb && (q & 1))) ++q;
+  return __longlong_as_double((long long)(((ab ^ bb) & 0x8000000000000000ull) |
+                                          (((unsigned long long)(e - lt - 1) << 52) + q)));
+}
+__device__ __forceinline__ double quot(double a, double b) { return div64(a, b); }
+__device__ __forceinline__ float quot(float a, float b) { return a / b; }
 
 // the same in FP32: the hardware estimate and one Newton step (about 1 ulp)
 __device__ __forceinline__ float rsqrt32(float d) {
