@@ -484,7 +484,7 @@ __device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __
           c[u] = fmaf(-l, lu, c[u]);
           e[u] = fmaf(-e[k], lu, e[u]);
         }
-        c[k] = lane == k ? d * r : l;
+        c[k] = lane == k ? pivot_sqrt(d, r) : l;
         if (lane == k) rinv[b + k] = r;
       }
       if (bad && lane == 0) atomicOr(status, ST_NOT_POSDEF);
@@ -503,12 +503,11 @@ __device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __
       else if ((q + 1) * (q + 2) / 2 <= x) ++q;
       const int tj = nt - 1 - q, ti = nt - 1 - (x - q * (q + 1) / 2);
       const int r0 = o + 4 * ti, c0 = o + 4 * tj;
-      float acc[4][4];  // acc[column][row]
+      float acc[4][4];  // acc[column][row]: summed before the entry, one rounding at its size
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const float4 y = *reinterpret_cast<const float4*>(&D[(c0 + v) * FLD + r0]);
-        acc[v][0] = y.x; acc[v][1] = y.y; acc[v][2] = y.z; acc[v][3] = y.w;
-      }
+      for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[v][u] = 0.f;
 #pragma unroll
       for (int k = 0; k < CB; ++k) {
         const float4 ra = *reinterpret_cast<const float4*>(&D[(b + k) * FLD + r0]);
@@ -517,13 +516,14 @@ __device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __
 #pragma unroll
         for (int v = 0; v < 4; ++v)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) acc[v][u] = fmaf(-rv[u], cv[v], acc[v][u]);
+          for (int u = 0; u < 4; ++u) acc[v][u] = fmaf(rv[u], cv[v], acc[v][u]);
       }
       // (entries above the diagonal of a diagonal tile are never used)
 #pragma unroll
-      for (int v = 0; v < 4; ++v)
-        *reinterpret_cast<float4*>(&D[(c0 + v) * FLD + r0]) =
-            make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+      for (int v = 0; v < 4; ++v) {
+        float4& y = *reinterpret_cast<float4*>(&D[(c0 + v) * FLD + r0]);
+        y = make_float4(y.x - acc[v][0], y.y - acc[v][1], y.z - acc[v][2], y.w - acc[v][3]);
+      }
     }
     __syncthreads();
   }

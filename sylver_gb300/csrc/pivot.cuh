@@ -80,10 +80,13 @@ __device__ __forceinline__ double div64(double a, double b) {
 __device__ __forceinline__ double quot(double a, double b) { return div64(a, b); }
 __device__ __forceinline__ float quot(float a, float b) { return a / b; }
 
-// the same in FP32: the hardware estimate and one Newton step (about 1 ulp)
+// the same in FP32: the hardware estimate and one step y (1 + e / 2), the residual
+// e = 1 - d y^2 with the product d y in two parts (about 0.5 ulp)
 __device__ __forceinline__ float rsqrt32(float d) {
   const float r = rsqrtf(d);
-  return d <= FLT_MAX ? r * fmaf(-0.5f * d * r, r, 1.5f) : 0.f;
+  const float h = d * r;
+  const float e = fmaf(-fmaf(d, r, -h), r, fmaf(-h, r, 1.f));
+  return d <= FLT_MAX ? fmaf(0.5f * r, e, r) : 0.f;
 }
 __device__ __forceinline__ double pivot_rsqrt(double d) { return rsqrt64(d); }
 __device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrt32(d); }
