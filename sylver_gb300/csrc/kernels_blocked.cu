@@ -468,15 +468,19 @@ __device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __
         e[u] = i1 < W ? D[(b + u) * FLD + i1] : 0.f;
       }
       bool bad = false;
+      // lane k + 1 forms the next pivot from its own l: one shuffle per column
+      // on the chain instead of two
+      float dn = __shfl_sync(FULL, c[0], 0);
 #pragma unroll
       for (int k = 0; k < CB; ++k) {
-        float d = __shfl_sync(FULL, c[k], k);
+        float d = dn;
         if (!(d > 0.f)) {
           bad = true;
           d = 1.f;
         }
         const float r = pivot_rsqrt(d);
         const float l = lane > k ? c[k] * r : 0.f;
+        if (k + 1 < CB) dn = __shfl_sync(FULL, fmaf(-l, l, c[k + 1]), k + 1);
         e[k] *= r;
 #pragma unroll
         for (int u = k + 1; u < CB; ++u) {
@@ -560,8 +564,11 @@ __device__ __forceinline__ void factor64(float* __restrict__ D, int w, float* __
 // itself, then solves rows [r0, r1) below it, 64 at a time.  A panel is latency
 // (four 16-column pivot chains, then four substitution steps), and a separate
 // launch for the diagonal block added its own start, a round trip of the block
-// and its inverses through memory, and the gap between the two (18 + 18 us a
-// panel at 80^3; see launch_blk_fused).  The CTA with xi >= 0 leaves the factor in
+// and its inverses through memory, and the gap between the two: 64^3 12.25 ms
+// of factorization with two launches, 11.2 with one; 14 us a panel where every
+// CTA has an SM to itself.  Repeating the block's factorization in each CTA is
+// not what bounds the launches of more rows: half or twice as many rows per CTA,
+// or 128 rows on eight warps, changed 80^3 by +0.5 to +3%.  The CTA with xi >= 0 leaves the factor in
 // dstore; k_diag_store32 moves it into the front when no CTA reads the
 // assembled block any more.
 __global__ void __launch_bounds__(PTHREADS) k_blk_fused(float* __restrict__ arena,

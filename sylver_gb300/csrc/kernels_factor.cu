@@ -290,7 +290,8 @@ __global__ void __launch_bounds__(256) k_assemble(T* __restrict__ arena,
 // tiles.  Bound by latency (FP32) and by the FP64 pipe: a rank-1 step
 // over the whole triangle per column, with an IEEE square root, a division and
 // three barriers on the chain and index divisions per entry, took 140-190 us
-// for fronts of 70 to 96 rows.
+// for fronts of 70 to 96 rows (12 x 12 grid, one launch: 0.13 ms of its 0.45 ms
+// call).
 template <typename T>
 __global__ void __launch_bounds__(256) k_small_chol(T* __restrict__ arena,
                                                     const SmallTask* __restrict__ tasks,
@@ -318,16 +319,21 @@ __global__ void __launch_bounds__(256) k_small_chol(T* __restrict__ arena,
       for (int u = 0; u < 8; ++u)
         c[u] = (u < w && lane >= u && i < m) ? s[(b + u) * lds + i] : T(0);
       bool bad = false;
+      // FP32: lane k + 1 forms the next pivot from its own l, one shuffle per
+      // column on the chain instead of two (FP64: one more instruction on its pipe)
+      constexpr bool AHEAD = sizeof(T) == 4;
+      T dn = __shfl_sync(FULL, c[0], 0);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         if (k >= w) break;
-        d[k] = __shfl_sync(FULL, c[k], k);
+        d[k] = AHEAD ? dn : __shfl_sync(FULL, c[k], k);
         if (!(d[k] > T(0))) {
           bad = true;
           d[k] = T(1);
         }
         r[k] = pivot_rsqrt(d[k]);
         c[k] = lane > k ? c[k] * r[k] : T(0);
+        if (AHEAD && k + 1 < 8) dn = __shfl_sync(FULL, fma(-c[k], c[k], c[k + 1]), k + 1);
 #pragma unroll
         for (int u = k + 1; u < 8; ++u) c[u] -= c[k] * __shfl_sync(FULL, c[k], u);
       }
