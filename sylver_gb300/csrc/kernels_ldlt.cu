@@ -420,11 +420,9 @@ __device__ __forceinline__ bool above(double x, double lim) {
 // into the apply panel; the least pivot with |x| > 1/u lowers npass_raw.
 // One row per thread with its 32 values in registers, every load in flight at
 // once, L read from shared memory in 16-byte broadcasts (with the row in shared
-// memory a multiply-add took two shared loads and a store).  FP64 is bound by
-// the FP64 pipe (560 multiply-adds per row at 2 per clock and SM, a warp
-// instruction every 64 clocks), so its rows are spread in CTAs of one warp.
-// Per launch on the shifted 48^3 (FP32) and the 14^3 saddle point (FP64): 42
-// and 50 us before, 14 and 31 us now.
+// memory a multiply-add took two shared loads and a store).  FP32 only; FP64
+// goes through k_app_apply64.  Per launch on the shifted 48^3: 42 us before,
+// 14 us now.
 template <typename T>
 __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict__ arena,
                                                              T* __restrict__ scratch,
@@ -643,8 +641,7 @@ __global__ void __launch_bounds__(T4) k_app_apply64(const double* __restrict__ a
 // columns).  The block's permutation is applied to its rows of the eliminated
 // columns.  The CTA with local index 0 stores D and the state.  One row per
 // thread, its 32 values in registers: 35 -> 16 us per launch on the shifted
-// 48^3 (FP32), 38 -> 22 us on the 14^3 saddle point (FP64; half of it the 32
-// FP64 divisions of a row).
+// 48^3.  FP32 only; FP64 goes through k_app_commit64.
 template <typename T>
 __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ arena,
                                                               T* __restrict__ scratch,

@@ -19,6 +19,15 @@
 // are each below 2^-62 of the product of the two row norms, against
 // 2^-53 per term of an FP64 sum; C itself is updated by one FP64 subtraction.
 //
+// Bound by the epilogue's conversions and additions as much as by the MMAs.  The
+// products with one digit of A take one or two MMAs, its digits of B side by side
+// (11 MMAs per 16 k instead of 28: one costs about 90 clocks for any N up to
+// 128); the seven accumulators change hands in two halves, so that one is
+// drained while the other fills; sixteen warps drain, and four of the seven
+// groups are rounded by adding a constant, since conversions run at 16 per clock
+// and SM.  Steady rate of useful FP64 operations: 26 TFLOP/s with an MMA per digit
+// pair and eight warps, 34 now (k_update on the FP64 pipe: 1.0).
+//
 // A row with an infinity or NaN gets a scale exponent that turns every entry
 // it touches into NaN, as the FP64 products would.
 #include "digits.cuh"

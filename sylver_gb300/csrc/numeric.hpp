@@ -217,8 +217,8 @@ struct FKeep {
   void set_scale(const double* scale_host, cudaStream_t s);  // null: none
   void apply_scale(cudaStream_t s);  // val <- S val S in place (no-op without S)
 
-  // tensor-core updates (FP32 Cholesky): stacked transposed operands, split
-  // into three BF16 planes
+  // tensor-core updates (Cholesky): stacked transposed operands, split into three
+  // BF16 planes (FP32) or seven digit planes (FP64)
   bool use_tc = true;
   struct TcLevel {
     int pitch;
@@ -226,7 +226,7 @@ struct FKeep {
     bool cb = false;         // operands in the contribution-block planes
   };
   std::vector<TcLevel> tclev;
-  std::vector<CUtensorMap> tmaps;   // three per tensor-core launch (one per BF16 plane)
+  std::vector<CUtensorMap> tmaps;   // per level: FP32 one per plane, FP64 A's and B's
   DevMem tcsplit, tctask, tcplanes, tcerr;
   // FP64: digit splits and row scale exponents; panel and diagonal-store tasks
   DevMem ozsplit, ozexp, panel64, diagst64;
