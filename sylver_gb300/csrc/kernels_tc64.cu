@@ -19,14 +19,19 @@
 // are each below 2^-62 of the product of the two row norms, against
 // 2^-53 per term of an FP64 sum; C itself is updated by one FP64 subtraction.
 //
-// Bound by the epilogue's conversions and additions as much as by the MMAs.  The
+// Bound by the MMAs, and next by the epilogue's additions (with those left out 55
+// TFLOP/s, with a third of the MMAs 56).  The
 // products with one digit of A take one or two MMAs, its digits of B side by side
 // (11 MMAs per 16 k instead of 28: one costs about 90 clocks for any N up to
 // 128); the seven accumulators change hands in two halves, so that one is
 // drained while the other fills; sixteen warps drain, and four of the seven
 // groups are rounded by adding a constant, since conversions run at 16 per clock
-// and SM.  Steady rate of useful FP64 operations: 26 TFLOP/s with an MMA per digit
-// pair and eight warps, 34 now (k_update on the FP64 pipe: 1.0).
+// and SM.  The additions of a group have no branch between them and the next
+// group's read: one wait per half, and warps without columns add too.  Steady rate
+// of useful FP64 operations (4500 rows, K = 2048): 26 TFLOP/s with an MMA per
+// digit pair and eight warps, 32 with a wait and a branch per group, 47 now
+// (k_update on the FP64 pipe: 1.0).  Loads do not bound it: handing a stage back
+// digit by digit instead of whole changed nothing.
 //
 // A row with an infinity or NaN gets a scale exponent that turns every entry
 // it touches into NaN, as the FP64 products would.
@@ -273,15 +278,18 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     int it = 0;
     bool ok = true;
     uint32_t ta = 0;  // this warp's columns of accumulator 0
-    // wait for group gr's accumulator and start its read into v (warp-uniform:
-    // tcgen05.ld is a warp-collective instruction)
+    // start the read of group gr's accumulator into v, after a wait for its half
+    // at the half's first group (warp-uniform: tcgen05.ld is a warp-collective
+    // instruction)
     auto fetch = [&](int gr, uint32_t (&v)[OZ_EC]) {
-      int ready = 0;
-      if (lane == 0)
-        ready = mbar_wait_or_abort(&acc_full[gr >= OZ_HALF], it & 1, err, abortp);
-      ready = __shfl_sync(0xffffffffu, ready, 0);
-      if (!ready) return false;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (gr == 0 || gr == OZ_HALF) {
+        int ready = 0;
+        if (lane == 0)
+          ready = mbar_wait_or_abort(&acc_full[gr >= OZ_HALF], it & 1, err, abortp);
+        ready = __shfl_sync(0xffffffffu, ready, 0);
+        if (!ready) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
       tmem_ld16_async(ta + (uint32_t)(gr * ON), v);
       return true;
     };
@@ -312,12 +320,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       for (int j = 0; j < OZ_EC; ++j) acc[j] = 0ull - bias;
       for (int kc = 0; kc < t.nk; kc += OZ_DRAIN) {
         uint32_t va[OZ_EC], vb[OZ_EC];
+        // (warps without columns add like the others: a branch around the
+        // additions kept them from mixing with the reads, 35.5 -> 31.9 TFLOP/s)
         auto add = [&](auto gc, uint32_t (&v)[OZ_EC]) {
-          if (on) {
 #pragma unroll
-            for (int j = 0; j < OZ_EC; ++j)
-              add_group<decltype(gc)::value>(acc[j], __uint_as_float(v[j]));
-          }
+          for (int j = 0; j < OZ_EC; ++j)
+            add_group<decltype(gc)::value>(acc[j], __uint_as_float(v[j]));
         };
         auto step = [&](auto gc, uint32_t (&cur)[OZ_EC], uint32_t (&nxt)[OZ_EC]) {
           constexpr int G = decltype(gc)::value;
