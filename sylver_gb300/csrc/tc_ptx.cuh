@@ -66,6 +66,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // K-major, 128-byte swizzle shared-memory matrix descriptor (tcgen05 format:
 // start >> 4 in bits 0-13, leading byte offset >> 4 in 16-29 (unused for a
 // swizzled K-major tile), stride byte offset >> 4 in 32-45 = 1024 B between
