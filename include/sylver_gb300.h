@@ -329,6 +329,13 @@ int sylver_gb300_tc_selfcheck(int rows, int k, double* max_rel_err);
  * row norms, in units of 2^-53; infinite if the infinity is not confined to
  * NaNs in its row and column. */
 int sylver_gb300_tc64_selfcheck(int rows, int k, int spread, int special, double* max_err);
+/* The same on a front whose every word holds a known value, rows scaled by up to
+ * 2^+-rowexp (at most 500), 32-column tiles if narrow: *max_err is the largest
+ * error of an entry over 2^-53 times ((k + 3) (|L| |L^T|)_ij + 9/8 |C_ij|), which an FP64
+ * update keeps to 1; *changed counts words outside the updated triangle that
+ * were written. */
+int sylver_gb300_tc64_entrycheck(int rows, int k, int spread, int rowexp, int narrow, int special,
+                                 double* max_err, long* changed);
 
 /* Diagnostic: the bounded wait of the dataflow solve sweep on a synthetic
  * one-task sweep.  starve != 0: the task waits on a counter nothing sets, so

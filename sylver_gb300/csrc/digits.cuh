@@ -39,20 +39,24 @@ __device__ __forceinline__ void norm_add(int& e, float& s, long long xb, bool& b
   }
 }
 
-// round(x 2^(62 - e)) as a 64-bit integer, |x| < 2^e
-__device__ __forceinline__ long long to_fixed(long long xb, int e) {
+// |round(x 2^(71 - e))| as a 72-bit integer (hi: its upper 8 bits), |x| < 2^e;
+// every bit of an entry down to 2^-18 of 2^e is kept
+__device__ __forceinline__ unsigned long long to_fixed(long long xb, int e, unsigned& hi) {
   const int ex = (int)((unsigned long long)xb >> 52) & 0x7ff;
   unsigned long long m = (unsigned long long)xb & 0xfffffffffffffull;
-  int sh = 62 - e - 1074;  // x = m 2^(max(ex, 1) - 1075)
+  int sh = 71 - e - 1074;  // x = m 2^(max(ex, 1) - 1075)
   if (ex) {
     m |= 1ull << 52;
     sh += ex - 1;
   }
-  unsigned long long f;
-  if (sh >= 0) f = m << min(sh, 63);
-  else if (sh < -54) f = 0;
-  else f = (m + (1ull << (-sh - 1))) >> (-sh);
-  return xb < 0 ? -(long long)f : (long long)f;
+  hi = 0;
+  if (sh > 0) {
+    sh = min(sh, 63);
+    hi = (unsigned)(m >> (64 - sh));
+    return m << sh;
+  }
+  if (sh < -54) return 0;
+  return sh < 0 ? (m + (1ull << (-sh - 1))) >> (-sh) : m;
 }
 
 // smallest exponent with 2^e above the norm of a running sum (a margin covers
@@ -69,25 +73,46 @@ __device__ __forceinline__ void norm_merge(int& e, float& s, int e2, float s2) {
   e = em;
 }
 
-// Digits of the fixed-point values of two neighbouring K columns, one 4-byte
-// store per plane at element offset o (even) of plane 0.
-__device__ __forceinline__ void store_digits(long long f0, long long f1, uint16_t* o,
-                                             int64_t pstride) {
+// Balanced digits (|d| <= 256, the sign included) of one entry of a row with
+// scale exponent e; zeros where the row is empty or has no finite scale.
+__device__ __forceinline__ void cut_digits(long long xb, int e, int (&d)[OZ_DIGITS]) {
+  unsigned hi = 0;
+  const unsigned long long lo =
+      e == OZ_EMPTY || e == OZ_NONFINITE ? 0ull : to_fixed(xb, e, hi);
+  const int sgn = xb < 0 ? -1 : 0;
+  auto cut = [](int& f) {  // the lowest digit of f; f <- the rest
+    const int q = ((f + 256) & 511) - 256;
+    f = (f - q) >> 9;
+    return q;
+  };
+  int f = (int)(lo & 0x3ffff);  // digits 8, 7 and a carry
+  d[7] = cut(f);
+  d[6] = cut(f);
+  const unsigned long long r = (((unsigned long long)hi << 46) | (lo >> 18)) + (unsigned)f;
+  f = (int)(r & 0x7ffffff);  // digits 6, 5, 4 and a carry
+  d[5] = cut(f);
+  d[4] = cut(f);
+  d[3] = cut(f);
+  f += (int)(r >> 27);
+  d[2] = cut(f);
+  d[1] = cut(f);
+  d[0] = f;
 #pragma unroll
-  for (int p = OZ_DIGITS - 1; p >= 0; --p) {
-    int d0, d1;
-    if (p > 0) {  // balanced digit in [-256, 255], the rest carries up
-      d0 = (((int)f0 + 256) & 511) - 256;
-      d1 = (((int)f1 + 256) & 511) - 256;
-      f0 = (f0 - d0) >> 9;
-      f1 = (f1 - d1) >> 9;
-    } else {
-      d0 = (int)f0;
-      d1 = (int)f1;
-    }
+  for (int p = 0; p < OZ_DIGITS; ++p) d[p] = (d[p] ^ sgn) - sgn;
+}
+
+// Digits of two neighbouring K columns of a row with scale exponent e, one
+// 4-byte store per plane at element offset o (even) of plane 0.
+__device__ __forceinline__ void store_digits(long long x0, long long x1, int e, uint16_t* o,
+                                             int64_t pstride) {
+  int d0[OZ_DIGITS], d1[OZ_DIGITS];
+  cut_digits(x0, e, d0);
+  cut_digits(x1, e, d1);
+#pragma unroll
+  for (int p = 0; p < OZ_DIGITS; ++p) {
     // small integers are exact in BF16: the upper half of the float
-    const unsigned b0 = __float_as_uint(__int2float_rn(d0));
-    const unsigned b1 = __float_as_uint(__int2float_rn(d1));
+    const unsigned b0 = __float_as_uint(__int2float_rn(d0[p]));
+    const unsigned b1 = __float_as_uint(__int2float_rn(d1[p]));
     *reinterpret_cast<uint32_t*>(o + p * pstride) = __byte_perm(b0, b1, 0x7632);
   }
 }

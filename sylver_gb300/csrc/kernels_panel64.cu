@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(P64_THREADS)
   constexpr int NC = PB / NG;         // columns per lane
   __shared__ double Ls[PB * PLD];     // Ls[k * PLD + i] = L(i, k), then L(i, k) / L(k, k)
   __shared__ double ds[PB], rinv[PB];
-  __shared__ long long F[RC][PB + 1];
+  __shared__ long long F[RC][PB + 1];  // rows to cut into digits
+  __shared__ int es[RC];               // and their scale exponents
   const P64Task t = tasks[blockIdx.x];
   double* a = arena + t.off;
   const int64_t ld = t.ld;
@@ -170,19 +171,18 @@ __global__ void __launch_bounds__(P64_THREADS)
       norm_merge(e, s, __shfl_xor_sync(0xffffffffu, e, o), __shfl_xor_sync(0xffffffffu, s, o));
       nf = __shfl_xor_sync(0xffffffffu, (int)nf, o) || nf;
     }
-    e = norm_exponent(e, s);
+    e = nf ? OZ_NONFINITE : norm_exponent(e, s);
     const int64_t srow = (int64_t)t.base + (r0 - t.r0);
-    if (cg == 0 && has) sexp[srow + tr] = nf ? OZ_NONFINITE : e;
-    const bool zero = nf || !(s > 0.f);
+    if (cg == 0) es[tr] = e;
+    if (cg == 0 && has) sexp[srow + tr] = e;
 #pragma unroll
-    for (int u = 0; u < NC; ++u)
-      F[tr][NG * u + cg] = zero ? 0ll : to_fixed(__double_as_longlong(v[u]), e);
+    for (int u = 0; u < NC; ++u) F[tr][NG * u + cg] = __double_as_longlong(v[u]);
     __syncthreads();
 #pragma unroll 1
     for (int rr = tid >> 4; rr < RC; rr += 8) {
       const int k = 2 * (tid & 15);
       if (r0 + rr < t.r1)
-        store_digits(F[rr][k], F[rr][k + 1], planes + (srow + rr) * pitch + k, pstride);
+        store_digits(F[rr][k], F[rr][k + 1], es[rr], planes + (srow + rr) * pitch + k, pstride);
     }
     __syncthreads();
   }

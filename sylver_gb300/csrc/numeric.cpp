@@ -379,6 +379,7 @@ void FKeep::plan_cholesky() {
   std::vector<UpdTask> upds;
   std::vector<TcSplit> tcs;
   std::vector<OzSplit> ozs;
+  std::vector<OzTask> ozt;
   std::vector<P64Task> pan64, dst64;
   dstore_blocks = 0;
   std::vector<TcTask> tct;
@@ -392,6 +393,8 @@ void FKeep::plan_cholesky() {
   // FP64 fronts: panel steps of NB columns in groups of OZ_GW, updates on the
   // tensor cores from operands cut into digits (kernels_tc64.cu)
   const bool oz = !f32 && use_tc && TC_ROWS > 0;
+  const int64_t oz_cap = 1ll << 29;  // operand entries per launch
+  oz_tasks = 0;
   // one update of rows [c, m) x columns [c, ce) of the given fronts by their
   // columns [k0, k0 + K), from digits of rows [c, m); with split a launch
   // before it cuts them, else the panel kernel did (level oz_level made)
@@ -427,17 +430,18 @@ void FKeep::plan_cholesky() {
       for (int col0 = u.c; col0 < u.ce; col0 += OZ_TILE_COLS)
         nt += (st.nrow[u.s] - col0 + 127) / 128;
     const int tw = nt <= OZ_FEW_TILES / 2 ? OZ_TILE_COLS / 2 : OZ_TILE_COLS;
-    const int64_t tk0 = (int64_t)tct.size();
+    const int64_t tk0 = (int64_t)ozt.size();
     for (const OzUpd& u : us) {
-      const int m = st.nrow[u.s], nk = (u.K + OZ_KC - 1) / OZ_KC;
+      const int m = st.nrow[u.s];
       for (int col0 = u.c; col0 < u.ce; col0 += tw)
         for (int row0 = col0; row0 < m; row0 += 128)
-          tct.push_back({off[u.s], ld[u.s], row0, col0, m, std::min(u.ce, col0 + tw),
-                         u.base + row0 - u.c, u.base + col0 - u.c, nk, 0});
+          ozt.push_back({off[u.s], ld[u.s], row0, col0, m, std::min(u.ce, col0 + tw),
+                         u.base + row0 - u.c, u.base + col0 - u.c, u.k0, u.K, 0});
       tc_flops[lvl] += 2.0 * u.K * ((double)(u.ce - u.c) * m -
                                     0.5 * (u.ce * (u.ce - 1.0) - u.c * (u.c - 1.0)));
     }
-    ops.push_back({Op::TCUPD, tk0, (int64_t)tct.size(), lvl});
+    ops.push_back({Op::TCUPD, tk0, (int64_t)ozt.size(), lvl});
+    oz_tasks = std::max(oz_tasks, (int64_t)ozt.size() - tk0);
   };
   std::vector<int> pos(st.n, -1);
   ops.clear();
@@ -747,19 +751,26 @@ void FKeep::plan_cholesky() {
                           n + cj * TM, m, m, 0, n, 0});
     }
     if ((int64_t)upds.size() > u0) ops.push_back({Op::UPD, u0, (int64_t)upds.size(), 0});
-    // FP64: fronts of like K together, so that the common pitch pads little,
-    // and at most 2^29 operand elements a launch (more only for one front)
+    // FP64: OZ_KB columns at a time, each with row scales of its own, for as many
+    // fronts as the digit planes hold
     std::stable_sort(ozc.begin(), ozc.end(), [](const OzUpd& x, const OzUpd& y) { return x.K > y.K; });
     for (size_t q = 0; q < ozc.size();) {
       std::vector<OzUpd> us;
-      const int pitch = round_up(ozc[q].K, 64), kmin = ozc[q].K / 2;
+      const int K = ozc[q].K;
       int64_t rows = 0;
-      while (q < ozc.size() && ozc[q].K >= kmin) {
-        rows += st.nrow[ozc[q].s] - ozc[q].c;
-        if (!us.empty() && rows * pitch > (1ll << 29)) break;
+      while (q < ozc.size()) {
+        const int64_t r = st.nrow[ozc[q].s] - ozc[q].c;
+        if (!us.empty() && (rows + r) * std::min(round_up(K, 64), OZ_KB) > oz_cap) break;
+        rows += r;
         us.push_back(ozc[q++]);
       }
-      oz_update(us, true, -1);
+      const int kb = (int)std::min<int64_t>(OZ_KB, std::max<int64_t>(64, oz_cap / rows / 64 * 64));
+      for (int k0 = 0; k0 < K; k0 += kb) {
+        std::vector<OzUpd> part;
+        for (const OzUpd& u : us)
+          if (u.K > k0) part.push_back({u.s, u.c, u.ce, k0, std::min(kb, u.K - k0), 0});
+        oz_update(part, true, -1);
+      }
     }
     if (!tcf.empty()) {
       const int pitch = cb_pitch;
@@ -837,6 +848,7 @@ void FKeep::plan_cholesky() {
   panel64.upload(pan64, s);
   diagst64.upload(dst64, s);
   tctask.upload(tct, s);
+  oztask.upload(ozt, s);
   blkdiag.upload(blkd, s);
   blkpanel.upload(blkp, s);
   upd.upload(upds, s);
@@ -880,7 +892,7 @@ void FKeep::upload_static(cudaStream_t s) {
     dstore.ensure((size_t)dstore_blocks * (precision == 1 ? BLK_B * BLK_B * sizeof(float) : 32 * 32 * sizeof(double)));
   if (blkinv_count > 0) blkinv.ensure((size_t)blkinv_count * BLK_B * BLK_B * sizeof(float));
   if (!tclev.empty() && precision != 1) {
-    // one buffer of seven digit planes and row exponents for all launches
+    // one buffer of digit planes and row exponents for all launches
     int64_t cap = 1, rows = 1;
     for (auto& L : tclev) {
       cap = std::max(cap, L.rows * L.pitch);
@@ -889,6 +901,7 @@ void FKeep::upload_static(cudaStream_t s) {
     plane_stride = round_up64(cap, 64);
     tcplanes.ensure((size_t)OZ_DIGITS * plane_stride * sizeof(uint16_t));
     ozexp.ensure((size_t)rows * sizeof(int));
+    ozredo.ensure(update_tc64_redo_words(oz_tasks) * sizeof(unsigned));
     tmaps.resize(2 * tclev.size());
     for (size_t l = 0; l < tclev.size(); ++l)
       make_digit_maps(&tmaps[2 * l], tcplanes.as<uint16_t>(), plane_stride, tclev[l].rows,
@@ -996,8 +1009,8 @@ void FKeep::run_ops(cudaStream_t s) {
           launch_update_tc(&tmaps[3 * op.aux], A, tctask.as<TcTask>() + op.a, (int)cnt,
                            tcerr.as<unsigned>(), s);
         else
-          launch_update_tc64(&tmaps[2 * op.aux], A, ozexp.as<int>(), tctask.as<TcTask>() + op.a,
-                             (int)cnt, tcerr.as<unsigned>(), s);
+          launch_update_tc64(&tmaps[2 * op.aux], A, ozexp.as<int>(), oztask.as<OzTask>() + op.a,
+                             (int)cnt, ozredo.as<unsigned>(), tcerr.as<unsigned>(), s);
         break;
     }
   }

@@ -218,7 +218,7 @@ struct FKeep {
   void apply_scale(cudaStream_t s);  // val <- S val S in place (no-op without S)
 
   // tensor-core updates (Cholesky): stacked transposed operands, split into three
-  // BF16 planes (FP32) or seven digit planes (FP64)
+  // BF16 planes (FP32) or eight digit planes (FP64)
   bool use_tc = true;
   struct TcLevel {
     int pitch;
@@ -228,8 +228,9 @@ struct FKeep {
   std::vector<TcLevel> tclev;
   std::vector<CUtensorMap> tmaps;   // per level: FP32 one per plane, FP64 A's and B's
   DevMem tcsplit, tctask, tcplanes, tcerr;
-  // FP64: digit splits and row scale exponents; panel and diagonal-store tasks
-  DevMem ozsplit, ozexp, panel64, diagst64;
+  // FP64: digit splits, row scale exponents and updates; panel and diagonal-store tasks
+  DevMem ozsplit, ozexp, oztask, ozredo, panel64, diagst64;
+  int64_t oz_tasks = 0;            // most tasks of an update launch
   // the factorised diagonal blocks of a level's panels, until its end
   DevMem dstore;
   int64_t dstore_blocks = 0;
