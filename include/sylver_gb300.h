@@ -345,6 +345,12 @@ int sylver_gb300_tc64_entrycheck(int rows, int k, int spread, int rowexp, int na
  * setting.  Returns 0 or a reference flag.  No reference counterpart. */
 int sylver_gb300_dataflow_selftest(int starve, unsigned* status, double* seconds);
 
+/* Diagnostic: the nth memory allocation of the library from now on reports out of
+ * memory without being tried (once; 0: none).  Returns how many allocations were
+ * left before the previous setting struck (0: it has, or there was none).
+ * Process-wide.  No reference counterpart. */
+int sylver_gb300_fail_allocation(int nth);
+
 /* Diagnostic: the device's FP64 fused multiply-add rate in TFLOP/s, from one
  * timed launch of independent fma chains on every SM (CUDA events, after a
  * warm-up launch); the denominator of the FP64 path's roofline.  Changes no

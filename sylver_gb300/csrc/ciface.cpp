@@ -11,6 +11,7 @@
 //   * CUDA failures return SYLVER_ERROR_CUDA_UNKNOWN instead of exit(1).
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <new>
 
 #include "../../include/sylver_gb300.h"
@@ -86,16 +87,24 @@ void factorize_common(bool posdef, const double* val_host, const double* val_dev
     FKeep* fk = fkeep ? static_cast<FKeep*>(*fkeep) : nullptr;
     if (fk && (fk->ak != ak || fk->posdef != posdef || fk->precision != precision)) {
       delete fk;
-      fk = nullptr;
+      *fkeep = fk = nullptr;
     }
     if (!fk) {
-      fk = new FKeep();
-      fk->ak = ak;
-      fk->posdef = posdef;
-      fk->precision = precision;
-      if (posdef) fk->plan_cholesky();
-      else plan_ldlt(*fk);
-      fk->upload_static(rt.stream);
+      // (a second time where the device has no room for the digit planes: FP64
+      // updates on the FP64 pipe, which need none)
+      std::unique_ptr<FKeep> nk;
+      for (bool tc : {true, false}) {
+        nk.reset();
+        nk.reset(new FKeep());
+        nk->ak = ak;
+        nk->posdef = posdef;
+        nk->precision = precision;
+        nk->use_tc = tc;
+        if (posdef) nk->plan_cholesky();
+        else plan_ldlt(*nk);
+        if (nk->upload_static(rt.stream)) break;
+      }
+      fk = nk.release();
       if (fkeep) *fkeep = fk;
     }
     fk->ir_tol = ir_tol;
@@ -678,6 +687,8 @@ void sylver_gb300_set_schedule(sylver_gb300_schedule_t const* s) {
   c.front_memory = s->front_memory;
   c.solve_dataflow = s->solve_dataflow;
 }
+
+int sylver_gb300_fail_allocation(int nth) { return fail_allocation(nth); }
 
 void sylver_gb300_get_schedule(sylver_gb300_schedule_t* s) {
   if (!s) return;

@@ -127,6 +127,7 @@ void grow(DevMem& d, size_t bytes, cudaStream_t s) {
   if (bytes <= d.bytes && d.p) return;
   size_t nb = std::max(bytes, d.bytes + d.bytes / 2);
   void* np = nullptr;
+  if (alloc_fails()) throw CudaError("out of device memory");
   SG_CUDA(cudaMalloc(&np, nb));
   if (d.p && d.bytes) SG_CUDA(cudaMemcpyAsync(np, d.p, d.bytes, cudaMemcpyDeviceToDevice, s));
   SG_CUDA(cudaStreamSynchronize(s));

@@ -12,6 +12,7 @@
 #include "../../include/sylver_gb300.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <climits>
@@ -31,6 +32,15 @@ Schedule& Schedule::current() {
   static Schedule s;
   return s;
 }
+
+static std::atomic<int> g_fail_alloc{0};
+bool alloc_fails() {
+  int n = g_fail_alloc.load(std::memory_order_relaxed);
+  while (n > 0 && !g_fail_alloc.compare_exchange_weak(n, n - 1)) {
+  }
+  return n == 1;
+}
+int fail_allocation(int nth) { return g_fail_alloc.exchange(std::max(nth, 0)); }
 
 bool Runtime::init() {
   if (ok) return true;
@@ -166,6 +176,10 @@ inline bool is_large(const FrontDesc& d) {
 }
 inline int round_up(int v, int a) { return (v + a - 1) / a * a; }
 inline int64_t round_up64(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
+// operand entries of an FP64 update launch, for front storage of `elems` entries
+inline int64_t oz_entries(int64_t elems) {
+  return std::min(OZ_MAX_ENTRIES, std::max(OZ_MIN_ENTRIES, elems / 8));
+}
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -182,6 +196,9 @@ void FKeep::plan_cholesky() {
   const Schedule& sched = Schedule::current();
   const int SMALL_M = sched.small_rows(f32 ? Tiles<float>::SMALL_M : Tiles<double>::SMALL_M, f32);
   const int TC_ROWS = sched.tc_rows();
+  // FP64 fronts: panel steps of NB columns in groups of OZ_GW, updates on the
+  // tensor cores from operands cut into digits (kernels_tc64.cu)
+  const bool oz = !f32 && use_tc && TC_ROWS > 0;
 
   order.resize(ns);
   std::iota(order.begin(), order.end(), 0);
@@ -211,8 +228,10 @@ void FKeep::plan_cholesky() {
   size_t freeb = 0, totb = 0;
   SG_CUDA(cudaMemGetInfo(&freeb, &totb));
   const int fmem = sched.front_memory;
-  reuse_blocks = fmem > 0 || (fmem == 0 && (double)blocks * (f32 ? sizeof(float) : sizeof(double)) >
-                                               0.5 * (double)totb);
+  const double planes = oz ? 2.0 * OZ_DIGITS * (double)oz_entries(blocks) : 0.0;
+  reuse_blocks =
+      fmem > 0 || (fmem == 0 && (double)blocks * (f32 ? sizeof(float) : sizeof(double)) + planes >
+                                    0.5 * (double)totb);
   {
     ArenaAlloc al;
     std::vector<int> pend;
@@ -390,14 +409,11 @@ void FKeep::plan_cholesky() {
   blkinv_count = 0;
   const int PW = (f32 && use_tc) ? sched.panel_cols() : 0;
   blk_pw = PW;
-  // FP64 fronts: panel steps of NB columns in groups of OZ_GW, updates on the
-  // tensor cores from operands cut into digits (kernels_tc64.cu)
-  const bool oz = !f32 && use_tc && TC_ROWS > 0;
-  const int64_t oz_cap = 1ll << 29;  // operand entries per launch
+  const int64_t oz_cap = oz_entries(arena_elems);  // operand entries per launch
   oz_tasks = 0;
   // one update of rows [c, m) x columns [c, ce) of the given fronts by their
-  // columns [k0, k0 + K), from digits of rows [c, m); with split a launch
-  // before it cuts them, else the panel kernel did (level oz_level made)
+  // columns [k0, k0 + K), from digits of rows [c, m) cut by a launch before it
+  // (split) or by the panel kernel (level oz_level made)
   struct OzUpd {
     int s, c, ce, k0, K, base;
   };
@@ -415,7 +431,7 @@ void FKeep::plan_cholesky() {
     tc_flops.push_back(0.0);
     return (int)tclev.size() - 1;
   };
-  auto oz_update = [&](std::vector<OzUpd>& us, bool split, int lvl) {
+  auto oz_launch = [&](std::vector<OzUpd>& us, bool split, int lvl) {
     if (us.empty()) return;
     if (split) {
       lvl = oz_level(us, 64);
@@ -442,6 +458,31 @@ void FKeep::plan_cholesky() {
     }
     ops.push_back({Op::TCUPD, tk0, (int64_t)ozt.size(), lvl});
     oz_tasks = std::max(oz_tasks, (int64_t)ozt.size() - tk0);
+  };
+  // the updates cut beforehand by launches of their own, as many fronts together as
+  // the planes hold (one whose columns they do not hold in pieces of K)
+  auto oz_update = [&](const std::vector<OzUpd>& us) {
+    for (size_t q = 0; q < us.size();) {
+      std::vector<OzUpd> part;
+      int64_t rows = 0;
+      int K = 0;
+      for (; q < us.size(); ++q) {
+        const int64_t r = rows + st.nrow[us[q].s] - us[q].c;
+        const int k = std::max(K, us[q].K);
+        if (!part.empty() && r * round_up(k, 64) > oz_cap) break;
+        rows = r;
+        K = k;
+        part.push_back(us[q]);
+      }
+      const int kb = (int)std::max<int64_t>(64, oz_cap / rows / 64 * 64);
+      for (int k0 = 0; k0 < K; k0 += kb) {
+        std::vector<OzUpd> piece;
+        for (const OzUpd& u : part)
+          if (u.K > k0)
+            piece.push_back({u.s, u.c, u.ce, u.k0 + k0, std::min(kb, u.K - k0), 0});
+        oz_launch(piece, true, -1);
+      }
+    }
   };
   std::vector<int> pos(st.n, -1);
   ops.clear();
@@ -669,7 +710,8 @@ void FKeep::plan_cholesky() {
       for (int s : large) maxsteps = std::max(maxsteps, (st.ncol[s] + NB - 1) / NB);
     }
     const int64_t ds0 = (int64_t)dst64.size();
-    for (int step = 0; step < maxsteps; ++step) {
+    // one panel step of the given fronts; what it updates outside its group
+    auto panel_step = [&](int step, const std::vector<int>& fronts, std::vector<OzUpd>& later) {
       int64_t p0 = (int64_t)panels.size(), u0 = (int64_t)upds.size();
       int64_t d0 = (int64_t)diags.size(), q0 = (int64_t)pan64.size();
       const int k0 = step * NB;
@@ -680,7 +722,7 @@ void FKeep::plan_cholesky() {
       const int g0 = k0 / OZ_GW * OZ_GW, o = k0 + NB;
       const bool gend = o == g0 + OZ_GW;
       int64_t below = 0;
-      for (int s : large) {
+      for (int s : fronts) {
         const int m = st.nrow[s], n = st.ncol[s];
         if (k0 < n) below += m - std::min(o, n);
         if (oz && o < n)
@@ -695,7 +737,7 @@ void FKeep::plan_cholesky() {
                            ? 16
                            : std::max(32, std::min(256, (int)(below / OZ_FEW_TILES) / 32 * 32));
       size_t qi = 0;
-      for (int s : large) {
+      for (int s : fronts) {
         const int m = st.nrow[s], n = st.ncol[s];
         if (k0 >= n) continue;
         const int w = std::min(NB, n - k0);
@@ -728,7 +770,25 @@ void FKeep::plan_cholesky() {
       if ((int64_t)panels.size() > p0) ops.push_back({Op::PANEL, p0, (int64_t)panels.size(), 0});
       if ((int64_t)pan64.size() > q0) ops.push_back({Op::PANEL, q0, (int64_t)pan64.size(), lvl, rt64});
       if ((int64_t)upds.size() > u0) ops.push_back({Op::UPD, u0, (int64_t)upds.size(), 0});
-      oz_update(ozp, gend, lvl);
+      if (gend) later.insert(later.end(), ozp.begin(), ozp.end());
+      else oz_launch(ozp, false, lvl);
+    };
+    for (int step = 0; step < maxsteps; ++step) {
+      // (the fronts whose rows the digit planes hold together)
+      std::vector<OzUpd> later;
+      for (size_t q = 0; q < large.size();) {
+        std::vector<int> fronts;
+        int64_t rows = 0;
+        for (; q < large.size(); ++q) {
+          const int m = st.nrow[large[q]], o = (step + 1) * NB;
+          const int64_t r = rows + (oz && o < st.ncol[large[q]] ? m - o : 0);
+          if (!fronts.empty() && r * OZ_KC > oz_cap) break;
+          rows = r;
+          fronts.push_back(large[q]);
+        }
+        panel_step(step, fronts, later);
+      }
+      oz_update(later);
     }
     if ((int64_t)dst64.size() > ds0) {
       ops.push_back({Op::DIAG, ds0, (int64_t)dst64.size(), 0});
@@ -751,26 +811,13 @@ void FKeep::plan_cholesky() {
                           n + cj * TM, m, m, 0, n, 0});
     }
     if ((int64_t)upds.size() > u0) ops.push_back({Op::UPD, u0, (int64_t)upds.size(), 0});
-    // FP64: OZ_KB columns at a time, each with row scales of its own, for as many
-    // fronts as the digit planes hold
+    // FP64: OZ_KB columns at a time, each with row scales of its own
     std::stable_sort(ozc.begin(), ozc.end(), [](const OzUpd& x, const OzUpd& y) { return x.K > y.K; });
-    for (size_t q = 0; q < ozc.size();) {
+    for (int k0 = 0; !ozc.empty() && k0 < ozc[0].K; k0 += OZ_KB) {
       std::vector<OzUpd> us;
-      const int K = ozc[q].K;
-      int64_t rows = 0;
-      while (q < ozc.size()) {
-        const int64_t r = st.nrow[ozc[q].s] - ozc[q].c;
-        if (!us.empty() && (rows + r) * std::min(round_up(K, 64), OZ_KB) > oz_cap) break;
-        rows += r;
-        us.push_back(ozc[q++]);
-      }
-      const int kb = (int)std::min<int64_t>(OZ_KB, std::max<int64_t>(64, oz_cap / rows / 64 * 64));
-      for (int k0 = 0; k0 < K; k0 += kb) {
-        std::vector<OzUpd> part;
-        for (const OzUpd& u : us)
-          if (u.K > k0) part.push_back({u.s, u.c, u.ce, k0, std::min(kb, u.K - k0), 0});
-        oz_update(part, true, -1);
-      }
+      for (const OzUpd& u : ozc)
+        if (u.K > k0) us.push_back({u.s, u.c, u.ce, k0, std::min(OZ_KB, u.K - k0), 0});
+      oz_update(us);
     }
     if (!tcf.empty()) {
       const int pitch = cb_pitch;
@@ -865,7 +912,7 @@ void FKeep::plan_cholesky() {
   num_flops = st.num_flops;
 }
 
-void FKeep::upload_static(cudaStream_t s) {
+bool FKeep::upload_static(cudaStream_t s) {
   AKeep& a = *ak;
   frow.upload(a.frow, s);
   fcol.upload(a.fcol, s);
@@ -899,7 +946,7 @@ void FKeep::upload_static(cudaStream_t s) {
       rows = std::max(rows, L.rows);
     }
     plane_stride = round_up64(cap, 64);
-    tcplanes.ensure((size_t)OZ_DIGITS * plane_stride * sizeof(uint16_t));
+    if (!tcplanes.try_ensure((size_t)OZ_DIGITS * plane_stride * sizeof(uint16_t))) return false;
     ozexp.ensure((size_t)rows * sizeof(int));
     ozredo.ensure(update_tc64_redo_words(oz_tasks) * sizeof(unsigned));
     tmaps.resize(2 * tclev.size());
@@ -923,6 +970,7 @@ void FKeep::upload_static(cudaStream_t s) {
         make_panel_map(&tmaps[3 * l + q], pl, tclev[l].rows, tclev[l].pitch);
       }
   }
+  return true;
 }
 
 template <typename T>

@@ -20,6 +20,11 @@
 
 namespace sylver_gb300 {
 
+// Test hook (sylver_gb300_fail_allocation): whether this allocation reports out of
+// memory without being tried.
+bool alloc_fails();
+int fail_allocation(int nth);
+
 // Owned device allocation.
 struct DevMem {
   void* p = nullptr;
@@ -33,12 +38,23 @@ struct DevMem {
     p = nullptr;
     bytes = 0;
   }
-  void ensure(size_t nbytes) {
-    if (nbytes <= bytes && p) return;
+  // false: out of device memory
+  bool try_ensure(size_t nbytes) {
+    if (nbytes <= bytes && p) return true;
     release();
-    if (nbytes == 0) return;
-    SG_CUDA(cudaMalloc(&p, nbytes));
+    if (nbytes == 0) return true;
+    const cudaError_t e = alloc_fails() ? cudaErrorMemoryAllocation : cudaMalloc(&p, nbytes);
+    if (e == cudaErrorMemoryAllocation) {
+      p = nullptr;
+      (void)cudaGetLastError();
+      return false;
+    }
+    SG_CUDA(e);
     bytes = nbytes;
+    return true;
+  }
+  void ensure(size_t nbytes) {
+    if (!try_ensure(nbytes)) throw CudaError("out of device memory");
   }
   template <typename T> T* as() const { return static_cast<T*>(p); }
   template <typename T> void upload(const std::vector<T>& v, cudaStream_t s) {
@@ -333,7 +349,8 @@ struct FKeep {
 
   ~FKeep();
   void plan_cholesky();
-  void upload_static(cudaStream_t s);
+  // false: no room for the digit planes (plan again with use_tc = false)
+  bool upload_static(cudaStream_t s);
   // Factorize from device values (val_dev: original val layout, nnz entries).
   int factorize(const double* val_dev, cudaStream_t s);
   // Solve in place on device; x is ldx x nrhs in user order.

@@ -48,6 +48,11 @@ constexpr int OZ_GW = 256;  // fully-summed columns per trailing update
 // own: 56^3 13.8 ms of updates, 14.1 with 256, 13.9 with 1024 columns (all K columns
 // at once: more rows far below their scale, 20 ms when their warps redid them).
 constexpr int OZ_KB = 512;
+// Operand entries an update launch cuts at most (16 bytes of digit planes each): an
+// eighth of the front storage's, within these limits (64 MiB to 2 GiB of planes).
+// Level and front sizes do not set the size of the planes: what does not fit goes
+// in several launches, each still of thousands of tile columns.
+constexpr int64_t OZ_MIN_ENTRIES = 1 << 22, OZ_MAX_ENTRIES = 1 << 27;
 constexpr int OZ_FEW_TILES = 304;  // launches below this many CTAs take smaller tiles
 // Digits of front rows [r0, r0 + rows) x columns [c0, c0 + K): stacked rows
 // [base, base + rows) of the planes (zeros from K to K rounded up to
