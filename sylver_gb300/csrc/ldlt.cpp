@@ -26,7 +26,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <numeric>
 #include <type_traits>
 
@@ -38,21 +41,37 @@ namespace sylver_gb300 {
 
 // Pinned host memory for the tables a level uploads, handed out front to back.
 // reset() once every copy out of it has completed; a request beyond the
-// capacity moves to a larger block, the old one is kept until the reset.
+// capacity moves to a larger block, the old one is kept until the reset.  Where the
+// host gives no pinned memory the block is pageable: copies from it then make the
+// host wait, with the same results.
 struct PinnedStage {
-  char* p = nullptr;
+  struct Block {
+    char* p = nullptr;
+    bool pinned = false;
+    explicit Block(size_t n) {
+      void* q = nullptr;
+      pinned = !alloc_fails() && cudaMallocHost(&q, n) == cudaSuccess;
+      if (!pinned) {
+        (void)cudaGetLastError();
+        q = std::malloc(n);
+        if (!q) throw std::bad_alloc();
+      }
+      p = static_cast<char*>(q);
+    }
+    Block(const Block&) = delete;
+    Block& operator=(const Block&) = delete;
+    ~Block() {
+      if (pinned) cudaFreeHost(p);
+      else std::free(p);
+    }
+  };
+  std::vector<std::unique_ptr<Block>> blocks;  // the last one is handed out
   size_t cap = 0, used = 0, want = 0;
-  std::vector<void*> old;
-  PinnedStage() = default;
-  PinnedStage(const PinnedStage&) = delete;
-  PinnedStage& operator=(const PinnedStage&) = delete;
-  ~PinnedStage() {
-    reset();
-    if (p) cudaFreeHost(p);
+  ~PinnedStage() {  // (a factorization that failed may have left copies in flight)
+    if (used) cudaStreamSynchronize(Runtime::get().stream);
   }
   void reset() {
-    for (void* q : old) cudaFreeHost(q);
-    old.clear();
+    if (blocks.size() > 1) blocks.erase(blocks.begin(), blocks.end() - 1);
     used = want = 0;
   }
   void* take(size_t bytes) {
@@ -60,14 +79,11 @@ struct PinnedStage {
     want += bytes;
     if (used + bytes > cap) {
       const size_t nc = std::max(2 * cap, std::max<size_t>(2 * want, 1 << 20));
-      void* np = nullptr;
-      SG_CUDA(cudaMallocHost(&np, nc));
-      if (p) old.push_back(p);
-      p = static_cast<char*>(np);
+      blocks.push_back(std::make_unique<Block>(nc));
       cap = nc;
       used = 0;
     }
-    void* q = p + used;
+    void* q = blocks.back()->p + used;
     used += bytes;
     return q;
   }
