@@ -657,9 +657,10 @@ __global__ void __launch_bounds__(4 * LB) k_inv_diag(const T* __restrict__ arena
 #pragma unroll
   for (int u = 0; u < NU; ++u) {
     const int i = 4 * u + c;
-    // z / L(i, i): product with the reciprocal, corrected by its remainder
+    // z / L(i, i): product with the reciprocal, corrected by its remainder (which
+    // an infinite L(i, i) does not have)
     const T q = z[u] * rd[i];
-    const T r = fma(-q, dg[i], z[u]);
+    const T r = rd[i] != T(0) ? fma(-q, dg[i], z[u]) : T(0);
     out[i] = fma(r, rd[i], q);
   }
 }
