@@ -337,6 +337,11 @@ int sylver_gb300_tc64_selfcheck(int rows, int k, int spread, int special, double
 int sylver_gb300_tc64_entrycheck(int rows, int k, int spread, int rowexp, int narrow, int special,
                                  double* max_err, long* changed);
 
+/* Self-check of the factorizations' scalar arithmetic on n operands (host memory):
+ * op 0 a / b, 1 1 / sqrt(a), 2 sqrt(a) (FP64); 3 1 / sqrt(a), 4 sqrt(a) with a
+ * rounded to FP32.  a > 0 for ops 1 to 4; b is read by op 0 only. */
+int sylver_gb300_pivot_math(int op, long n, double const* a, double const* b, double* out);
+
 /* Diagnostic: the bounded wait of the dataflow solve sweep on a synthetic
  * one-task sweep.  starve != 0: the task waits on a counter nothing sets, so
  * the wait must give up (ST_TIMEOUT, 32, in *status) and the launch finish;

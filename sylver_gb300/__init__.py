@@ -129,6 +129,7 @@ EXPORTS = (
     "sylver_gb300_fkeep_fronts", "sylver_gb300_akeep_scaling", "sylver_gb300_profile_levels",
     "sylver_gb300_stream", "sylver_gb300_profile_factor", "spldlt_tree_solve_fwd_noalloc_dbl",
     "sylver_gb300_tc_selfcheck", "sylver_gb300_tc64_selfcheck", "sylver_gb300_tc64_entrycheck",
+    "sylver_gb300_pivot_math",
     "sylver_gb300_fail_allocation", "sylver_gb300_fp64_fma_rate", "sylver_gb300_fkeep_factor_bytes",
     "sylver_gb300_dataflow_selftest",
     "sylver_gb300_solve_history", "sylver_gb300_set_schedule",
@@ -184,6 +185,7 @@ def load(path: str | None = None):
         "sylver_gb300_tc64_selfcheck": (I, [I, I, I, I, ctypes.POINTER(D)]),
         "sylver_gb300_tc64_entrycheck": (I, [I, I, I, I, I, I, ctypes.POINTER(D),
                                              ctypes.POINTER(L)]),
+        "sylver_gb300_pivot_math": (I, [I, L, P, P, P]),
         "sylver_gb300_fail_allocation": (I, [I]),
         "sylver_gb300_dataflow_selftest": (I, [I, ctypes.POINTER(ctypes.c_uint), ctypes.POINTER(D)]),
         "sylver_gb300_fp64_fma_rate": (I, [ctypes.POINTER(D)]),
