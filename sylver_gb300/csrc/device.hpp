@@ -13,6 +13,11 @@
 
 namespace sylver_gb300 {
 
+// SMs of a GB300.  Launches are cut and blocks are dealt out for this number (a launch of
+// another size runs as well, a little less evenly); where a kernel rotates work over an
+// SM's schedulers it assumes blocks b and b + NUM_SMS to share one, for speed only.
+constexpr int NUM_SMS = 152;
+
 struct CudaError : std::runtime_error {
   explicit CudaError(const std::string& s) : std::runtime_error(s) {}
 };
@@ -138,7 +143,7 @@ struct UpdTask {
 // most BLK_W columns (a multiple of BLK_B by schedule choice).
 constexpr int BLK_B = 64;
 constexpr int BLK_W = 256;
-constexpr int BLK_FEW_CTAS = 608;  // four CTAs of the fused panel kernel per SM
+constexpr int BLK_FEW_CTAS = 4 * NUM_SMS;  // four CTAs of the fused panel kernel per SM
 // k per pipeline stage of the tensor-core update (BF16 elements); stacked
 // panel pitches are multiples of it
 constexpr int TC_KCHUNK = 64;
@@ -225,7 +230,7 @@ void launch_extend_add_grouped(T* arena, const ChildDesc* cd, const EaItem* item
 // arow/asrc[acp[cbase + j], acp[cbase + j + 1]) (distinct rows >= j) and the
 // children's CB columns that land in it are items[gptr[cbase + j],
 // gptr[cbase + j + 1]) in child order (at most 32, maps that keep row order).
-constexpr int ASM_TASKS = 152 * 6;  // CTAs a level's assembly is cut into, if it can be
+constexpr int ASM_TASKS = NUM_SMS * 6;  // CTAs a level's assembly is cut into, if it can be
 struct AsmTask {
   int64_t off;
   int ld, m, j0, j1, cbase, pad;

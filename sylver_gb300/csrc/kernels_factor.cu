@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) k_small_chol(T* __restrict__ arena,
   for (int b = 0; b < n; b += 8) {
     const int w = min(8, n - b);
     // (CTAs that share an SM spread over its schedulers)
-    if (warp == (blockIdx.x / 152 & 7)) {
+    if (warp == (blockIdx.x / NUM_SMS & 7)) {
       const int i = b + lane;
       T c[8], d[8], r[8];
 #pragma unroll
@@ -540,7 +540,7 @@ template <typename T>
 void launch_init_a(T* arena, const double* val, const int64_t* src, const int64_t* dst,
                    int64_t count, bool atomic, cudaStream_t s) {
   if (count <= 0) return;
-  int64_t blocks = std::min<int64_t>((count + 255) / 256, 152 * 32);
+  int64_t blocks = std::min<int64_t>((count + 255) / 256, NUM_SMS * 32);
   k_init_a<T><<<(int)blocks, 256, 0, s>>>(arena, val, src, dst, count, atomic);
 }
 

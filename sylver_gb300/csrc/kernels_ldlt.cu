@@ -39,7 +39,6 @@
 // that a CPU restatement with std::fma in the same order reproduces the
 // factors bit for bit.
 #include <cfloat>
-#include <type_traits>
 
 #include "ldlt_dev.hpp"
 #include "pivot.cuh"
@@ -114,7 +113,7 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
 // Output: the factored block (unit L, lower) in blk, D^-1, the local
 // permutation, the number of pivots taken (ndiag, also the initial
 // npass_raw), the L rows of the e extra rows into the apply panel; the block
-// permutation is applied to the variable list (k_app_commit applies it to the
+// permutation is applied to the variable list (the commit applies it to the
 // rows of the eliminated columns).
 //
 // Bound by the serial chain of pivots.  The triangle stays in registers, three
@@ -420,19 +419,14 @@ __device__ __forceinline__ bool above(double x, double lim) {
 // into the apply panel; the least pivot with |x| > 1/u lowers npass_raw.
 // One row per thread with its 32 values in registers, every load in flight at
 // once, L read from shared memory in 16-byte broadcasts (with the row in shared
-// memory a multiply-add took two shared loads and a store).  FP32 only; FP64
-// goes through k_app_apply64.  Per launch on the shifted 48^3: 42 us before,
+// memory a multiply-add took two shared loads and a store).  FP64 goes
+// through k_app_apply64.  Per launch on the shifted 48^3: 42 us before,
 // 14 us now.
-template <typename T>
-__global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict__ arena,
-                                                             T* __restrict__ scratch,
-                                                             const LdltFront* __restrict__ fr,
-                                                             const CtaMap* __restrict__ cm,
-                                                             LdltStep st) {
-  using C = T;
-  constexpr int RT = AppRows<T>::v, V = 16 / (int)sizeof(C), LP = BW + V;
-  using Vec = typename std::conditional<sizeof(C) == 4, float4, double2>::type;
-  __shared__ __align__(16) C L[BW][LP];  // zero past the ndiag pivots
+__global__ void __launch_bounds__(AppRows<float>::v)
+    k_app_apply32(const float* __restrict__ arena, float* __restrict__ scratch,
+                  const LdltFront* __restrict__ fr, const CtaMap* __restrict__ cm, LdltStep st) {
+  constexpr int RT = AppRows<float>::v;
+  __shared__ __align__(16) float L[BW][BW + 4];  // zero past the ndiag pivots
   __shared__ double dv[2 * BW];
   __shared__ int perm[BW], kind[BW];
   __shared__ int fail;
@@ -441,13 +435,13 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
   const int q = F.fidx, w = block_width(F, st.k), e = extra_rows(F, w);
   const int p = st.p_cur[q], nd = st.ndiag[q];
   if (nd == 0) return;
-  const T* A = arena + F.off;
+  const float* A = arena + F.off;
   const int64_t ld = F.ld, pm = F.m;
   const int tid = threadIdx.x;
-  const C* blk = reinterpret_cast<const C*>(st.blk) + (int64_t)q * BW * LDB;
+  const float* blk = reinterpret_cast<const float*>(st.blk) + (int64_t)q * BW * LDB;
   for (int idx = tid; idx < BW * BW; idx += RT) {
     const int j = idx / BW, k = idx % BW;
-    L[j][k] = (j < nd && k < nd) ? blk[j * LDB + k] : C(0);
+    L[j][k] = (j < nd && k < nd) ? blk[j * LDB + k] : 0.f;
   }
   for (int k = tid; k < 2 * BW; k += RT) dv[k] = st.bdinv[q * 2 * BW + k];
   if (tid < BW) perm[tid] = st.lperm[q * BW + tid];
@@ -458,31 +452,26 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
   const BelowRows br{p + w, F.n, e, F.m};
   const int nrow = br.count();
   const double lim = quot(1.0, st.u);
-  T* pan = scratch + F.pan_off;
+  float* pan = scratch + F.pan_off;
   for (int t0 = c.local * RT; t0 < nrow; t0 += c.count * RT) {
     const int ci = t0 + tid;
     if (ci < nrow) {
       const int r = br.row(ci);
-      C x[BW];
+      float x[BW];
 #pragma unroll
-      for (int k = 0; k < BW; ++k) x[k] = k < nd ? (C)A[(p + perm[k]) * ld + r] : C(0);
+      for (int k = 0; k < BW; ++k) x[k] = k < nd ? A[(p + perm[k]) * ld + r] : 0.f;
       // x L^T = a  (unit lower L)
 #pragma unroll
       for (int j = 0; j < BW - 1; ++j) {
         if (j >= nd) break;
-        const C xj = -x[j];
+        const float xj = -x[j];
 #pragma unroll
-        for (int kv = (j + 1) / V * V; kv < BW; kv += V) {
-          const Vec lv = *reinterpret_cast<const Vec*>(&L[j][kv]);
-          if constexpr (V == 4) {
-            if (kv > j) x[kv] = fma_(xj, lv.x, x[kv]);
-            if (kv + 1 > j) x[kv + 1] = fma_(xj, lv.y, x[kv + 1]);
-            if (kv + 2 > j) x[kv + 2] = fma_(xj, lv.z, x[kv + 2]);
-            x[kv + 3] = fma_(xj, lv.w, x[kv + 3]);
-          } else {
-            if (kv > j) x[kv] = fma_(xj, lv.x, x[kv]);
-            x[kv + 1] = fma_(xj, lv.y, x[kv + 1]);
-          }
+        for (int kv = (j + 1) / 4 * 4; kv < BW; kv += 4) {
+          const float4 lv = *reinterpret_cast<const float4*>(&L[j][kv]);
+          if (kv > j) x[kv] = fma_(xj, lv.x, x[kv]);
+          if (kv + 1 > j) x[kv + 1] = fma_(xj, lv.y, x[kv + 1]);
+          if (kv + 2 > j) x[kv + 2] = fma_(xj, lv.z, x[kv + 2]);
+          x[kv + 3] = fma_(xj, lv.w, x[kv + 3]);
         }
       }
       // times D^-1 (apply_pivot OP_N)
@@ -491,16 +480,16 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
         if (k >= nd) break;
         const int kd = kind[k];
         if (kd == PV_ONE) {
-          x[k] = mul_(x[k], (C)dv[2 * k]);
+          x[k] = mul_(x[k], (float)dv[2 * k]);
         } else if (kd == PV_FIRST) {
           if (k + 1 < BW) {
             const double x1 = x[k], x2 = x[k + 1];
-            x[k] = (C)fma_(dv[2 * k], x1, mul_(dv[2 * k + 1], x2));
-            x[k + 1] = (C)fma_(dv[2 * k + 1], x1, mul_(dv[2 * k + 3], x2));
+            x[k] = (float)fma_(dv[2 * k], x1, mul_(dv[2 * k + 1], x2));
+            x[k + 1] = (float)fma_(dv[2 * k + 1], x1, mul_(dv[2 * k + 3], x2));
           }
         } else if (kd == PV_ZERO) {
           const double v = x[k];
-          x[k] = (C)((fabs(v) < st.small) ? 0.0 : dinf() * v);
+          x[k] = (float)((fabs(v) < st.small) ? 0.0 : dinf() * v);
         }
       }
       int first = nd;
@@ -510,7 +499,7 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
       if (first < nd) atomicMin(&fail, first);
 #pragma unroll
       for (int k = 0; k < BW; ++k)
-        if (k < nd) pan[k * pm + r] = (T)x[k];
+        if (k < nd) pan[k * pm + r] = x[k];
     }
   }
   __syncthreads();
@@ -523,7 +512,8 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_apply(const T* __restrict
 // pipes idle wherever a launch has fewer rows than the chip has warps.  Every
 // entry keeps its operations and their order.  14^3 saddle point: 30 -> 16 us per
 // launch.
-constexpr int R4 = 32, T4 = 128, NC4 = BW / 4, RW4 = 8;  // rows, threads, columns a lane, rows a warp
+constexpr int R4 = AppRows<double>::v, T4 = 4 * R4;  // rows, threads
+constexpr int NC4 = BW / 4, RW4 = 8;                 // columns a lane, rows a warp
 // the row's values in columns k - 1 and k + 1, k = 4 u + c
 __device__ __forceinline__ void neighbours4(const double (&x)[NC4], int u, int rl, int c,
                                             double& prev, double& next) {
@@ -641,16 +631,12 @@ __global__ void __launch_bounds__(T4) k_app_apply64(const double* __restrict__ a
 // columns).  The block's permutation is applied to its rows of the eliminated
 // columns.  The CTA with local index 0 stores D and the state.  One row per
 // thread, its 32 values in registers: 35 -> 16 us per launch on the shifted
-// 48^3.  FP32 only; FP64 goes through k_app_commit64.
-template <typename T>
-__global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ arena,
-                                                              T* __restrict__ scratch,
-                                                              const LdltFront* __restrict__ fr,
-                                                              const CtaMap* __restrict__ cm,
-                                                              LdltStep st) {
-  using C = T;
-  constexpr int RT = AppRows<T>::v;
-  __shared__ C L[BW][LDB];
+// 48^3.  FP64 goes through k_app_commit64.
+__global__ void __launch_bounds__(AppRows<float>::v)
+    k_app_commit32(float* __restrict__ arena, float* __restrict__ scratch,
+                   const LdltFront* __restrict__ fr, const CtaMap* __restrict__ cm, LdltStep st) {
+  constexpr int RT = AppRows<float>::v;
+  __shared__ float L[BW][LDB];
   __shared__ double dv[2 * BW];
   __shared__ double dca[BW], dcb[BW];  // D of a 2x2 pair's two columns
   __shared__ int perm[BW], kind[BW];
@@ -658,10 +644,10 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
   const LdltFront F = fr[c.f];
   const int q = F.fidx, w = block_width(F, st.k);
   const int p = st.p_cur[q], nd = st.ndiag[q];
-  T* A = arena + F.off;
+  float* A = arena + F.off;
   const int64_t ld = F.ld, pm = F.m;
   const int tid = threadIdx.x;
-  const C* blk = reinterpret_cast<const C*>(st.blk) + (int64_t)q * BW * LDB;
+  const float* blk = reinterpret_cast<const float*>(st.blk) + (int64_t)q * BW * LDB;
   // only the tile of the block's own rows reads L (the rest come from apply)
   if (c.local == 0)
     for (int idx = tid; idx < BW * LDB; idx += RT) (&L[0][0])[idx] = blk[idx];
@@ -677,10 +663,10 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
     if (__any_sync(0xffffffffu, lane < w && pl != lane))
       for (int c0 = (c.local * (RT / 32) + (tid >> 5)) * PU; c0 < p;
            c0 += c.count * (RT / 32) * PU) {
-        T v[PU];
+        float v[PU];
 #pragma unroll
         for (int u = 0; u < PU; ++u)
-          v[u] = (lane < w && c0 + u < p) ? A[(c0 + u) * ld + p + pl] : T(0);
+          v[u] = (lane < w && c0 + u < p) ? A[(c0 + u) * ld + p + pl] : 0.f;
         __syncwarp();
 #pragma unroll
         for (int u = 0; u < PU; ++u)
@@ -702,8 +688,8 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
     }
   }
   __syncthreads();
-  const T* pan = scratch + F.pan_off;
-  T* ldp = scratch + F.ldp_off;
+  const float* pan = scratch + F.pan_off;
+  float* ldp = scratch + F.ldp_off;
   for (int t0 = p + c.local * RT; t0 < F.m; t0 += c.count * RT) {
     const int r = t0 + tid;
     const bool in_blk = r < p + w;
@@ -711,20 +697,20 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
     // phase 1: L of the passed columns, the values failed columns keep
     // (in-block rows all belong to the tile that starts at p, so no other
     // CTA writes what this one reads)
-    C l[BW];
+    float l[BW];
     if (r < F.m && !in_blk) {
 #pragma unroll
       for (int k = 0; k < BW; ++k)
-        l[k] = k < np ? (C)pan[k * pm + r] : k < w ? (C)A[(p + perm[k]) * ld + r] : C(0);
+        l[k] = k < np ? pan[k * pm + r] : k < w ? A[(p + perm[k]) * ld + r] : 0.f;
     } else if (r < F.m) {
 #pragma unroll
       for (int k = 0; k < BW; ++k) {
-        C v = C(0);
+        float v = 0.f;
         if (k < np) {
-          v = (i > k) ? L[k][i] : (i == k ? C(1) : C(0));
+          v = (i > k) ? L[k][i] : (i == k ? 1.f : 0.f);
         } else if (k < w && i >= k) {
           const int ai = perm[i], ak = perm[k];
-          v = (C)A[(p + min(ai, ak)) * ld + p + max(ai, ak)];
+          v = A[(p + min(ai, ak)) * ld + p + max(ai, ak)];
         }
         l[k] = v;
       }
@@ -733,21 +719,21 @@ __global__ void __launch_bounds__(AppRows<T>::v) k_app_commit(T* __restrict__ ar
     if (r < F.m) {
 #pragma unroll
       for (int k = 0; k < BW; ++k)
-        if (k < w && !(in_blk && i < k)) A[(p + k) * ld + r] = (T)l[k];
+        if (k < w && !(in_blk && i < k)) A[(p + k) * ld + r] = l[k];
       if (r >= p + np) {
 #pragma unroll
         for (int k = 0; k < BW; ++k) {
           if (k >= np) break;
           const int kd = kind[k];
-          C v = C(0);
+          float v = 0.f;
           if (kd == PV_ONE) {
-            v = l[k] / (C)dv[2 * k];
+            v = l[k] / (float)dv[2 * k];
           } else if (kd == PV_FIRST) {
-            if (k + 1 < BW) v = (C)fma_((double)l[k], dca[k], mul_((double)l[k + 1], dcb[k]));
+            if (k + 1 < BW) v = (float)fma_((double)l[k], dca[k], mul_((double)l[k + 1], dcb[k]));
           } else if (kd == PV_SECOND) {
-            if (k > 0) v = (C)fma_((double)l[k - 1], dca[k], mul_((double)l[k], dcb[k]));
+            if (k > 0) v = (float)fma_((double)l[k - 1], dca[k], mul_((double)l[k], dcb[k]));
           }
-          ldp[k * pm + r] = (T)v;
+          ldp[k * pm + r] = v;
         }
       }
     }
@@ -1246,14 +1232,14 @@ void launch_app_apply(const T* arena, T* scratch, const LdltFront* fr, const Cta
                       LdltStep st, cudaStream_t s) {
   if (ncta <= 0) return;
   if constexpr (sizeof(T) == 8) k_app_apply64<<<ncta, T4, 0, s>>>(arena, scratch, fr, cm, st);
-  else k_app_apply<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
+  else k_app_apply32<<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_commit(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,
                        LdltStep st, cudaStream_t s) {
   if (ncta <= 0) return;
   if constexpr (sizeof(T) == 8) k_app_commit64<<<ncta, T4, 0, s>>>(arena, scratch, fr, cm, st);
-  else k_app_commit<T><<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
+  else k_app_commit32<<<ncta, AppRows<T>::v, 0, s>>>(arena, scratch, fr, cm, st);
 }
 template <typename T>
 void launch_app_move(T* arena, T* scratch, const LdltFront* fr, const CtaMap* cm, int ncta,

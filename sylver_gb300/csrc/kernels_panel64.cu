@@ -24,7 +24,6 @@ namespace {
 constexpr int PB = 32;         // panel width
 constexpr int PLD = PB + 1;
 constexpr int P64_THREADS = 128;
-constexpr int NUM_SMS = 152;
 
 // One CTA of four warps: rows [r0, r1) of a panel.
 //   diagonal block: in blocks of eight columns; one warp, a row per lane,

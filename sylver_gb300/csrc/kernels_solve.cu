@@ -1734,7 +1734,7 @@ void launch_residual(const int64_t* rowptr, const int* col, const double* aval, 
 void launch_maxnorms(const double* res, const double* x, int ldx, const double* b, int ldb,
                      int n, int nrhs, double* norms, cudaStream_t s) {
   if (n == 0) return;
-  dim3 grid(std::min(nblocks(n, 256), 152), nrhs);
+  dim3 grid(std::min(nblocks(n, 256), NUM_SMS), nrhs);
   k_maxnorms<<<grid, 256, 0, s>>>(res, x, ldx, b, ldb, n, nrhs, norms);
 }
 

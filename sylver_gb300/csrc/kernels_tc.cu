@@ -359,7 +359,7 @@ void launch_update_tc(const CUtensorMap* maps, float* arena, const TcTask* t, in
                       unsigned* err, cudaStream_t s) {
   if (ntask <= 0) return;
   // one persistent CTA per SM (the shared-memory ring admits one per SM)
-  const int grid = std::min(ntask, g_num_sms > 0 ? g_num_sms : 148);
+  const int grid = std::min(ntask, g_num_sms > 0 ? g_num_sms : NUM_SMS);
   k_update_tc<<<grid, TC_THREADS, tc_smem_bytes(), s>>>(maps[0], maps[1], maps[2], arena, t,
                                                          ntask, err);
 }

@@ -675,7 +675,7 @@ void launch_oz_split(const double* arena, const OzSplit* sp, int nsplit, int64_t
 void launch_update_tc64(const CUtensorMap* maps, double* arena, const int* sexp, const OzTask* t,
                         int ntask, unsigned* redo, unsigned* err, cudaStream_t s) {
   if (ntask <= 0) return;
-  const int sms = g_num_sms64 > 0 ? g_num_sms64 : 148;
+  const int sms = g_num_sms64 > 0 ? g_num_sms64 : NUM_SMS;
   k_update_tc64<<<std::min(ntask, sms), OZ_THREADS, tc64_smem_bytes(), s>>>(
       maps[0], maps[1], arena, sexp, t, ntask, redo, err);
   launch_pdl(k_redo64, dim3(std::min(ntask * OZ_EPI_WARPS, 8 * sms)), dim3(32 * REDO_WARPS), 0, s,

@@ -644,7 +644,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
           const int64_t c = ceil_div(L.m[s2] - L.n[s2], TM);
           nt += c * (c + 1) / 2;
         }
-        if (nt < 4 * 152) UT = TM / 2;
+        if (nt < 4 * NUM_SMS) UT = TM / 2;
       }
       for (int q = 0; q < nslot; ++q) {
         int s2 = F[q];

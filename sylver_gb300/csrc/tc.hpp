@@ -53,7 +53,7 @@ constexpr int OZ_KB = 512;
 // Level and front sizes do not set the size of the planes: what does not fit goes
 // in several launches, each still of thousands of tile columns.
 constexpr int64_t OZ_MIN_ENTRIES = 1 << 22, OZ_MAX_ENTRIES = 1 << 27;
-constexpr int OZ_FEW_TILES = 304;  // launches below this many CTAs take smaller tiles
+constexpr int OZ_FEW_TILES = 2 * NUM_SMS;  // launches below this many CTAs take smaller tiles
 // Digits of front rows [r0, r0 + rows) x columns [c0, c0 + K): stacked rows
 // [base, base + rows) of the planes (zeros from K to K rounded up to
 // OZ_KC), and each row's scale exponent in sexp[base ..].
