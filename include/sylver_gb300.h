@@ -387,13 +387,17 @@ int spldlt_tree_solve_fwd_noalloc_dbl(bool posdef, void const* tree, int nrhs, d
 /* ---- schedule (kernel-path choices; no reference counterpart) ------------ */
 
 /* Kernel paths of the level schedule.  They select which kernels process a
- * front, never the arithmetic.  0 keeps the built-in default. */
+ * front, not the method or its precision: results of two schedules differ by
+ * roundings (the order of sums), and both keep to the same bounds.  0 keeps the
+ * built-in default. */
 typedef struct {
   int small_front_rows;  /* Cholesky: fronts with at most this many rows are factorised whole
                             by one CTA (capped at 96 FP64 / 128 FP32; default 80 / 128) */
   int tc_min_cb_rows;    /* FP32 Cholesky: contribution blocks with at least this many rows
                             use the tensor-core update (default 64; negative: never, and
-                            FP64 fronts then keep to the FP64 pipe as well) */
+                            FP64 fronts then keep to the FP64 pipe as well: sums of rounded
+                            multiply-adds in place of digit products, of which an entry
+                            leaves out at most as much as such a sum rounds away) */
   int solve_large_cols;  /* fronts with at least this many eliminated columns use the blocked
                             multi-CTA solve (default 96) */
   int ldlt_tpp_cols;     /* LDL^T: fronts with at most this many fully-summed columns skip the

@@ -7,8 +7,10 @@
 // costs no more than half of its own rows' solve and saves a launch and a
 // round trip through memory per step; pivots take 1/sqrt from an FP32
 // estimate and one cubic step instead of an IEEE square root and division, which
-// ran on every thread of the block before.  A panel of any size takes at least
-// 22 us (about 200 clocks a pivot); a launch of 1500 panels' blocks on 33x29x31
+// ran on every thread of the block before.  A panel takes at least 18 us with 16 rows
+// a CTA and 24 us with 32: 29,000 clocks for the block (32 pivots of about 600 with
+// their updates of the block of four, eight updates of 1,200 behind it) and 9,400 or
+// 15,700 for the rows' substitution; a launch of 1500 panels' blocks on 33x29x31
 // was 69 us with a kernel each for block and rows.  33x29x31: 6.8 ms of
 // block and row kernels -> 2.3 ms; 56^3: 24 ms -> 11.1 ms.
 //
@@ -26,7 +28,7 @@ constexpr int PLD = PB + 1;
 constexpr int P64_THREADS = 128;
 
 // One CTA of four warps: rows [r0, r1) of a panel.
-//   diagonal block: in blocks of eight columns; one warp, a row per lane,
+//   diagonal block: in blocks of four columns; one warp, a row per lane,
 //     factorises the block's columns in registers (its pivots reach the other
 //     lanes by shuffles, no barrier), then all threads apply it to the triangle
 //     behind it, an entry per thread;

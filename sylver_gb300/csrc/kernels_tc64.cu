@@ -25,9 +25,9 @@
 // digits where |d| >= 2^-15 2^(ei + ej), which keeps what is left out below
 // (K + 1) 2^-53 |d|, or where |C| >= K 2^-12 2^(ei + ej), which keeps it below 2^-56 |C|; others
 // (rows whose large entries do not meet: graded rows, nodes far from one another) are
-// summed in FP64 by k_redo64.  Seven digits, 2^-59 of the norms and no such test
-// left entries of L L^T of 12 x 12 x 12 boxes with edge weights over 10^+-3 up to
-// thousands of FP64 bounds off.
+// summed in FP64 by k_redo64.  Seven digits and no such test left entries of a 20^3
+// box up to 2700 units of 2^-53 |L| |L^T| off (an FP64 sum: 22), and those of distant nodes
+// of a 100 x 100 grid with a mass term without a correct bit.
 //
 // Bound by the MMAs.  The products with one digit of A take one or two MMAs, its
 // digits of B side by side (12 MMAs per 16 k instead of 36: one costs about 90

@@ -788,7 +788,7 @@ static int factorize_ldlt_t(FKeep& fk, cudaStream_t s) {
   put(L, L.sdoff, L.hsdoff, s);
   // per-step launches unless asked for: on the shifted 7-point 48^3 matrix (4
   // right-hand sides, five corrections) the dataflow sweeps measured slower
-  // (refined solve 23.0-24.2 ms against 21.0-22.4 ms)
+  // (refined solve 15.8 ms against 15.2 ms)
   fk.splan.dataflow = Schedule::current().solve_dataflow > 0;
   fk.splan.build_tasks(L.hsfr, fk.levels, (int)sizeof(T), s);
   fk.splan.compute_inverses<T>(static_cast<const T*>(fk.factor_base()), L.sfr.as<FrontDesc>(),

@@ -1106,6 +1106,8 @@ int FKeep::factorize(const double* val_dev, cudaStream_t s) {
   }
   SG_CUDA(cudaEventRecord(e1, s));
   launches = (long)ops.size();
+  if (precision != 1)  // each with k_redo64 behind it
+    launches += std::count_if(ops.begin(), ops.end(), [](const Op& o) { return o.kind == Op::TCUPD; });
   unsigned st = 0, tce = 0;
   SG_CUDA(cudaMemcpyAsync(&st, status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   SG_CUDA(cudaMemcpyAsync(&tce, tcerr.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));

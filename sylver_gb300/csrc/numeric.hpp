@@ -64,7 +64,7 @@ struct DevMem {
   }
 };
 
-// Kernel-path choices of the schedule (never the arithmetic).  Read when a
+// Kernel-path choices of the schedule (results differ by roundings).  Read when a
 // factorization is planned; 0 selects the built-in default.
 struct Schedule {
   int small_front_rows = 0;  // Cholesky: fronts with <= rows factorised whole by one CTA

@@ -3,8 +3,8 @@
 A *schedule* (``sylver_gb300_schedule_t``) chooses which kernels process
 which fronts -- for LDL^T, the column count below which a front skips the
 a-posteriori block steps and goes straight to threshold partial pivoting;
-for Cholesky, the small-front cutoff and the tensor-core threshold.  It never
-changes the arithmetic of a pivot decision or an update.
+for Cholesky, the small-front cutoff and the tensor-core threshold.  Results of two
+schedules differ by roundings (the order of sums), not in method or precision.
 
 * ``Autotuner`` measures every candidate schedule on the matrix (CUDA-event
   factor time reported by the library) and keeps the fastest: exact, but it
@@ -37,6 +37,9 @@ its training range.
     python -m sylver_gb300.scheduler chol-record OUT.npz [count] [seed0]
     python -m sylver_gb300.scheduler chol-train DATA.npz OUT_WEIGHTS.npz [epochs]
     python -m sylver_gb300.scheduler chol-evaluate WEIGHTS.npz [k ...]
+
+data/sched_timings.npz holds the LDL^T timings behind sched_mlp.npz; those behind
+sched_chol_mlp.npz (chol-record on a GB300) were not kept.
 """
 from __future__ import annotations
 
